@@ -333,8 +333,7 @@ extern "C" int pes_fisher_batch(PesPlan* p, const double* theta, int64_t B, doub
     PES_CHECK_CUDA(cudaMalloc(&p->fisher_partial, sizeof(double) * M * kFisherBlocks * kPairs));
   }
   auto* blocks = reinterpret_cast<SampleBlock<FisherScalar>*>(p->fisher_blocks);
-  k_setup<FisherScalar><<<(unsigned)ceil_div(B, kPerSampleThreads), kPerSampleThreads, 0, st>>>(
-      p->dev, theta, B, 0, blocks, hm_blocks<FisherScalar>(p));
+  k_setup<FisherScalar><<<setup_blocks(B), 64, 0, st>>>(p->dev, theta, B, 0, blocks, hm_blocks<FisherScalar>(p));
   PES_CHECK_LAUNCH();
   const bool hm = p->desc.approximant == PES_APPROX_PHENOMHM;
   if (p->mixed && !hm)  // mixed IMRPhenomD plans: FP32 structured derivatives

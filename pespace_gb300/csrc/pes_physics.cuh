@@ -9,6 +9,8 @@
 //     per-sample coefficient block as polynomials in u = (M f)^{1/3}.
 #pragma once
 
+#include <type_traits>
+
 #include "pes_common.cuh"
 #include "pes_ff.cuh"
 #include "../../include/pespace_gb300.h"
@@ -366,7 +368,7 @@ constexpr double kMfCut = 0.2;         // PhenomD is zero above Mf = 0.2
 // xi = chi_PN - 1.
 enum { kFV2, kFG1, kFG2, kFG3, kFS1, kFS2, kFS3, kFS4, kFB1, kFB2, kFB3, kFA1, kFA2, kFA3, kFA4, kFA5,
        kFR1, kFR2, kFR3, kFCount };
-__device__ __constant__ static const double kPhenomFits[kFCount][11] = {
+__device__ static const double kPhenomFits[kFCount][11] = {
   {0.8149838730507785, 2.5747553517454658, 1.1610198035496786, -2.3627771785551537, 6.771038707057573, 0.7570782938606834, -2.7256896890432474, 7.1140380397149965, 0.1766934149293479, -0.7978690983168183, 2.1162391502005153},
   {0.006927402739328343, 0.03020474290328911, 0.006308024337706171, -0.12074130661131138, 0.26271598905781324, 0.0034151773647198794, -0.10779338611188374, 0.27098966966891747, 0.0007374185938559283, -0.02749621038376281, 0.0733150789135702},
   {1.010344404799477, 0.0008993122007234548, 0.283949116804459, -4.049752962958005, 13.207828172665366, 0.10396278486805426, -7.025059158961947, 24.784892370130475, 0.03093202475605892, -2.6924023896851663, 9.609374464684983},
@@ -407,12 +409,23 @@ struct PhenomDCoef {
   T af, erad, eta, v2;  // remnant spin, radiated energy, symmetric mass ratio, amplitude collocation value
 };
 
-template <class T>
-PES_HD T phenom_fit(int w, const T& eta, const T& xi) {
+// One coefficient fit and its partial derivatives: out = (value, d/d eta, d/d xi).
+PES_HD void phenom_fit_row(int w, double eta, double xi, double out[3]) {
   const double* c = kPhenomFits[w];
-  T eta2 = eta * eta;
-  return c[0] + c[1] * eta + xi * (c[2] + c[3] * eta + c[4] * eta2) +
-         xi * xi * ((c[5] + c[6] * eta + c[7] * eta2) + xi * (c[8] + c[9] * eta + c[10] * eta2));
+  const double a0 = c[2] + eta * (c[3] + eta * c[4]), a1 = c[5] + eta * (c[6] + eta * c[7]),
+               a2 = c[8] + eta * (c[9] + eta * c[10]);
+  out[0] = c[0] + c[1] * eta + xi * (a0 + xi * (a1 + xi * a2));
+  out[1] = c[1] + xi * ((c[3] + 2.0 * c[4] * eta) + xi * ((c[6] + 2.0 * c[7] * eta) + xi * (c[9] + 2.0 * c[10] * eta)));
+  out[2] = a0 + xi * (2.0 * a1 + 3.0 * xi * a2);
+}
+PES_HD double fit_value(const double* row, const double&, const double&) { return row[0]; }
+template <int N, class D, class V>
+PES_HD Dual<N, D, V> fit_value(const double* row, const Dual<N, D, V>& eta, const Dual<N, D, V>& xi) {
+  Dual<N, D, V> r;
+  r.v = V(row[0]);
+#pragma unroll
+  for (int i = 0; i < N; ++i) r.d[i] = D(row[1]) * eta.d[i] + D(row[2]) * xi.d[i];
+  return r;
 }
 
 // Phase and its Mf-derivative from the coefficient block (region by Mf).
@@ -487,6 +500,288 @@ PES_HD void amp_peak_jump(const PhenomDCoef<T>& c, T& ahat_pk, T& jump) {
   jump = d2m - d2i;
 }
 
+// The intermediate amplitude's quartic in Mf from its conditions: value A1 and
+// slope D1 at f1, A3 and D3 at f3, value v2 midway.  In x = (f - f1) / h,
+// h = f3 - f1, it is the cubic Hermite interpolant plus e x^2 (1 - x)^2, and e
+// follows from the midpoint value alone, so no linear system is solved (its
+// pivoted elimination took 15 FP64 divisions and about 250 further operations
+// in the serial chain of every set-up).
+template <class T>
+PES_HD void quartic_coef(const T& f1, const T& f3, const T& A1, const T& D1, const T& A3, const T& D3, const T& v2,
+                         T dl[5]) {
+  const T h = f3 - f1, ih = 1.0 / h;
+  const T b = h * D1, g = h * D3, dA = A3 - A1;
+  // x^2 (1 - x)^2 = x^2 - 2 x^3 + x^4, 1/16 at the midpoint
+  const T e = 16.0 * v2 - 8.0 * (A1 + A3) - 2.0 * (b - g);
+  // powers of (f - f1)
+  const T c1 = D1, c2 = (3.0 * dA - 2.0 * b - g + e) * (ih * ih);
+  const T ih2 = ih * ih;
+  const T c3 = (b + g - 2.0 * dA - 2.0 * e) * (ih2 * ih), c4 = e * (ih2 * ih2);
+  // Taylor shift by -f1
+  const T p3 = c3 - f1 * c4, q3 = p3 - f1 * c4, r3 = q3 - f1 * c4;
+  const T p2 = c2 - f1 * p3, q2 = p2 - f1 * q3;
+  const T p1 = c1 - f1 * p2;
+  dl[4] = c4;
+  dl[3] = r3 - f1 * c4;
+  dl[2] = q2 - f1 * r3;
+  dl[1] = p1 - f1 * q2;
+  dl[0] = A1 - f1 * p1;
+}
+
+// The inspiral's joins are at the same Mf for every source (0.014 amplitude,
+// 0.018 phase): the powers of u = Mf^{1/3} there are constants.
+constexpr double kJoinU = 0.26207413942088964, kJoinLnU = -1.3391278403619908, kJoinLnF = -4.017383521085972;
+
+// The (2,2) inspiral amplitude hat and its Mf-derivative at Mf = 0.014.
+template <class T>
+PES_HD void amp_join(const PhenomDCoef<T>& c, T& A, T& dA) {
+  // u^(j+2) and (j+2)/3 u^(j-1) at Mf = 0.014
+  constexpr double kJoinAmp[8] = {0.05808785733563704, 0.014, 0.003374199169845322, 0.0008132300026989185,
+      0.000196, 4.723878837783451e-05, 1.138522003778486e-05, 2.744e-06};
+  constexpr double kJoinDAmp[8] = {2.766088444554145, 1.0, 0.32135230189003067, 0.09681309555939507, 0.028,
+      0.00787313139630575, 0.0021686133405304495, 0.000588};
+  A = 1.0 + c.ai[0] * kJoinAmp[0];
+  dA = c.ai[0] * kJoinDAmp[0];
+#pragma unroll
+  for (int j = 1; j < 8; ++j) {
+    A = A + c.ai[j] * kJoinAmp[j];
+    dA = dA + c.ai[j] * kJoinDAmp[j];
+  }
+}
+
+// Merger-ringdown amplitude hat of width w (= gamma3 f_DM) at Mf and its derivative.
+template <class T>
+PES_HD void amp_mrd(const PhenomDCoef<T>& c, const T& w, const T& Mf, T& A, T& dA) {
+  const T x = Mf - c.fRD, iw = 1.0 / w, iden = 1.0 / (x * x + w * w), g = c.g2 * iw;
+  A = c.g1 * w * iden * dexp(-(g * x));
+  dA = A * (-g - 2.0 * (x * iden));
+}
+
+// Build the coefficient block from the 11-parameter vector (see the C header).
+//
+// A group of nlane threads sets up one sample: they evaluate the 19
+// coefficient fits side by side into `rows` (value and the derivatives with
+// respect to eta and xi, shared by the group), and every thread then runs the
+// rest.  GB300 issues an FP64 instruction of a warp over 64 cycles whatever
+// the number of its active lanes, and the serial chain of one sample is what a
+// small batch waits for: the fits side by side, the closed form of the
+// intermediate amplitude and the tabulated joins cut that chain.  With T = a
+// dual number of one tangent each thread of a group carries its own parameter's
+// tangent, so that a gradient set-up costs about two value set-ups.
+// kRole: which fields are wanted, kPhasePart (Msec .. fpeak, the phase's
+// coefficients, tscale) and/or kAmpPart (the amplitude's and the polarisation
+// factors, af .. v2); two warps on different SM partitions take one each.
+constexpr int kPhasePart = 1, kAmpPart = 2;
+template <class T, int kRole = 3>
+PES_HD void phenomd_setup(const T* th, double f_ref, double (*rows)[3], int lane, int nlane, unsigned mask,
+                          PhenomDCoef<T>& c) {
+  const T one = lift<T>(1.0);
+  const T q = th[1];
+  const T chi1 = th[2], chi2 = th[3];
+  const T iopq = 1.0 / (one + q);
+  const T m1 = q * iopq, m2 = iopq;
+  const T eta = m1 * m2;
+  const T ieta = 1.0 / eta;
+  const T M = dexp(th[0]) * dexp(-0.6 * dlog(eta));
+  const T seta = (q - 1.0) * iopq;
+  const T eta2 = eta * eta, eta3 = eta2 * eta;
+  c.Msec = M * kMTSun;
+  c.tscale = c.Msec * (1.0 / (2.0 * kPi));
+  const T xi = m1 * chi1 + m2 * chi2 - (38.0 / 113.0) * eta * (chi1 + chi2) - 1.0;
+  for (int w = lane; w < kFCount; w += nlane) phenom_fit_row(w, val(eta), val(xi), rows[w]);
+#ifdef __CUDA_ARCH__
+  __syncwarp(mask);
+#else
+  (void)mask;
+#endif
+  auto fit = [&](int w) { return fit_value(rows[w], eta, xi); };
+  // remnant spin and radiated energy (Husa et al. 2016)
+  const T s = m1 * m1 * chi1 + m2 * m2 * chi2;
+  const T af = eta * (3.4641016151377544 - 4.399247300629289 * eta + 9.397292189321194 * eta2 -
+                13.180949901606242 * eta3 +
+                s * ((ieta - 0.0850917821418767 - 5.837029316602263 * eta) +
+                     s * ((0.1014665242971878 - 2.0967746996832157 * eta) +
+                          s * ((-1.3546806617824356 + 4.108962025369336 * eta) +
+                               s * (-0.8676969352555539 + 2.064046835273906 * eta)))));
+  const T sn = s / (m1 * m1 + m2 * m2);
+  const T erad = ((0.055974469826360077 + 0.5809510763115132 * eta - 0.9606726679372312 * eta2 +
+             3.352411249771192 * eta3) * eta *
+            (1.0 + (-0.0030302335878845507 - 2.0066110851351073 * eta + 7.7050567802399215 * eta2) * sn)) /
+           (1.0 + (-0.6714403054720589 - 1.4756929437702908 * eta + 7.304676214885011 * eta2) * sn);
+  // (2,2,0) quasi-normal mode of the remnant (mass 1 - E_rad, spin af)
+  T wR, wI;
+  qnm_interp<T>(0, af, wR, wI);
+  const T irem = (1.0 / (2.0 * kPi)) / (one - erad);
+  c.fRD = wR * irem;
+  c.fDM = wI * irem;
+  const T v2 = fit(kFV2);
+  c.af = af;
+  c.erad = erad;
+  c.eta = eta;
+  c.v2 = v2;
+  c.g1 = fit(kFG1);
+  c.g2 = fit(kFG2);
+  c.g3fDM = fit(kFG3) * c.fDM;
+  if (val(c.g2) <= 1.0)
+    c.fpeak = dabs(c.fRD + c.g3fDM * (dsqrt(one - c.g2 * c.g2) - 1.0) / c.g2);
+  else
+    c.fpeak = dabs(c.fRD - c.g3fDM / c.g2);
+  constexpr double pi13 = 1.4645918875615234, pi23 = 2.1450293971110255, pi43 = 4.60115111447049,
+                   pi53 = 6.738808595698141, pi2 = kPi * kPi;
+  const T c12 = chi1 * chi1, c22 = chi2 * chi2, c1c2 = chi1 * chi2;
+  if constexpr ((kRole & kAmpPart) != 0) {
+    // 3PN SPA amplitude of the inspiral in powers of u = Mf^{1/3}
+    const T sp = one + seta, sm = one - seta;
+    c.ai[0] = (-969.0 + 1804.0 * eta) * (pi23 / 672.0);
+    c.ai[1] = (chi1 * (81.0 * sp - 44.0 * eta) + chi2 * (81.0 * sm - 44.0 * eta)) * (kPi / 48.0);
+    c.ai[2] = (-27312085.0 - 10287648.0 * (c12 * sp + c22 * sm) +
+               24.0 * (-1975055.0 + 857304.0 * (c12 + c22) - 994896.0 * c1c2) * eta + 35371056.0 * eta2) *
+              (pi43 / 8128512.0);
+    c.ai[3] = (chi1 * (285197.0 * sp - 4.0 * (91902.0 + 1579.0 * seta) * eta - 35632.0 * eta2) +
+               chi2 * (285197.0 * sm - 4.0 * (91902.0 - 1579.0 * seta) * eta - 35632.0 * eta2) +
+               42840.0 * kPi * (-1.0 + 4.0 * eta)) *
+              (pi53 / 32256.0);
+    c.ai[4] = (336.0 * (-3248849057.0 + 2943675504.0 * (c12 + c22) - 3339284256.0 * c1c2) * eta2 +
+               324322727232.0 * eta3 +
+               7.0 * (-177520268561.0 + 107414046432.0 * (c12 * sp + c22 * sm) +
+                      11087290368.0 * kPi * (chi1 * sp + chi2 * sm)) -
+               12.0 * eta *
+                   (-545384828789.0 - 176491177632.0 * c1c2 + 77616.0 * 2610335.0 * (c12 + c22) +
+                    77616.0 * 995766.0 * seta * (c12 - c22) + 5841690624.0 * kPi * (chi1 + chi2) +
+                    21384760320.0 * pi2)) *
+              (pi2 / 60085960704.0);
+    // calibrated terms rho1 Mf^{7/3} + rho2 Mf^{8/3} + rho3 Mf^3 (Khan et al. 2016 eq. 29)
+    c.ai[5] = fit(kFR1);
+    c.ai[6] = fit(kFR2);
+    c.ai[7] = fit(kFR3);
+  }
+  if constexpr ((kRole & kPhasePart) != 0) {
+    // TaylorF2 aligned-spin phasing (3.5PN, spin-orbit to 3.5PN, 2PN spin-spin,
+    // no 3PN spin-spin) plus the sigma terms, as a series in u.
+    const T SL = s;
+    const T dSL = seta * (m2 * chi2 - m1 * chi1);
+    const T pn_sigma = (474.0 / 48.0) * eta * c1c2 + (486.0 / 96.0) * (m1 * m1 * c12 + m2 * m2 * c22);
+    const T pn_gamma = (554345.0 / 1134.0 + (110.0 / 9.0) * eta) * SL + (13915.0 / 84.0 - (10.0 / 3.0) * eta) * dSL;
+    const T pfaN = (3.0 / 128.0) * ieta;
+    const T b5 = kPi * (7729.0 / 84.0 - 13.0 * eta);
+    const T v5 = (5.0 / 9.0) * b5 - pn_gamma;
+    const T vl5 = (5.0 / 3.0) * b5 - 3.0 * pn_gamma;
+    const T v6 = lift<T>(11583.231236531 / 4.694215680 - 640.0 / 3.0 * pi2 - 6848.0 / 21.0 * kEulerGamma -
+                   6848.0 / 21.0 * 1.3862943611198906) +
+           eta * (-15737.765635 / 3.048192 + 2255.0 / 12.0 * pi2) + eta2 * (76055.0 / 1728.0) -
+           eta3 * (127825.0 / 1296.0) + (kPi / 3.0) * (3760.0 * SL + 1490.0 * dSL);
+    constexpr double vl6 = -6848.0 / 21.0;
+    const T a7 = kPi * (77096675.0 / 254016.0 + (378515.0 / 1512.0) * eta - (74045.0 / 756.0) * eta2) +
+           (-8980424995.0 / 762048.0 + (6586595.0 / 756.0) * eta - (305.0 / 36.0) * eta2) * SL -
+           (170978035.0 / 48384.0 - (2876425.0 / 672.0) * eta - (4735.0 / 144.0) * eta2) * dSL;
+    // v = pi^{1/3} u: pin_k = pfaN (a_k + vl_k ln pi^{1/3}) pi^{(k-5)/3}; ln v = ln pi^{1/3} + ln u
+    constexpr double lnpi13 = 0.38157662861646674;
+    c.pin[0] = pfaN * (1.0 / pi53);
+    c.pin[1] = lift<T>(0.0);
+    c.pin[2] = pfaN * ((5.0 / 9.0) * (743.0 / 84.0 + 11.0 * eta)) * (1.0 / kPi);
+    c.pin[3] = pfaN * (-16.0 * kPi + (188.0 / 3.0) * SL + 25.0 * dSL) * (1.0 / pi23);
+    c.pin[4] = pfaN * ((5.0 / 72.0) * (3058.673 / 7.056 + (5429.0 / 7.0) * eta + 617.0 * eta2) - 10.0 * pn_sigma) *
+               (1.0 / pi13);
+    c.pin[5] = pfaN * (v5 + vl5 * lnpi13) - 0.25 * kPi;
+    c.pin[6] = pfaN * (v6 + vl6 * lnpi13) * pi13;
+    c.pin[7] = pfaN * a7 * pi23;
+    c.pin[8] = fit(kFS1) * ieta;
+    c.pin[9] = 0.75 * (fit(kFS2) * ieta);
+    c.pin[10] = 0.6 * (fit(kFS3) * ieta);
+    c.pin[11] = 0.5 * (fit(kFS4) * ieta);
+    c.lg0 = pfaN * vl5;
+    c.lg1 = pfaN * (vl6 * pi13);
+    c.pint[0] = lift<T>(0.0);
+    c.pint[1] = fit(kFB1) * ieta;
+    c.pint[2] = (-1.0 / 3.0) * (fit(kFB3) * ieta);
+    c.pint[3] = fit(kFB2) * ieta;
+    c.pm[0] = lift<T>(0.0);
+    c.pm[1] = fit(kFA1) * ieta;
+    c.pm[2] = -(fit(kFA2) * ieta);
+    c.pm[3] = (4.0 / 3.0) * (fit(kFA3) * ieta);
+    c.pm[4] = fit(kFA4) * ieta;
+    c.pm[5] = fit(kFA5) * c.fRD;
+    // C1 continuity of the phase: intermediate matched at Mf = 0.018, merger-ringdown at fRD/2
+    {
+      // u^(j-5) and (j-5)/3 u^(j-8) at Mf = 0.018
+      constexpr double kJoinPhi[12] = {808.8708006817582, 211.98411899135775, 55.55555555555556, 14.559674412271647,
+        3.8157141418444396, 1.0, 0.26207413942088964, 0.06868285455319992, 0.018, 0.004717334509576014,
+        0.0012362913819575984, 0.000324};
+      constexpr double kJoinDPhi[12] = {-74895.44450757021, -15702.527332693167, -3086.41975308642,
+        -539.2472004545054, -70.66137299711924, 0.0, 4.85322480409055, 2.543809427896293, 1.0, 0.3494321858945195,
+        0.11447142425533319, 0.036};
+      T pI = (c.lg0 + c.lg1 * kJoinU) * kJoinLnU, dI = (c.lg1 * ((kJoinLnU + 1.0) / 3.0)) * (1.0 / (kJoinU * kJoinU)) +
+                                                      c.lg0 * (1.0 / (3.0 * kPhiJoinIns));
+#pragma unroll
+      for (int j = 11; j >= 0; --j) {  // smallest terms first
+        if (j == 1) continue;          // pin[1] = 0
+        pI = pI + c.pin[j] * kJoinPhi[j];
+        if (j != 5) dI = dI + c.pin[j] * kJoinDPhi[j];
+      }
+      constexpr double if1 = 1.0 / kPhiJoinIns;
+      const T pN = c.pint[1] * kPhiJoinIns + c.pint[2] * (if1 * if1 * if1) + c.pint[3] * kJoinLnF;
+      const T dN = c.pint[1] - c.pint[2] * (3.0 * if1 * if1 * if1 * if1) + c.pint[3] * if1;
+      const T C2 = dI - dN;
+      c.pint[0] = pI - pN - C2 * kPhiJoinIns;
+      c.pint[1] = c.pint[1] + C2;
+      const T f2 = 0.5 * c.fRD;
+      const T if2 = 1.0 / f2, if23 = if2 * if2 * if2;
+      const T pI2 = c.pint[0] + c.pint[1] * f2 + c.pint[2] * if23 + c.pint[3] * dlog(f2);
+      const T dI2 = c.pint[1] - 3.0 * c.pint[2] * (if23 * if2) + c.pint[3] * if2;
+      const T q2 = dsqrt(dsqrt(f2)), q23 = q2 * q2 * q2;
+      const T x2 = f2 - c.pm[5];
+      const T pM = c.pm[1] * f2 + c.pm[2] * if2 + c.pm[3] * q23 + c.pm[4] * datan(x2 / c.fDM);
+      const T dM = c.pm[1] - c.pm[2] * if2 * if2 + 0.75 * c.pm[3] * (q23 * if2) +
+                   c.pm[4] * c.fDM / (c.fDM * c.fDM + x2 * x2);
+      const T C2m = dI2 - dM;
+      c.pm[0] = pI2 - pM - C2m * f2;
+      c.pm[1] = c.pm[1] + C2m;
+    }
+  }
+  if constexpr ((kRole & kAmpPart) != 0) {
+    // intermediate amplitude: value/derivative at 0.014 and fpeak, value v2 midway
+    {
+      T Ains, dAins, Amrd, dAmrd;
+      amp_join(c, Ains, dAins);
+      amp_mrd(c, c.g3fDM, c.fpeak, Amrd, dAmrd);
+      quartic_coef(lift<T>(kAmpJoinIns), c.fpeak, Ains, dAins, Amrd, dAmrd, v2, c.dl);
+    }
+  }
+  if constexpr ((kRole & kPhasePart) != 0) {
+    // alignment: t(fpeak) = 0 and Psi(f_ref) = -2 phi_c
+    {
+      T pp, t0;
+      phenomd_phase(c, c.fpeak, dcbrt(c.fpeak), pp, t0);
+      const T MfRef = c.Msec * f_ref;
+      T pr, dr;
+      phenomd_phase(c, MfRef, dcbrt(MfRef), pr, dr);
+      const T shift = t0 * MfRef - pr - 2.0 * th[9];
+      // fold -t0 Mf + shift into every region
+      c.pin[5] = c.pin[5] + shift;
+      c.pin[8] = c.pin[8] - t0;
+      c.pint[0] = c.pint[0] + shift;
+      c.pint[1] = c.pint[1] - t0;
+      c.pm[0] = c.pm[0] + shift;
+      c.pm[1] = c.pm[1] - t0;
+    }
+  }
+  if constexpr ((kRole & kAmpPart) != 0) {
+    const T DLm = dexp(th[4]) * (1.0e6 * kPc);
+    constexpr double amp_norm = 0.2606104117397385;  // 2 sqrt(5/(64 pi)) / pi^{1/6}
+    c.amp_scale = amp_norm * (M * kMRSun) * (M * kMTSun) / DLm * dsqrt(eta * (2.0 / 3.0));
+    c.pfac = 0.5 * (one + th[5] * th[5]);
+    c.cfac = th[5];
+  }
+}
+
+template <class T>
+PES_HD T phenom_fit(int w, const T& eta, const T& xi) {
+  const double* c = kPhenomFits[w];
+  T eta2 = eta * eta;
+  return c[0] + c[1] * eta + xi * (c[2] + c[3] * eta + c[4] * eta2) +
+         xi * xi * ((c[5] + c[6] * eta + c[7] * eta2) + xi * (c[8] + c[9] * eta + c[10] * eta2));
+}
+
 template <class T>
 PES_HD void solve5(T A[5][5], T b[5], T x[5]) {
   for (int col = 0; col < 5; ++col) {
@@ -510,9 +805,24 @@ PES_HD void solve5(T A[5][5], T b[5], T x[5]) {
   }
 }
 
-// Build the coefficient block from the 11-parameter vector (see the C header).
-template <class T>
-PES_HD void phenomd_setup(const T* th, double f_ref, PhenomDCoef<T>& c) {
+PES_HD double rounded_product(double a, double b) {
+#ifdef __CUDA_ARCH__
+  return __dmul_rn(a, b);
+#else
+  return a * b;
+#endif
+}
+
+// The coefficient block in the plain order of its formulae, for mixed IMRPhenomD
+// plans.  Their float-float nodes, FP32 splines and FP32 derivative passes
+// round what they read: a last-bit change of a coefficient moves phases of 1e5
+// rad by a float-float rounding (1e-9 rad), and some coefficients of the
+// intermediate amplitude by 1e-11 (ill-conditioned in powers of Mf), which
+// moved gradients by 7e-9 of their norm with phenomd_setup.  kRole as there;
+// `rows` (nullable): the fits' values by the group's threads (T = double).
+template <class T, int kRole>
+PES_HD void phenomd_setup_serial(const T* th, double f_ref, double (*rows)[3], int lane, int nlane, unsigned mask,
+                                 PhenomDCoef<T>& c) {
   const T one = lift<T>(1.0);
   T Mc = dexp(th[0]);
   T q = th[1];
@@ -525,8 +835,30 @@ PES_HD void phenomd_setup(const T* th, double f_ref, PhenomDCoef<T>& c) {
   T eta2 = eta * eta, eta3 = eta2 * eta;
   c.Msec = M * kMTSun;
   c.tscale = c.Msec * (1.0 / (2.0 * kPi));
-  T chipn = m1 * chi1 + m2 * chi2 - (38.0 / 113.0) * eta * (chi1 + chi2);
+  // the products enter several sums: rounded on their own (a compiler is free
+  // to contract a product that one sum uses, which would depend on kRole)
+  T mc1, mc2;
+  if constexpr (std::is_same<T, double>::value) {
+    mc1 = rounded_product(m1, chi1);
+    mc2 = rounded_product(m2, chi2);
+  } else {
+    mc1 = m1 * chi1;
+    mc2 = m2 * chi2;
+  }
+  T chipn = mc1 + mc2 - (38.0 / 113.0) * eta * (chi1 + chi2);
   T xi = chipn - 1.0;
+  if constexpr (std::is_same<T, double>::value) {
+    for (int w = lane; w < kFCount; w += nlane) rows[w][0] = phenom_fit<double>(w, eta, xi);
+#ifdef __CUDA_ARCH__
+    __syncwarp(mask);
+#endif
+  }
+  auto fit = [&](int w) -> T {
+    if constexpr (std::is_same<T, double>::value)
+      return rows[w][0];
+    else
+      return phenom_fit(w, eta, xi);
+  };
   // remnant spin and radiated energy (Husa et al. 2016)
   T s = m1 * m1 * chi1 + m2 * m2 * chi2;
   T af = eta * (3.4641016151377544 - 4.399247300629289 * eta + 9.397292189321194 * eta2 -
@@ -545,14 +877,14 @@ PES_HD void phenomd_setup(const T* th, double f_ref, PhenomDCoef<T>& c) {
   qnm_interp<T>(0, af, wR, wI);
   c.fRD = wR / (2.0 * kPi) / (one - erad);
   c.fDM = wI / (2.0 * kPi) / (one - erad);
-  T v2 = phenom_fit(kFV2, eta, xi);
+  T v2 = fit(kFV2);
   c.af = af;
   c.erad = erad;
   c.eta = eta;
   c.v2 = v2;
-  c.g1 = phenom_fit(kFG1, eta, xi);
-  c.g2 = phenom_fit(kFG2, eta, xi);
-  T g3 = phenom_fit(kFG3, eta, xi);
+  c.g1 = fit(kFG1);
+  c.g2 = fit(kFG2);
+  T g3 = fit(kFG3);
   c.g3fDM = g3 * c.fDM;
   if (val(c.g2) <= 1.0)
     c.fpeak = dabs(c.fRD + c.fDM * g3 * (dsqrt(one - c.g2 * c.g2) - 1.0) / c.g2);
@@ -581,13 +913,13 @@ PES_HD void phenomd_setup(const T* th, double f_ref, PhenomDCoef<T>& c) {
                   21384760320.0 * pi2)) *
             (pi2 / 60085960704.0);
   // calibrated terms rho1 Mf^{7/3} + rho2 Mf^{8/3} + rho3 Mf^3 (Khan et al. 2016 eq. 29)
-  c.ai[5] = phenom_fit(kFR1, eta, xi);
-  c.ai[6] = phenom_fit(kFR2, eta, xi);
-  c.ai[7] = phenom_fit(kFR3, eta, xi);
+  c.ai[5] = fit(kFR1);
+  c.ai[6] = fit(kFR2);
+  c.ai[7] = fit(kFR3);
   // TaylorF2 aligned-spin phasing (3.5PN, spin-orbit to 3.5PN, 2PN spin-spin,
   // no 3PN spin-spin) plus the sigma terms, as a series in u.
   T SL = m1 * m1 * chi1 + m2 * m2 * chi2;
-  T dSL = seta * (m2 * chi2 - m1 * chi1);
+  T dSL = seta * (mc2 - mc1);
   T pn_sigma = (474.0 / 48.0) * eta * c1c2 + (486.0 / 96.0) * (m1 * m1 * c12 + m2 * m2 * c22);
   T pn_gamma = (554345.0 / 1134.0 + (110.0 / 9.0) * eta) * SL + (13915.0 / 84.0 - (10.0 / 3.0) * eta) * dSL;
   T pfaN = 3.0 / (128.0 * eta);
@@ -618,8 +950,8 @@ PES_HD void phenomd_setup(const T* th, double f_ref, PhenomDCoef<T>& c) {
   pin[5] = pfaN * (v5 + vl5 * lnpi13) - 0.25 * kPi;
   pin[6] = pfaN * (v6 + vl6 * lnpi13) * pi13;
   pin[7] = pfaN * a[7] * pi23;
-  T s1 = phenom_fit(kFS1, eta, xi), s2 = phenom_fit(kFS2, eta, xi), s3 = phenom_fit(kFS3, eta, xi),
-    s4 = phenom_fit(kFS4, eta, xi);
+  T s1 = fit(kFS1), s2 = fit(kFS2), s3 = fit(kFS3),
+    s4 = fit(kFS4);
   T ieta = one / eta;
   pin[8] = s1 * ieta;
   pin[9] = 0.75 * s2 * ieta;
@@ -629,105 +961,111 @@ PES_HD void phenomd_setup(const T* th, double f_ref, PhenomDCoef<T>& c) {
   for (int j = 0; j < 12; ++j) c.pin[j] = pin[j];
   c.lg0 = pfaN * vl5;
   c.lg1 = pfaN * vl6 * pi13;
-  T b1 = phenom_fit(kFB1, eta, xi), b2 = phenom_fit(kFB2, eta, xi), b3 = phenom_fit(kFB3, eta, xi);
+  T b1 = fit(kFB1), b2 = fit(kFB2), b3 = fit(kFB3);
   c.pint[0] = lift<T>(0.0);
   c.pint[1] = b1 * ieta;
   c.pint[2] = -b3 * ieta * (1.0 / 3.0);
   c.pint[3] = b2 * ieta;
-  T a1 = phenom_fit(kFA1, eta, xi), a2 = phenom_fit(kFA2, eta, xi), a3 = phenom_fit(kFA3, eta, xi),
-    a4 = phenom_fit(kFA4, eta, xi), a5 = phenom_fit(kFA5, eta, xi);
+  T a1 = fit(kFA1), a2 = fit(kFA2), a3 = fit(kFA3),
+    a4 = fit(kFA4), a5 = fit(kFA5);
   c.pm[0] = lift<T>(0.0);
   c.pm[1] = a1 * ieta;
   c.pm[2] = -a2 * ieta;
   c.pm[3] = (4.0 / 3.0) * a3 * ieta;
   c.pm[4] = a4 * ieta;
   c.pm[5] = a5 * c.fRD;
-  // C1 continuity of the phase: intermediate matched at Mf = 0.018, merger-ringdown at fRD/2
-  {
-    T f1 = lift<T>(kPhiJoinIns);
-    T u1 = dcbrt(f1);
-    T pI, dI, pN, dN;
-    {  // inspiral branch at the join (Mf = 0.018 itself belongs to the intermediate region)
-      T lu = dlog(u1);
-      T P = c.pin[11], R = c.pin[11] * 2.0;
-      for (int j = 10; j >= 0; --j) { P = P * u1 + c.pin[j]; R = R * u1 + c.pin[j] * ((j - 5) / 3.0); }
-      T iu = 1.0 / u1, iu2 = iu * iu, iu4 = iu2 * iu2;
-      pI = P * iu4 * iu + (c.lg0 + c.lg1 * u1) * lu;
-      dI = R * iu4 * iu4 + (c.lg1 * (lu + 1.0) * (1.0 / 3.0)) * iu2 + c.lg0 * (1.0 / 3.0) * iu2 * iu;
+  if constexpr ((kRole & kPhasePart) != 0) {
+    // C1 continuity of the phase: intermediate matched at Mf = 0.018, merger-ringdown at fRD/2
+    {
+      T f1 = lift<T>(kPhiJoinIns);
+      T u1 = dcbrt(f1);
+      T pI, dI, pN, dN;
+      {  // inspiral branch at the join (Mf = 0.018 itself belongs to the intermediate region)
+        T lu = dlog(u1);
+        T P = c.pin[11], R = c.pin[11] * 2.0;
+        for (int j = 10; j >= 0; --j) { P = P * u1 + c.pin[j]; R = R * u1 + c.pin[j] * ((j - 5) / 3.0); }
+        T iu = 1.0 / u1, iu2 = iu * iu, iu4 = iu2 * iu2;
+        pI = P * iu4 * iu + (c.lg0 + c.lg1 * u1) * lu;
+        dI = R * iu4 * iu4 + (c.lg1 * (lu + 1.0) * (1.0 / 3.0)) * iu2 + c.lg0 * (1.0 / 3.0) * iu2 * iu;
+      }
+      T if1 = 1.0 / f1;
+      pN = c.pint[1] * f1 + c.pint[2] * if1 * if1 * if1 + c.pint[3] * dlog(f1);
+      dN = c.pint[1] - 3.0 * c.pint[2] * if1 * if1 * if1 * if1 + c.pint[3] * if1;
+      T C2 = dI - dN;
+      T C1 = pI - pN - C2 * f1;
+      c.pint[0] = C1;
+      c.pint[1] = c.pint[1] + C2;
+      T f2 = 0.5 * c.fRD;
+      T if2 = 1.0 / f2;
+      T pI2 = c.pint[0] + c.pint[1] * f2 + c.pint[2] * if2 * if2 * if2 + c.pint[3] * dlog(f2);
+      T dI2 = c.pint[1] - 3.0 * c.pint[2] * if2 * if2 * if2 * if2 + c.pint[3] * if2;
+      T q2 = dsqrt(dsqrt(f2));
+      T x2 = f2 - c.pm[5];
+      T pM = c.pm[1] * f2 + c.pm[2] * if2 + c.pm[3] * (q2 * q2 * q2) + c.pm[4] * datan(x2 / c.fDM);
+      T dM = c.pm[1] - c.pm[2] * if2 * if2 + 0.75 * c.pm[3] / q2 + c.pm[4] * c.fDM / (c.fDM * c.fDM + x2 * x2);
+      T C2m = dI2 - dM;
+      c.pm[0] = pI2 - pM - C2m * f2;
+      c.pm[1] = c.pm[1] + C2m;
     }
-    T if1 = 1.0 / f1;
-    pN = c.pint[1] * f1 + c.pint[2] * if1 * if1 * if1 + c.pint[3] * dlog(f1);
-    dN = c.pint[1] - 3.0 * c.pint[2] * if1 * if1 * if1 * if1 + c.pint[3] * if1;
-    T C2 = dI - dN;
-    T C1 = pI - pN - C2 * f1;
-    c.pint[0] = C1;
-    c.pint[1] = c.pint[1] + C2;
-    T f2 = 0.5 * c.fRD;
-    T if2 = 1.0 / f2;
-    T pI2 = c.pint[0] + c.pint[1] * f2 + c.pint[2] * if2 * if2 * if2 + c.pint[3] * dlog(f2);
-    T dI2 = c.pint[1] - 3.0 * c.pint[2] * if2 * if2 * if2 * if2 + c.pint[3] * if2;
-    T q2 = dsqrt(dsqrt(f2));
-    T x2 = f2 - c.pm[5];
-    T pM = c.pm[1] * f2 + c.pm[2] * if2 + c.pm[3] * (q2 * q2 * q2) + c.pm[4] * datan(x2 / c.fDM);
-    T dM = c.pm[1] - c.pm[2] * if2 * if2 + 0.75 * c.pm[3] / q2 + c.pm[4] * c.fDM / (c.fDM * c.fDM + x2 * x2);
-    T C2m = dI2 - dM;
-    c.pm[0] = pI2 - pM - C2m * f2;
-    c.pm[1] = c.pm[1] + C2m;
   }
-  // intermediate amplitude: value/derivative at 0.014 and fpeak, value v2 midway
-  {
-    T f1 = lift<T>(kAmpJoinIns), f3 = c.fpeak, f2 = 0.5 * (f1 + f3);
-    T u1 = dcbrt(f1);
-    T u12 = u1 * u1;
-    T Ains = one + u12 * (c.ai[0] + u1 * (c.ai[1] + u1 * (c.ai[2] + u1 * (c.ai[3] + u1 * (c.ai[4] +
-                   u1 * (c.ai[5] + u1 * (c.ai[6] + u1 * c.ai[7])))))));
-    // dAhat/dMf = (1/(3u^2)) dAhat/du
-    T dAdu = u1 * (2.0 * c.ai[0] + u1 * (3.0 * c.ai[1] + u1 * (4.0 * c.ai[2] + u1 * (5.0 * c.ai[3] + u1 * (6.0 * c.ai[4] +
-                   u1 * (7.0 * c.ai[5] + u1 * (8.0 * c.ai[6] + u1 * 9.0 * c.ai[7])))))));
-    T dAins = dAdu / (3.0 * u12);
-    T x3 = f3 - c.fRD;
-    T den = x3 * x3 + c.g3fDM * c.g3fDM;
-    T Amrd = c.g1 * c.g3fDM / den * dexp(-c.g2 * x3 / c.g3fDM);
-    T dAmrd = Amrd * (-c.g2 / c.g3fDM - 2.0 * x3 / den);
-    T A[5][5], b[5];
-    T fs[3] = {f1, f2, f3};
-    for (int r = 0; r < 3; ++r) {
-      T pw = one;
-      for (int j = 0; j < 5; ++j) { A[r][j] = pw; pw = pw * fs[r]; }
+  if constexpr ((kRole & kAmpPart) != 0) {
+    // intermediate amplitude: value/derivative at 0.014 and fpeak, value v2 midway
+    {
+      T f1 = lift<T>(kAmpJoinIns), f3 = c.fpeak, f2 = 0.5 * (f1 + f3);
+      T u1 = dcbrt(f1);
+      T u12 = u1 * u1;
+      T Ains = one + u12 * (c.ai[0] + u1 * (c.ai[1] + u1 * (c.ai[2] + u1 * (c.ai[3] + u1 * (c.ai[4] +
+                     u1 * (c.ai[5] + u1 * (c.ai[6] + u1 * c.ai[7])))))));
+      // dAhat/dMf = (1/(3u^2)) dAhat/du
+      T dAdu = u1 * (2.0 * c.ai[0] + u1 * (3.0 * c.ai[1] + u1 * (4.0 * c.ai[2] + u1 * (5.0 * c.ai[3] + u1 * (6.0 * c.ai[4] +
+                     u1 * (7.0 * c.ai[5] + u1 * (8.0 * c.ai[6] + u1 * 9.0 * c.ai[7])))))));
+      T dAins = dAdu / (3.0 * u12);
+      T x3 = f3 - c.fRD;
+      T den = x3 * x3 + c.g3fDM * c.g3fDM;
+      T Amrd = c.g1 * c.g3fDM / den * dexp(-c.g2 * x3 / c.g3fDM);
+      T dAmrd = Amrd * (-c.g2 / c.g3fDM - 2.0 * x3 / den);
+      T A[5][5], b[5];
+      T fs[3] = {f1, f2, f3};
+      for (int r = 0; r < 3; ++r) {
+        T pw = one;
+        for (int j = 0; j < 5; ++j) { A[r][j] = pw; pw = pw * fs[r]; }
+      }
+      T fd[2] = {f1, f3};
+      for (int r = 0; r < 2; ++r) {
+        A[3 + r][0] = lift<T>(0.0);
+        A[3 + r][1] = one;
+        A[3 + r][2] = 2.0 * fd[r];
+        A[3 + r][3] = 3.0 * fd[r] * fd[r];
+        A[3 + r][4] = 4.0 * fd[r] * fd[r] * fd[r];
+      }
+      b[0] = Ains;
+      b[1] = v2;
+      b[2] = Amrd;
+      b[3] = dAins;
+      b[4] = dAmrd;
+      solve5(A, b, c.dl);
     }
-    T fd[2] = {f1, f3};
-    for (int r = 0; r < 2; ++r) {
-      A[3 + r][0] = lift<T>(0.0);
-      A[3 + r][1] = one;
-      A[3 + r][2] = 2.0 * fd[r];
-      A[3 + r][3] = 3.0 * fd[r] * fd[r];
-      A[3 + r][4] = 4.0 * fd[r] * fd[r] * fd[r];
-    }
-    b[0] = Ains;
-    b[1] = v2;
-    b[2] = Amrd;
-    b[3] = dAins;
-    b[4] = dAmrd;
-    solve5(A, b, c.dl);
   }
-  // alignment: t(fpeak) = 0 and Psi(f_ref) = -2 phi_c
-  {
-    T up = dcbrt(c.fpeak);
-    T pp, dp;
-    phenomd_phase(c, c.fpeak, up, pp, dp);
-    T t0 = dp;
-    T MfRef = c.Msec * f_ref;
-    T ur = dcbrt(MfRef);
-    T pr, dr;
-    phenomd_phase(c, MfRef, ur, pr, dr);
-    T shift = t0 * MfRef - pr - 2.0 * th[9];
-    // fold -t0 Mf + shift into every region
-    c.pin[5] = c.pin[5] + shift;
-    c.pin[8] = c.pin[8] - t0;
-    c.pint[0] = c.pint[0] + shift;
-    c.pint[1] = c.pint[1] - t0;
-    c.pm[0] = c.pm[0] + shift;
-    c.pm[1] = c.pm[1] - t0;
+  if constexpr ((kRole & kPhasePart) != 0) {
+    // alignment: t(fpeak) = 0 and Psi(f_ref) = -2 phi_c
+    {
+      T up = dcbrt(c.fpeak);
+      T pp, dp;
+      phenomd_phase(c, c.fpeak, up, pp, dp);
+      T t0 = dp;
+      T MfRef = c.Msec * f_ref;
+      T ur = dcbrt(MfRef);
+      T pr, dr;
+      phenomd_phase(c, MfRef, ur, pr, dr);
+      T shift = t0 * MfRef - pr - 2.0 * th[9];
+      // fold -t0 Mf + shift into every region
+      c.pin[5] = c.pin[5] + shift;
+      c.pin[8] = c.pin[8] - t0;
+      c.pint[0] = c.pint[0] + shift;
+      c.pint[1] = c.pint[1] - t0;
+      c.pm[0] = c.pm[0] + shift;
+      c.pm[1] = c.pm[1] - t0;
+    }
   }
   T DLm = dexp(th[4]) * (1.0e6 * kPc);
   // 2 sqrt(5/(64 pi)) M_m M_s / D * sqrt(2 eta / 3) pi^{-1/6}
@@ -785,32 +1123,35 @@ struct PhenomHMCoef {
   T eta, dlt, chis, chia;  // for the PN amplitude ratios
   T fRDmax;                // largest ringdown frequency of the modes (Mf)
   T v2;                    // the (2,2) intermediate amplitude collocation value
-  T ainsf1, dainsf1;       // the (2,2) inspiral amplitude and its Mf-derivative at Mf = 0.014
   HMMode<T> md[kHMModes];
 };
 
-PES_HD double hm_fact(int n) {
-  double r = 1.0;
-  for (int i = 2; i <= n; ++i) r *= i;
-  return r;
-}
+// Prefactors of the s = -2 harmonics' sums over k = 0, 1, 2 for (l, m) and
+// (l, -m) of each mode: sqrt((2l+1)/4pi) (-1)^k sqrt((l+m)! (l-m)! (l+2)! (l-2)!)
+// / ((l+m-k)! (l-2-k)! k! (k+2-m)!), 0 where a factorial has no value.
+__device__ static const double kHMHarm[kHMModes][2][3] = {
+    {{0.63078313050504, 0.0, 0.0}, {0.63078313050504, 0.0, 0.0}},
+    {{1.26156626101008, 0.0, 0.0}, {1.26156626101008, 0.0, 0.0}},
+    {{0.0, -1.8281831978578629, 0.0}, {1.8281831978578629, 0.0, 0.0}},
+    {{0.7463526651802308, -3.731763325901154, 0.0}, {3.731763325901154, -0.7463526651802308, 0.0}},
+    {{0.0, 0.0, 4.478115991081385}, {4.478115991081385, 0.0, 0.0}},
+    {{0.0, -3.166506184233564, 9.499518552700692}, {9.499518552700692, -3.166506184233564, 0.0}}};
 
-// s = -2 spherical harmonic at azimuth 0 from cos(iota): sqrt((2l+1)/4pi) d^l_{m,2}
+// s = -2 spherical harmonic at azimuth 0 of mode `mode` (sgn 0) or of its -m
+// (sgn 1) from ch = cos(iota / 2), sh = sin(iota / 2): sqrt((2l+1)/4pi) d^l_{m,2}
 template <class T>
-PES_HD T hm_sylm(int l, int m, const T& cosi) {
-  const T ch = dsqrt(0.5 * (1.0 + cosi)), sh = dsqrt(0.5 * (1.0 - cosi));
+PES_HD T hm_sylm(int mode, int sgn, const T& ch, const T& sh) {
+  const int l = kHMlm[mode][0], m = sgn ? -kHMlm[mode][1] : kHMlm[mode][1];
   T sum = lift<T>(0.0);
-  for (int k = 0; k <= l + m; ++k) {
-    if (l + m - k < 0 || l - 2 - k < 0 || k + 2 - m < 0) continue;
-    const double c = ((k & 1) ? -1.0 : 1.0) *
-                     ::sqrt(hm_fact(l + m) * hm_fact(l - m) * hm_fact(l + 2) * hm_fact(l - 2)) /
-                     (hm_fact(l + m - k) * hm_fact(l - 2 - k) * hm_fact(k) * hm_fact(k + 2 - m));
+  for (int k = 0; k < 3; ++k) {
+    const double c = kHMHarm[mode][sgn][k];
+    if (c == 0.0) continue;
     T term = lift<T>(c);
     for (int e = 0; e < 2 * l + m - 2 * k - 2; ++e) term = term * ch;
     for (int e = 0; e < 2 * k + 2 - m; ++e) term = term * sh;
     sum = sum + term;
   }
-  return ::sqrt((2.0 * l + 1.0) / (4.0 * kPi)) * sum;
+  return sum;
 }
 
 // Signed PN amplitude ratio beta_lm(v) (Blanchet 2014 eq. 327; leading spin term of (2,1))
@@ -947,130 +1288,106 @@ PES_HD void hm_kink(const PhenomDCoef<T>& c, const PhenomHMCoef<T>& h, int k, T&
   jump = md.Rholm * md.Rholm * (d2m - d2i) - ypp * (A * L1 - (7.0 / 6.0) * A / fp);
 }
 
-// The modes' coefficients from the (2,2) block c (already set up from th)
-// and the remnant spin af and radiated energy erad of that set-up.
+// The sample's constants that the modes share, from the (2,2) block c
+// (already set up from th); fRDmax of the (2,2) mode alone.
 template <class T>
-PES_HD void phenomhm_setup(const T* th, const PhenomDCoef<T>& c, PhenomHMCoef<T>& h) {
-  const T one = lift<T>(1.0);
-  const T af = c.af, erad = c.erad, eta = c.eta, v2 = c.v2;
+PES_HD void phenomhm_common(const T* th, const PhenomDCoef<T>& c, PhenomHMCoef<T>& h) {
   const T q = th[1];
-  h.eta = eta;
+  h.eta = c.eta;
   h.dlt = (q - 1.0) / (q + 1.0);
   h.chis = 0.5 * (th[2] + th[3]);
   h.chia = 0.5 * (th[2] - th[3]);
-  h.v2 = v2;
+  h.v2 = c.v2;
   h.fRDmax = c.fRD;
-  const double nrm = 2.0 * ::sqrt(5.0 / (64.0 * kPi));
-  const T f1 = lift<T>(kAmpJoinIns);
-  const T u1 = dcbrt(f1);
-  for (int k = 0; k < kHMModes; ++k) {
-    HMMode<T>& md = h.md[k];
-    const int l = kHMlm[k][0], m = kHMlm[k][1];
-    md.tm = lift<T>(2.0 / m);
-    md.hm = lift<T>(0.5 * m);
-    md.tpm = lift<T>(2.0 * kPi / m);
-    md.qt = lift<T>(kHMlm[k][2] * (0.5 * kPi));
-    const T Yp = hm_sylm<T>(l, m, th[5]), Ym = hm_sylm<T>(l, -m, th[5]);
-    const double sg = (l & 1) ? -1.0 : 1.0;
-    md.P = (sg * Ym + Yp) * (1.0 / (2.0 * nrm));
-    md.C = (sg * Ym - Yp) * (1.0 / (2.0 * nrm));
-    T wR, wI;
-    qnm_interp<T>(k, af, wR, wI);
-    md.fRD = wR / (2.0 * kPi) / (one - erad);
-    const T fDMlm = wI / (2.0 * kPi) / (one - erad);
-    if (val(md.fRD) > val(h.fRDmax)) h.fRDmax = md.fRD;
-    if (k == 0) {  // the (2,2) mode is PhenomD's, bit for bit
-      md.fRD = c.fRD;
-      md.Rholm = one;
-      md.fDMeff = c.fDM;
-      md.g3fDMeff = c.g3fDM;
-      md.fpeak = c.fpeak;
-      for (int j = 0; j < 5; ++j) md.dl[j] = c.dl[j];
-      md.fiA = f1;
-      md.frA = c.fpeak;
-      md.fiP = lift<T>(kPhiJoinIns);
-      md.frP = 0.5 * c.fRD;
-      md.aP = one;
-      md.bP = lift<T>(0.0);
-      md.cI0 = md.cI1 = md.cR0 = md.cR1 = lift<T>(0.0);
-      continue;
-    }
-    md.Rholm = c.fRD / md.fRD;
-    md.fDMeff = md.Rholm * fDMlm;
-    const T g3 = c.g3fDM / c.fDM;
-    md.g3fDMeff = g3 * md.fDMeff;
-    if (val(c.g2) <= 1.0)
-      md.fpeak = dabs(c.fRD + md.fDMeff * g3 * (dsqrt(one - c.g2 * c.g2) - 1.0) / c.g2);
-    else
-      md.fpeak = dabs(c.fRD - md.fDMeff * g3 / c.g2);
-    // intermediate amplitude with the mode's merger-ringdown
-    {
-      const T f3 = md.fpeak, f2 = 0.5 * (f1 + f3);
-      const T u12 = u1 * u1;
-      const T Ains = one + u12 * (c.ai[0] + u1 * (c.ai[1] + u1 * (c.ai[2] + u1 * (c.ai[3] + u1 * (c.ai[4] +
-                     u1 * (c.ai[5] + u1 * (c.ai[6] + u1 * c.ai[7])))))));
-      const T dAdu = u1 * (2.0 * c.ai[0] + u1 * (3.0 * c.ai[1] + u1 * (4.0 * c.ai[2] + u1 * (5.0 * c.ai[3] + u1 * (6.0 * c.ai[4] +
-                     u1 * (7.0 * c.ai[5] + u1 * (8.0 * c.ai[6] + u1 * 9.0 * c.ai[7])))))));
-      const T dAins = dAdu / (3.0 * u12);
-      const T x3 = f3 - c.fRD;
-      const T den = x3 * x3 + md.g3fDMeff * md.g3fDMeff;
-      const T Amrd = c.g1 * md.g3fDMeff / den * dexp(-c.g2 * x3 / md.g3fDMeff);
-      const T dAmrd = Amrd * (-c.g2 / md.g3fDMeff - 2.0 * x3 / den);
-      T A[5][5], b[5];
-      const T fs[3] = {f1, f2, f3};
-      for (int r = 0; r < 3; ++r) {
-        T pw = one;
-        for (int j = 0; j < 5; ++j) { A[r][j] = pw; pw = pw * fs[r]; }
-      }
-      const T fd[2] = {f1, f3};
-      for (int r = 0; r < 2; ++r) {
-        A[3 + r][0] = lift<T>(0.0);
-        A[3 + r][1] = one;
-        A[3 + r][2] = 2.0 * fd[r];
-        A[3 + r][3] = 3.0 * fd[r] * fd[r];
-        A[3 + r][4] = 4.0 * fd[r] * fd[r] * fd[r];
-      }
-      b[0] = Ains;
-      b[1] = v2;
-      b[2] = Amrd;
-      b[3] = dAins;
-      b[4] = dAmrd;
-      solve5(A, b, md.dl);
-    }
-    // maps
-    md.fiA = (0.5 * m) * f1;
-    md.frA = md.fpeak / md.Rholm;
-    md.fiP = lift<T>((0.5 * m) * kPhiJoinIns);
-    md.frP = (0.5 * c.fRD) / md.Rholm;
-    md.aP = (0.5 * c.fRD - kPhiJoinIns) / (md.frP - md.fiP);
-    md.bP = kPhiJoinIns - md.aP * md.fiP;
-    // C1 matching of the phase at fiP and frP
+}
+
+// Mode k's coefficients from the (2,2) block c.  The modes are independent:
+// the value set-up gives each to its own thread.  kRole as in phenomd_setup:
+// kAmpPart takes P .. frA (and fRD, tm .. qt), kPhasePart fiP .. cR1.
+template <class T, int kRole = 3>
+PES_HD void phenomhm_mode(const T* th, const PhenomDCoef<T>& c, int k, HMMode<T>& md) {
+  const T one = lift<T>(1.0);
+  constexpr double nrm = 0.31539156525252;  // 2 sqrt(5/(64 pi))
+  const int l = kHMlm[k][0], m = kHMlm[k][1];
+  md.tm = lift<T>(2.0 / m);
+  md.hm = lift<T>(0.5 * m);
+  md.tpm = lift<T>(2.0 * kPi / m);
+  md.qt = lift<T>(kHMlm[k][2] * (0.5 * kPi));
+  const T ch = dsqrt(0.5 * (1.0 + th[5])), sh = dsqrt(0.5 * (1.0 - th[5]));
+  const T Yp = hm_sylm<T>(k, 0, ch, sh), Ym = hm_sylm<T>(k, 1, ch, sh);
+  const double sg = (l & 1) ? -1.0 : 1.0;
+  md.P = (sg * Ym + Yp) * (1.0 / (2.0 * nrm));
+  md.C = (sg * Ym - Yp) * (1.0 / (2.0 * nrm));
+  if (k == 0) {  // the (2,2) mode is PhenomD's, bit for bit
+    md.fRD = c.fRD;
+    md.Rholm = one;
+    md.fDMeff = c.fDM;
+    md.g3fDMeff = c.g3fDM;
+    md.fpeak = c.fpeak;
+    for (int j = 0; j < 5; ++j) md.dl[j] = c.dl[j];
+    md.fiA = lift<T>(kAmpJoinIns);
+    md.frA = c.fpeak;
+    md.fiP = lift<T>(kPhiJoinIns);
+    md.frP = 0.5 * c.fRD;
+    md.aP = one;
+    md.bP = lift<T>(0.0);
     md.cI0 = md.cI1 = md.cR0 = md.cR1 = lift<T>(0.0);
-    T v1, d1, va, da;
-    {
-      const T f22 = (2.0 / m) * md.fiP;
-      phenomd_phase<T>(c, f22, dcbrt(f22), v1, d1);
-      v1 = (0.5 * m) * v1;
-    }
-    {
-      const T f22 = md.aP * md.fiP + md.bP;
-      phenomd_phase<T>(c, f22, dcbrt(f22), va, da);
-      va = va / md.aP;
-    }
-    md.cI1 = d1 - da;
-    md.cI0 = v1 - va - md.cI1 * md.fiP;
-    T vb, db, vr, dr;
-    {
-      const T f22 = md.aP * md.frP + md.bP;
-      phenomd_phase<T>(c, f22, dcbrt(f22), vb, db);
-      vb = vb / md.aP + md.cI0 + md.cI1 * md.frP;
-      db = db + md.cI1;
-    }
-    hm_psi_mrd<T>(c, md.fDMeff, md.Rholm * md.frP, vr, dr);
-    vr = vr / md.Rholm;
-    md.cR1 = db - dr;
-    md.cR0 = vb - vr - md.cR1 * md.frP;
+    return;
   }
+  T wR, wI;
+  qnm_interp<T>(k, c.af, wR, wI);
+  const T irem = (1.0 / (2.0 * kPi)) / (one - c.erad);
+  md.fRD = wR * irem;
+  const T fDMlm = wI * irem;
+  md.Rholm = c.fRD / md.fRD;
+  const T iR = md.fRD / c.fRD;
+  md.fDMeff = md.Rholm * fDMlm;
+  md.g3fDMeff = c.g3fDM / c.fDM * md.fDMeff;
+  if (val(c.g2) <= 1.0)
+    md.fpeak = dabs(c.fRD + md.g3fDMeff * (dsqrt(one - c.g2 * c.g2) - 1.0) / c.g2);
+  else
+    md.fpeak = dabs(c.fRD - md.g3fDMeff / c.g2);
+  // intermediate amplitude with the mode's merger-ringdown
+  if constexpr ((kRole & kAmpPart) != 0) {
+    T Ains, dAins, Amrd, dAmrd;
+    amp_join(c, Ains, dAins);
+    amp_mrd(c, md.g3fDMeff, md.fpeak, Amrd, dAmrd);
+    quartic_coef(lift<T>(kAmpJoinIns), md.fpeak, Ains, dAins, Amrd, dAmrd, c.v2, md.dl);
+  }
+  // maps
+  md.fiA = lift<T>((0.5 * m) * kAmpJoinIns);
+  md.frA = md.fpeak * iR;
+  md.fiP = lift<T>((0.5 * m) * kPhiJoinIns);
+  md.frP = (0.5 * c.fRD) * iR;
+  md.aP = (0.5 * c.fRD - kPhiJoinIns) / (md.frP - md.fiP);
+  md.bP = kPhiJoinIns - md.aP * md.fiP;
+  if constexpr ((kRole & kPhasePart) == 0) return;
+  // C1 matching of the phase at fiP and frP
+  T v1, d1, va, da;
+  const T iaP = (md.frP - md.fiP) / (0.5 * c.fRD - kPhiJoinIns);
+  {
+    const T f22 = (2.0 / m) * md.fiP;
+    phenomd_phase<T>(c, f22, dcbrt(f22), v1, d1);
+    v1 = (0.5 * m) * v1;
+  }
+  {
+    const T f22 = md.aP * md.fiP + md.bP;
+    phenomd_phase<T>(c, f22, dcbrt(f22), va, da);
+    va = va * iaP;
+  }
+  md.cI1 = d1 - da;
+  md.cI0 = v1 - va - md.cI1 * md.fiP;
+  T vb, db, vr, dr;
+  {
+    const T f22 = md.aP * md.frP + md.bP;
+    phenomd_phase<T>(c, f22, dcbrt(f22), vb, db);
+    vb = vb * iaP + md.cI0 + md.cI1 * md.frP;
+    db = db + md.cI1;
+  }
+  hm_psi_mrd<T>(c, md.fDMeff, md.Rholm * md.frP, vr, dr);
+  vr = vr * iR;
+  md.cR1 = db - dr;
+  md.cR0 = vb - vr - md.cR1 * md.frP;
 }
 
 }  // namespace pes

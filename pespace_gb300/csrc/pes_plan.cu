@@ -280,8 +280,7 @@ int run_dense(PesPlan* p, const double* theta, int64_t B, int pass, double* lnl,
   SampleBlock<T>* blocks = reinterpret_cast<SampleBlock<T>*>(p->blocks);
   {
     ProfScope ps(p, kKSetup, st);
-    k_setup<T><<<ceil_div(B, p->sample_threads), p->sample_threads, 0, st>>>(p->dev, theta, B, pass, blocks,
-                                                                            hm_blocks<T>(p));
+    k_setup<T><<<setup_blocks(B), 64, 0, st>>>(p->dev, theta, B, pass, blocks, hm_blocks<T>(p));
   }
   PES_CHECK_LAUNCH();
   const int nblk = (int)ceil_div(p->desc.nbins, kDenseBinsPerBlock);
@@ -482,7 +481,7 @@ int pes_plan_model_tdi(PesPlan* p, int32_t det, int32_t orthogonal, const double
     return PES_OK;
   }
   SampleBlock<double>* blocks = reinterpret_cast<SampleBlock<double>*>(p->blocks);
-  k_setup<double><<<1, 1, 0, st>>>(p->dev, d_theta, 1, 0, blocks, hm_blocks<double>(p));
+  k_setup<double><<<1, 64, 0, st>>>(p->dev, d_theta, 1, 0, blocks, hm_blocks<double>(p));
   PES_CHECK_LAUNCH();
   k_model_tdi<<<ceil_div(p->desc.nbins, 128), 128, 0, st>>>(p->dev, blocks, hm_blocks<double>(p), det, orthogonal != 0,
                                                             reinterpret_cast<double2*>(out));

@@ -1,6 +1,7 @@
 // Plan object shared by the batched-likelihood translation units.
 #pragma once
 
+#include <cstddef>
 #include <utility>
 #include <vector>
 
@@ -60,7 +61,7 @@ enum KernelClass : int {
   kKOther = 7,
 };
 
-// Threads per block of the per-sample kernels (set-up, ranges, kink): each
+// Threads per block of the one-thread-per-sample kernels (ranges, kink): each
 // thread runs a long FP64 chain, and GB300 issues FP64 at 2 lanes per cycle
 // per SM, so small blocks spread the samples over all SMs instead of
 // queueing 64 lanes on each SM's FP64 pipe.
@@ -210,48 +211,190 @@ __device__ __forceinline__ bool hm_mode_container(const SampleBlock<T>& b, const
   return true;
 }
 
+// The same cut from the quotient of the limits, adjusted to the predicate at
+// the neighbouring bins (a bisection's 17 probes each cost an FP64 conversion
+// and three FP64 operations of the set-up's serial chain); the bisection where
+// the quotient is not a number that is off by at most a few bins.
+PES_HD int64_t find_kcut_near(const PlanDev& P, double Msec, double fcut, double mf_max) {
+  if (!(Msec > 0.0) || !isfinite(Msec)) return find_kcut(P, Msec, fcut, mf_max);
+  const double kf = fmin(fcut, mf_max / Msec) / P.f_step;
+  const double top = (double)(P.k0 + P.nbins);
+  int64_t i = kf < (double)P.k0 ? 0 : (kf >= top ? P.nbins : (int64_t)kf - P.k0 + 1);
+  if (i > P.nbins) i = P.nbins;
+  auto live = [&](int64_t k) {
+    const double f = (double)(P.k0 + k) * P.f_step;
+    return (f <= fcut) && (Msec * f <= mf_max);
+  };
+  for (int n = 0; n < 4 && i > 0 && !live(i - 1); ++n) --i;
+  for (int n = 0; n < 4 && i < P.nbins && live(i); ++n) ++i;
+  if ((i > 0 && !live(i - 1)) || (i < P.nbins && live(i))) return find_kcut(P, Msec, fcut, mf_max);
+  return i;
+}
+
 // ------------------------------------------------------------------ kernels
-// hmb: the samples' IMRPhenomHM mode coefficients (IMRPhenomHM plans; may be null otherwise)
-template <class T>
-__global__ void k_setup(PlanDev P, const double* __restrict__ theta, int64_t B, int pass,
-                        SampleBlock<T>* __restrict__ blocks, PhenomHMCoef<T>* __restrict__ hmb) {
-  int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (s >= B) return;
+// Per-sample set-up by groups of kSetupLanes threads (phenomd_setup).  The
+// scalar each thread works in: FP64, or an FP64 dual number of one tangent,
+// that of its own lane.
+constexpr int kSetupLanes = 16;
+template <class T> struct LaneScalar { using type = double; };
+template <int N, class D, class V> struct LaneScalar<Dual<N, D, V>> {
+  static_assert(N <= kSetupLanes, "one lane per tangent");
+  using type = Dual<1>;
+};
+template <class T> struct ScalarStride { static constexpr int n = 1; };
+template <int N> struct ScalarStride<Dual<N>> { static constexpr int n = 1 + N; };
+// Scalars [k0, k1) of a lane's block of S into the same scalars of a block of T.
+template <class T, class S>
+__device__ __forceinline__ void lane_store(void* block, int lane, const void* src, int k0, int k1) {
+  constexpr int stride = ScalarStride<T>::n;
+  double* out = reinterpret_cast<double*>(block);
+  const S* x = reinterpret_cast<const S*>(src);
+#pragma unroll
+  for (int k = k0; k < k1; ++k) {
+    if constexpr (stride == 1) {
+      if (lane == 0) out[k] = x[k];
+    } else {
+      if (lane == 0) out[k * stride] = x[k].v;
+      if (lane < stride - 1) out[k * stride + 1 + lane] = x[k].d[0];
+    }
+  }
+}
+#define PES_SCALAR(B, S, f) ((int)(offsetof(B<S>, f) / sizeof(S)))
+
+// hmb: the samples' IMRPhenomHM mode coefficients (IMRPhenomHM plans; may be null otherwise).
+// A group of kSetupLanes lanes per sample and part: the fits side by side,
+// each lane's own tangent for dual numbers, each mode of a value set-up on its
+// own lane; warp 0 of a block takes the phase part of two samples, warp 1 (on
+// another SM partition, with an FP64 pipe of its own) their amplitude part and
+// cut.  Bound by the latency of one sample's FP64 chain (64 cycles per warp
+// instruction): one thread per sample took 75-83 us (double), 340 (Dual<4>)
+// and 614-746 us (Dual<11>).
+constexpr int kSetupSamples = 32 / kSetupLanes;  // samples per block
+template <class T, int kRole, bool kSerial>
+__device__ __forceinline__ void setup_part(const PlanDev& P, const double* __restrict__ raw, int pass, int lane,
+                                           unsigned mask, double (*rows)[3], SampleBlock<T>& b,
+                                           PhenomHMCoef<T>* __restrict__ ho) {
   constexpr int NT = NumTangents<T>::value;
+  using S = typename LaneScalar<T>::type;
+  S th[11];
+#pragma unroll
+  for (int j = 0; j < 11; ++j) th[j] = Seed<S>::make(raw[j], NT > 0 && lane < NT && j == pass * NT + lane ? 0 : -1);
+  PhenomDCoef<S> wf;
+  if constexpr (kSerial)
+    phenomd_setup_serial<S, kRole>(th, P.f_ref, rows, lane, kSetupLanes, mask, wf);
+  else
+    phenomd_setup<S, kRole>(th, P.f_ref, rows, lane, kSetupLanes, mask, wf);
+  constexpr int amp0 = PES_SCALAR(PhenomDCoef, S, amp_scale), pin0 = PES_SCALAR(PhenomDCoef, S, pin),
+                pfac0 = PES_SCALAR(PhenomDCoef, S, pfac), end = (int)(sizeof(PhenomDCoef<S>) / sizeof(S));
+  constexpr int fi0 = PES_SCALAR(HMMode, S, fiP), frd0 = PES_SCALAR(HMMode, S, fRD),
+                hend = (int)(sizeof(HMMode<S>) / sizeof(S));
+  const bool hm = P.approximant == PES_APPROX_PHENOMHM;
+  if constexpr (kRole == kPhasePart) {
+    lane_store<T, S>(&b.wf, lane, &wf, 0, amp0);
+    lane_store<T, S>(&b.wf, lane, &wf, pin0, pfac0);
+    if (!hm) return;
+    if constexpr (NT == 0) {  // a mode per lane
+      if (lane < kHMModes) {
+        HMMode<S> md;
+        phenomhm_mode<S, kRole>(th, wf, lane, md);
+        lane_store<T, S>(&ho->md[lane], 0, &md, fi0, frd0);
+      }
+    } else {
+#pragma unroll 1
+      for (int k = 0; k < kHMModes; ++k) {
+        HMMode<S> md;
+        phenomhm_mode<S, kRole>(th, wf, k, md);
+        lane_store<T, S>(&ho->md[k], lane, &md, fi0, frd0);
+      }
+    }
+    return;
+  }
+  lane_store<T, S>(&b.wf, lane, &wf, amp0, pin0);
+  lane_store<T, S>(&b.wf, lane, &wf, pfac0, end);
+  {
+    Polar<S> pol;
+    const S sb = th[7];
+    const S cb = dsqrt((1.0 - sb) * (1.0 + sb));
+    make_polar<S>(th[6], sb, cb, th[8], pol);
+    lane_store<T, S>(&b.pol, lane, &pol, 0, (int)(sizeof(pol) / sizeof(S)));
+    lane_store<T, S>(&b.tc, lane, &th[10], 0, 1);
+  }
+  const double Msec = val(wf.Msec);
+  double frd = val(wf.fRD), iR = 1.0;  // the largest ringdown frequency of the modes, and 1 / Rholm
+  if (hm) {
+    PhenomHMCoef<S> h;
+    phenomhm_common<S>(th, wf, h);
+    if constexpr (NT == 0) {
+      if (lane < kHMModes) {
+        HMMode<S> md;
+        phenomhm_mode<S, kRole>(th, wf, lane, md);
+        lane_store<T, S>(&ho->md[lane], 0, &md, 0, fi0);
+        lane_store<T, S>(&ho->md[lane], 0, &md, frd0, hend);
+        frd = md.fRD;
+        iR = 1.0 / md.Rholm;
+      }
+#pragma unroll
+      for (int o = kSetupLanes / 2; o > 0; o >>= 1) {
+        const double f2 = __shfl_xor_sync(mask, frd, o), r2 = __shfl_xor_sync(mask, iR, o);
+        frd = f2 > frd ? f2 : frd;
+        iR = r2 > iR ? r2 : iR;
+      }
+      h.fRDmax = frd;
+    } else {
+#pragma unroll 1
+      for (int k = 0; k < kHMModes; ++k) {
+        HMMode<S> md;
+        phenomhm_mode<S, kRole>(th, wf, k, md);
+        lane_store<T, S>(&ho->md[k], lane, &md, 0, fi0);
+        lane_store<T, S>(&ho->md[k], lane, &md, frd0, hend);
+        if (val(md.fRD) > val(h.fRDmax)) h.fRDmax = md.fRD;
+        const double r2 = 1.0 / val(md.Rholm);
+        iR = r2 > iR ? r2 : iR;
+      }
+      frd = val(h.fRDmax);
+    }
+    lane_store<T, S>(ho, lane, &h, 0, PES_SCALAR(PhenomHMCoef, S, md));
+  }
+  if (lane == 0) {
+    const double fmax = (double)(P.k0 + P.nbins - 1) * P.f_step + 1.0;
+    double fcut = fmax;
+    // the model's cut: cut_factor times the largest ringdown frequency of its modes
+    if (P.cut_factor > 0.0) fcut = fmin(fmax, P.cut_factor * frd / Msec);
+    b.fcut = fcut;
+    // PhenomD: zero above Mf = 0.2; HM: each mode above its mapped Mf = 0.2
+    b.kcut = find_kcut_near(P, Msec, fcut, kMfCut * iR);
+    b.status = kSampleOk;
+  }
+}
+
+template <class T, bool kSerial = false>
+__global__ void __launch_bounds__(64) k_setup(PlanDev P, const double* __restrict__ theta, int64_t B, int pass,
+                        SampleBlock<T>* __restrict__ blocks, PhenomHMCoef<T>* __restrict__ hmb) {
+  __shared__ double rows[64 / kSetupLanes][kFCount][3];
+  const int lane = threadIdx.x % kSetupLanes, grp = threadIdx.x / kSetupLanes;
+  const unsigned mask = ((1u << kSetupLanes) - 1u) << ((threadIdx.x & 31) / kSetupLanes * kSetupLanes);
+  const int64_t s = blockIdx.x * (int64_t)kSetupSamples + grp % kSetupSamples;
+  if (s >= B) return;
   double raw[11];
   for (int j = 0; j < 11; ++j) raw[j] = theta[11 * s + j];
   SampleBlock<T>& b = blocks[s];
+  const bool phase = threadIdx.x < 32;
   if (!theta_in_domain(raw)) {
-    b.status = kSampleOutOfDomain;
-    b.kcut = 0;
-    b.fcut = 0.0;
+    if (lane == 0 && !phase) {
+      b.status = kSampleOutOfDomain;
+      b.kcut = 0;
+      b.fcut = 0.0;
+    }
     return;
   }
-  T th[11];
-  for (int j = 0; j < 11; ++j) th[j] = Seed<T>::make(raw[j], NT > 0 ? j - pass * NT : -1);
-  phenomd_setup<T>(th, P.f_ref, b.wf);
-  const bool hm = P.approximant == PES_APPROX_PHENOMHM;
-  if (hm) phenomhm_setup<T>(th, b.wf, hmb[s]);
-  T sb = th[7];
-  T cb = dsqrt((1.0 - sb) * (1.0 + sb));
-  make_polar<T>(th[6], sb, cb, th[8], b.pol);
-  b.tc = th[10];
-  const double Msec = val(b.wf.Msec);
-  const double fmax = (double)(P.k0 + P.nbins - 1) * P.f_step + 1.0;
-  double fcut = fmax;
-  // the model's cut: cut_factor times the largest ringdown frequency of its modes
-  const double frd = hm ? val(hmb[s].fRDmax) : val(b.wf.fRD);
-  if (P.cut_factor > 0.0) fcut = fmin(fmax, P.cut_factor * frd / Msec);
-  b.fcut = fcut;
-  double mf_max = kMfCut;  // PhenomD: zero above Mf = 0.2; HM: each mode above its mapped Mf = 0.2
-  if (hm)
-    for (int k = 1; k < kHMModes; ++k) {
-      const double mk = kMfCut / val(hmb[s].md[k].Rholm);
-      mf_max = mk > mf_max ? mk : mf_max;
-    }
-  b.kcut = find_kcut(P, Msec, fcut, mf_max);
-  b.status = kSampleOk;
+  PhenomHMCoef<T>* ho = hmb ? hmb + s : nullptr;
+  if (phase)
+    setup_part<T, kPhasePart, kSerial>(P, raw, pass, lane, mask, rows[grp], b, ho);
+  else
+    setup_part<T, kAmpPart, kSerial>(P, raw, pass, lane, mask, rows[grp], b, ho);
 }
+
+inline unsigned setup_blocks(int64_t B) { return ceil_div(B, kSetupSamples); }
 
 
 // out[k] = sum_{i >= k} row[i] for k = 0..n (FP64, fixed order; set-up only)

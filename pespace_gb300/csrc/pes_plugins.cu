@@ -161,7 +161,12 @@ struct ThetaArg {
 __global__ void k_phenomd(ThetaArg th, double f_ref, double f_cut, const double* __restrict__ freqs, int64_t n,
                           double2* __restrict__ hp, double2* __restrict__ hc, double* __restrict__ tf) {
   __shared__ PhenomDCoef<double> c;
-  if (threadIdx.x == 0) phenomd_setup<double>(th.v, f_ref, c);
+  __shared__ double rows[kFCount][3];
+  if (threadIdx.x < 32) {
+    PhenomDCoef<double> own;
+    phenomd_setup<double>(th.v, f_ref, rows, threadIdx.x, 32, 0xffffffffu, own);
+    if (threadIdx.x == 0) c = own;
+  }
   __syncthreads();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -189,9 +194,15 @@ __global__ void k_phenomhm(ThetaArg th, double f_ref, double f_cut, const double
                            double2* __restrict__ hp, double2* __restrict__ hc, double* __restrict__ tf) {
   __shared__ PhenomDCoef<double> c;
   __shared__ PhenomHMCoef<double> h;
-  if (threadIdx.x == 0) {
-    phenomd_setup<double>(th.v, f_ref, c);
-    phenomhm_setup<double>(th.v, c, h);
+  __shared__ double rows[kFCount][3];
+  if (threadIdx.x < 32) {
+    PhenomDCoef<double> own;
+    phenomd_setup<double>(th.v, f_ref, rows, threadIdx.x, 32, 0xffffffffu, own);
+    if (threadIdx.x == 0) {
+      c = own;
+      phenomhm_common<double>(th.v, own, h);
+    }
+    if (threadIdx.x < kHMModes) phenomhm_mode<double>(th.v, own, threadIdx.x, h.md[threadIdx.x]);
   }
   __syncthreads();
   const int k = blockIdx.y;

@@ -7,8 +7,8 @@ atomics may sum in another order):
   each run's inputs one run ahead into shared memory, or loads them
   directly.  Copying wins when the inputs stream from DRAM; direct loads win
   when they sit in L2.  The default is a size threshold (64 MB).
-* ``sample_threads``: threads per block of the per-sample kernels (set-up,
-  ranges, peak kink), whose FP64 chains run one per sample.
+* ``sample_threads``: threads per block of the one-thread-per-sample kernels
+  of the mixed plan (exact-bin ranges, peak kink).
 
 ``autotune`` searches one option at a time (the others held at their current
 values).  It times every candidate on the caller's batch with CUDA events on
