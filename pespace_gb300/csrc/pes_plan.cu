@@ -1,6 +1,7 @@
 // Batched lnL / lnL+gradient plans: set-up, data ingestion and the dense FP64
-// path (every bin evaluated in FP64: waveform -> links -> TDI -> residual,
-// fused, with a deterministic two-pass reduction per sample).
+// path of IMRPhenomHM (every bin evaluated in FP64: waveform -> links -> TDI ->
+// residual, fused, with a deterministic two-pass reduction per sample).
+// IMRPhenomD plans: pes_fp64.cu.
 #include <cstring>
 #include <cmath>
 #include <cstdlib>
@@ -51,44 +52,6 @@ __device__ __forceinline__ T bin_residual_hm(const PlanDev& P, const SampleBlock
   return sum;
 }
 
-// Model (A/E/T) of every detector at one dense bin, accumulated into the
-// residual sum sum_det sum_c |d - h|^2 w.
-template <class T>
-__device__ __forceinline__ T bin_residual(const PlanDev& P, const SampleBlock<T>& b, const PhenomHMCoef<T>* h,
-                                          int64_t i) {
-  if (P.approximant == PES_APPROX_PHENOMHM) return bin_residual_hm<T>(P, b, *h, i);
-  const double f = (double)(P.k0 + i) * P.f_step;
-  T Mf = b.wf.Msec * f;
-  T amp, psi, tf;
-  phenomd_eval<T>(b.wf, Mf, amp, psi, tf);
-  T s, c;
-  dsincos(psi, &s, &c);
-  T ap = b.wf.pfac * amp, ac = b.wf.cfac * amp;
-  Cx<T> hp = cx(ap * c, -(ap * s));
-  Cx<T> hc = cx(-(ac * s), -(ac * c));
-  Cx<T> ts;
-  dsincos((-2.0 * kPi * f) * b.tc, &ts.im, &ts.re);
-  hp = cmul(hp, ts);
-  hc = cmul(hc, ts);
-  T tft = tf + b.tc;
-  T sum = lift<T>(0.0);
-  for (int d = 0; d < P.n_det; ++d) {
-    Cx<T> L[6], C[3];
-    single_links<T>(P.orbit[d], f, hp, hc, tft, b.pol, L);
-    const TdiFactor dp = P.tdi[d * P.nbins + i];
-    tdi_channels<T>(cx(dp.dre, dp.dim), cx(dp.pre, dp.pim), 1, L, C);
-#pragma unroll
-    for (int ch = 0; ch < 3; ++ch) {
-      if (!((P.chan_mask >> ch) & 1)) continue;
-      const size_t off = ((size_t)d * 3 + ch) * P.nbins + i;
-      const double2 dv = P.data[off];
-      T rr = dv.x - C[ch].re, ri = dv.y - C[ch].im;
-      sum = sum + (rr * rr + ri * ri) * P.w[off];
-    }
-  }
-  return sum;
-}
-
 template <class T>
 __global__ void __launch_bounds__(kDenseThreads) k_dense_fp64(PlanDev P, const SampleBlock<T>* __restrict__ blocks,
                                                               const PhenomHMCoef<T>* __restrict__ hmb, int nblk,
@@ -110,7 +73,7 @@ __global__ void __launch_bounds__(kDenseThreads) k_dense_fp64(PlanDev P, const S
 #pragma unroll 1
     for (int j = 0; j < kDenseBinsPerThread; ++j) {
       const int64_t i = base + (int64_t)j * kDenseThreads;
-      if (i < sb.kcut) acc = acc + bin_residual<T>(P, sb, hmb ? hmb + s : nullptr, i);
+      if (i < sb.kcut) acc = acc + bin_residual_hm<T>(P, sb, hmb[s], i);
     }
   }
   double v[NV];
@@ -354,7 +317,7 @@ int pes_plan_create(const PesPlanDesc* desc, PesPlan** out) {
   if (e == cudaSuccess) e = cudaMalloc(&p->blocks, p->blocks_bytes);
   if (e == cudaSuccess && desc->approximant == PES_APPROX_PHENOMHM)  // the largest scalar: the Fisher duals
     e = cudaMalloc(&p->hm_blocks, (size_t)B * sizeof(PhenomHMCoef<Dual<11>>));
-  if (e == cudaSuccess && desc->precision == PES_PRECISION_FP64)
+  if (e == cudaSuccess && desc->precision == PES_PRECISION_FP64 && desc->approximant == PES_APPROX_PHENOMHM)
     e = cudaMalloc(&p->partial, sizeof(double) * p->partial_len);
   if (e == cudaSuccess) e = cudaMalloc(&p->status, sizeof(int32_t) * B);
   if (e != cudaSuccess) {
@@ -375,6 +338,13 @@ int pes_plan_create(const PesPlanDesc* desc, PesPlan** out) {
       return rc;
     }
   }
+  if (desc->precision == PES_PRECISION_FP64 && desc->approximant == PES_APPROX_PHENOMD) {
+    int rc = fp64_create(p);
+    if (rc != PES_OK) {
+      pes_plan_destroy(p);
+      return rc;
+    }
+  }
   *out = p;
   return PES_OK;
 }
@@ -387,6 +357,7 @@ int pes_plan_destroy(PesPlan* p) {
   }
   for (auto e : p->prof.pool) cudaEventDestroy(e);
   if (p->mixed) mixed_destroy(p);
+  if (p->fp64) fp64_destroy(p);
   cudaFree(p->fisher_blocks);
   cudaFree(p->fisher_partial);
   cudaFree(p->data);
@@ -440,6 +411,7 @@ int pes_lnl_batch(PesPlan* p, const double* theta, int64_t B, double* lnl, int32
   if (B == 0) return PES_OK;
   cudaStream_t st = as_stream(stream);
   if (p->desc.precision == PES_PRECISION_MIXED) return mixed_lnl(p, theta, B, lnl, nullptr, status, st);
+  if (p->fp64) return fp64_lnl(p, theta, B, lnl, nullptr, status, st);
   return run_dense<double>(p, theta, B, 0, lnl, nullptr, status, st);
 }
 
@@ -451,6 +423,7 @@ int pes_lnl_grad_batch(PesPlan* p, const double* theta, int64_t B, double* lnl, 
   if (B == 0) return PES_OK;
   cudaStream_t st = as_stream(stream);
   if (p->desc.precision == PES_PRECISION_MIXED) return mixed_lnl(p, theta, B, lnl, grad, status, st);
+  if (p->fp64) return fp64_lnl(p, theta, B, lnl, grad, status, st);
   constexpr int NT = kGradTangents;
   for (int pass = 0; pass * NT < 11; ++pass) {
     rc = run_dense<Dual<NT>>(p, theta, B, pass, lnl, grad, status, st);

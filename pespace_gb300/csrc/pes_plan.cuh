@@ -48,6 +48,8 @@ struct SampleBlock {
 
 // Mixed-precision plan buffers (allocated only for PES_PRECISION_MIXED).
 struct MixedBuffers;
+// Buffers of FP64 IMRPhenomD plans (pes_fp64.cu).
+struct Fp64Buffers;
 
 // Kernel classes for the measurement hooks.
 enum KernelClass : int {
@@ -105,6 +107,7 @@ struct PesPlan {
   int32_t* status = nullptr;   // [max_batch] internal status when the caller passes NULL
   unsigned data_set_mask = 0;
   pes::MixedBuffers* mixed = nullptr;
+  pes::Fp64Buffers* fp64 = nullptr;
   int sample_threads = pes::kPerSampleThreads;  // block size of the per-sample lnL kernels (PES_OPT_SAMPLE_THREADS)
   void* fisher_blocks = nullptr;     // [max_batch] SampleBlock<Dual<11>> (first Fisher call)
   double* fisher_partial = nullptr;  // [max_batch][blocks][66]
@@ -400,6 +403,10 @@ inline unsigned setup_blocks(int64_t B) { return ceil_div(B, kSetupSamples); }
 // out[k] = sum_{i >= k} row[i] for k = 0..n (FP64, fixed order; set-up only)
 void suffix_sum(int64_t n, const double* row, double* out, cudaStream_t st);
 
+int fp64_create(PesPlan* p);
+void fp64_destroy(PesPlan* p);
+int fp64_lnl(PesPlan* p, const double* theta, int64_t B, double* lnl, double* grad, int32_t* status,
+             cudaStream_t st);
 int mixed_create(PesPlan* p);
 void mixed_destroy(PesPlan* p);
 int mixed_ingest(PesPlan* p, int det, const double* data, const double* psd, cudaStream_t st);
