@@ -506,11 +506,22 @@ static int launch_td_tdi(const TdLayout& lay, const double* links, int64_t B, in
 // the FP32 pipe.  Each block scales its window by a power of two (its largest
 // exponent to 2^0, exact) and splits every double into a float-float pair from
 // the bits alone (integer operations: the FP64 pipe is not used on the way
-// in); interpolations, sums and the A/E/T combination run in float-float
-// (about 2^-46 of the operands per operation); each channel goes back to a
-// double from the bits and one FP64 add.  Scaled magnitudes below 2^-126
-// (2^-126 of the window's largest link sample) flush to zero; a NaN or an
-// infinity among the inputs gives NaN in the outputs that read it.
+// in).  Every delay that a channel applies to one link it applies with the
+// opposite sign to another, to links 13 and 12 (difference P) or 31 and 21 (Q)
+// for X and cyclically for Y and Z:
+//   X = P + D1 Q - D2 P - D3 Q  [- D4 P - D5 Q + D6 P + D7 Q, TDI 2.0],
+// so a block forms the six differences (and those of neighbouring samples)
+// once per window sample and a channel interpolates 3 or 7 terms instead of 6
+// or 14.  Each channel goes back to a double from the
+// bits and one FP64 add.  Scaled magnitudes below 2^-126 (2^-126 of the
+// window's largest link sample), and the tails of those below 2^-74, flush to
+// zero; a NaN or an infinity among the inputs gives NaN in the outputs that
+// read it.
+//
+// The FP32 pipe binds: about 430 operations of the sums, 200 of the window and
+// 60 of the way out per sample.  8 388 609 samples, TDI 2.0, A/E/T: 682 us with
+// 14 interpolated terms per channel and loads link by link, 476 us with the
+// differences, 338 us with all of a block's loads in flight (1.8 TB/s).
 struct TdLayoutFF {
   int max_delay;
   int64_t added;
@@ -536,30 +547,62 @@ static void td_layout_ff(const TdLayout& lay, TdLayoutFF& out) {
   out.rs3 = ff_pair(1.0 / std::sqrt(3.0));
 }
 
-// x * 2^-scale as a float-float pair: head = sign, exponent and the top 23
-// fraction bits; tail = the other 29 fraction bits, normalised (truncated to
-// 24 significant bits).
-__device__ __forceinline__ FF td_split(double x, int scale) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const unsigned sign = (unsigned)(b >> 32) & 0x80000000u;
-  const int E = (int)((b >> 52) & 0x7FF);
-  if (E == 0x7FF) return ff_make(__uint_as_float(0x7fc00000u), 0.0f);
-  const int e = E - 1023 - scale;
-  if (E == 0 || e < -126) return ff_make(0.0f, 0.0f);
-  const unsigned long long m = b & 0xFFFFFFFFFFFFFull;
-  const float hi = __uint_as_float(sign | ((unsigned)(e + 127) << 23) | (unsigned)(m >> 29));
-  const unsigned r = (unsigned)(m & 0x1FFFFFFFull);
-  float lo = 0.0f;
-  if (r != 0u) {
-    const int lz = __clz((int)r);    // r < 2^29: 3 <= lz <= 31
-    const int el = e - 52 + 31 - lz;  // exponent of r's leading bit
-    if (el >= -126) {
-      const unsigned frac = (unsigned)((((unsigned long long)r << (lz + 1)) & 0xFFFFFFFFull) >> 9);
-      lo = __uint_as_float(sign | ((unsigned)(el + 127) << 23) | frac);
-    }
-  }
-  return ff_make(hi, lo);
+// The scaling of a block's window, x -> x * 2^-scale: limits on the high word
+// of |x| and the exponent's shift.
+struct TdScale {
+  unsigned rebias;        // (896 + scale) << 23
+  unsigned head0, tail0;  // high words from which x * 2^-scale is at least 2^-126 (and x normal), 2^-74
+};
+__device__ __forceinline__ TdScale td_scale(int scale) {
+  TdScale s;
+  s.rebias = (unsigned)(896 + scale) << 23;
+  s.head0 = (unsigned)max(1, 1023 - 126 + scale) << 20;
+  s.tail0 = (unsigned)max(1, 1023 - 74 + scale) << 20;
+  return s;
 }
+
+// x * 2^-scale as a float-float pair: head = sign, exponent and the top 23
+// fraction bits (the exponent's low 9 bits, shifted modulo 2^32); tail = the
+// other 29 fraction bits, rounded to 24 significant bits, times the head's
+// power of two.
+__device__ __forceinline__ FF td_split(double x, const TdScale& s) {
+  const unsigned H = (unsigned)__double2hiint(x), L = (unsigned)__double2loint(x);
+  const unsigned a = H & 0x7fffffffu, sign = H & 0x80000000u;
+  unsigned hb = (__funnelshift_l(L, H, 3) - s.rebias) | sign;
+  const float pw = __uint_as_float((hb & 0xff800000u) - (52u << 23));  // +-2^(e - 52)
+  float lo = __uint2float_rn(L & 0x1fffffffu) * pw;
+  lo = a < s.tail0 ? 0.0f : lo;
+  hb = a < s.head0 ? 0u : hb;
+  hb = a >= 0x7ff00000u ? 0x7fc00000u : hb;
+  return ff_make(__uint_as_float(hb), lo);
+}
+
+// global to shared memory, 8 bytes (bytes = 0: zeros)
+__device__ __forceinline__ void td_copy8(void* smem, const void* gmem, int bytes) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(a), "l"(gmem), "r"(bytes) : "memory");
+}
+
+// A channel's running sum: heads added exactly (two_sum), the errors and tails
+// in lo, folded into the head after each delay.
+struct TdSum {
+  float hi, lo;
+  __device__ __forceinline__ void add(float h, float l) {
+    const FF s = ff_two_sum(hi, h);
+    hi = s.hi;
+    lo = (lo + s.lo) + l;
+  }
+  __device__ __forceinline__ void renorm() {
+    const FF s = ff_fast_two_sum(hi, lo);
+    hi = s.hi;
+    lo = s.lo;
+  }
+  // + d * f
+  __device__ __forceinline__ void fma(const FF& d, float fh, float fl) {
+    const float p = d.hi * fh;
+    add(p, fmaf(d.lo, fh, fmaf(d.hi, fl, fmaf(d.hi, fh, -p))));
+  }
+};
 
 // float f * 2^scale as a double, from the bits
 __device__ __forceinline__ double td_widen(float f, int scale) {
@@ -579,7 +622,7 @@ __global__ void __launch_bounds__(kTdThreads) k_td_tdi_ff(TdLayoutFF lay, const 
                                                           int64_t n_ext, int64_t n, int orth,
                                                           double* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char td_raw[];
-  const int64_t win = kTdTile + lay.added + 1;
+  const int win = kTdTile + (int)lay.added + 1;  // at most kTdMaxWindow
   FF* val = reinterpret_cast<FF*>(td_raw);  // [6][win]: the doubles first, then their float-float pairs
   FF* dif = val + 6 * win;                  // [6][win]: right - left
   double* raw = reinterpret_cast<double*>(td_raw);
@@ -587,17 +630,24 @@ __global__ void __launch_bounds__(kTdThreads) k_td_tdi_ff(TdLayoutFF lay, const 
   const double* src = links + (int64_t)blockIdx.y * 6 * n_ext;
   double* dst = out + (int64_t)blockIdx.y * 3 * n;
   const int64_t i0 = (int64_t)blockIdx.x * kTdTile;
-  const int64_t avail = n_ext - i0;
-  int emax = 0;  // largest finite biased exponent in the window
+  const int avail = (int)min((int64_t)win, n_ext - i0);
+  // all of a thread's loads in flight at once (in turn per link, they took a
+  // third of the block's time)
 #pragma unroll 1
-  for (int l = 0; l < 6; ++l) {
-    const double* s = src + (int64_t)l * n_ext + i0;
-    double* w = raw + l * win;
-#pragma unroll 4
-    for (int64_t j = threadIdx.x; j < win; j += kTdThreads) {
-      const double x = j < avail ? __ldg(s + j) : 0.0;
-      w[j] = x;
-      const int E = (int)(((unsigned long long)__double_as_longlong(x) >> 52) & 0x7FF);
+  for (int j = threadIdx.x; j < win; j += kTdThreads) {
+#pragma unroll
+    for (int l = 0; l < 6; ++l) {
+      const bool in = j < avail;
+      td_copy8(raw + l * win + j, src + l * n_ext + i0 + (in ? j : 0), in ? 8 : 0);
+    }
+  }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  int emax = 0;  // largest finite biased exponent in the window (each thread's own slots)
+#pragma unroll 1
+  for (int j = threadIdx.x; j < win; j += kTdThreads) {
+#pragma unroll
+    for (int l = 0; l < 6; ++l) {
+      const int E = (__double2hiint(raw[l * win + j]) >> 20) & 0x7FF;
       if (E != 0x7FF) emax = max(emax, E);
     }
   }
@@ -607,46 +657,54 @@ __global__ void __launch_bounds__(kTdThreads) k_td_tdi_ff(TdLayoutFF lay, const 
 #pragma unroll
   for (int w = 0; w < kTdThreads / 32; ++w) emax = max(emax, wmax[w]);
   const int scale = emax - 1023;  // the window's largest magnitude maps into [1, 2)
-  // each thread rewrites the slots it loaded: doubles -> float-float pairs in place
+  const TdScale sc = td_scale(scale);
+  // each thread rewrites the slots it loaded: the six links become, for channel
+  // c, the differences P (slot 2c) and Q (slot 2c + 1), in place
 #pragma unroll 1
-  for (int l = 0; l < 6; ++l) {
-    double* w = raw + l * win;
-    FF* v = val + l * win;
-#pragma unroll 4
-    for (int64_t j = threadIdx.x; j < win; j += kTdThreads) v[j] = td_split(w[j], scale);
+  for (int j = threadIdx.x; j < win; j += kTdThreads) {
+    FF l[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) l[k] = td_split(raw[k * win + j], sc);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      val[2 * c * win + j] = l[(5 + 2 * c) % 6] - l[2 * c];
+      val[(2 * c + 1) * win + j] = l[(4 + 2 * c) % 6] - l[2 * c + 1];
+    }
   }
   __syncthreads();
 #pragma unroll 1
-  for (int l = 0; l < 6; ++l) {
-    const FF* v = val + l * win;
-    FF* df = dif + l * win;
-#pragma unroll 4
-    for (int64_t j = threadIdx.x; j + 1 < win; j += kTdThreads) df[j] = v[j + 1] - v[j];
+  for (int j = threadIdx.x; j + 1 < win; j += kTdThreads) {
+#pragma unroll
+    for (int l = 0; l < 6; ++l) dif[l * win + j] = val[l * win + j + 1] - val[l * win + j];
   }
   __syncthreads();
-  constexpr int kTerms = kMaxDelay + 1;
-  constexpr int xp[8] = {5, 4, 0, 1, 0, 1, 5, 4};
-  constexpr int xm[8] = {0, 1, 5, 4, 5, 4, 0, 1};
 #pragma unroll 1
   for (int r = 0; r < kTdTile / kTdThreads; ++r) {
-    const int64_t t = threadIdx.x + r * kTdThreads;
+    const int t = threadIdx.x + r * kTdThreads;
     const int64_t i = i0 + t;
     if (i >= n) break;
-    auto term = [&](int l, int k) -> FF {
-      if (k < 0) return val[l * win + t + lay.added];
-      const int64_t o = l * win + t + lay.shift[k];
-      const float2 f = lay.frac[k];
-      return val[o] + dif[o] * ff_make(f.x, f.y);
-    };
     FF ch[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      FF acc = term((xp[0] + 2 * c) % 6, -1);
+      const FF v0 = val[2 * c * win + t + (int)lay.added];
+      TdSum acc;
+      acc.hi = v0.hi;
+      acc.lo = v0.lo;
 #pragma unroll
-      for (int j = 1; j < kTerms; ++j) acc = acc + term((xp[j] + 2 * c) % 6, j - 1);
-#pragma unroll
-      for (int j = 0; j < kTerms; ++j) acc = acc - term((xm[j] + 2 * c) % 6, j - 1);
-      ch[c] = acc;
+      for (int k = 0; k < kMaxDelay; ++k) {
+        const int o = (2 * c + 1 - (k & 1)) * win + t + (int)lay.shift[k];
+        const FF v = val[o], d = dif[o];
+        const float2 f = lay.frac[k];
+        if (k == 0 || k > 4) {
+          acc.add(v.hi, v.lo);
+          acc.fma(d, f.x, f.y);
+        } else {
+          acc.add(-v.hi, -v.lo);
+          acc.fma(d, -f.x, -f.y);
+        }
+        acc.renorm();
+      }
+      ch[c] = ff_two_sum(acc.hi, acc.lo);
     }
     FF o3[3];
     if (orth) {
