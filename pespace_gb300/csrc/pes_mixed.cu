@@ -173,17 +173,21 @@ struct MixedDev {
   // the few bins that carry the weight, so neither the correction nor the
   // split form's error estimate uses it.
   const int32_t* wspike;    // [n_det][J] 1 where max_bin W > kSpikeRatio x mean W over the interval
-  int32_t rblocks;          // blocks per sample of the exact re-evaluation
+  int32_t rblocks;          // partial sums per sample of the exact re-evaluation
   int32_t refine_all;       // 1: every sample in the domain is re-evaluated (exactly where its spline
                             //   estimate says so, else in float-float)
   double* rpart;            // [B][rblocks] exact dense-range partials of re-evaluated samples
+  int32_t* rcount;          // [2] samples on the float-float and the exact list
+  int32_t* rlist;           // [2][B] the samples of either list (in no particular order)
+  int32_t list_cap;         // B
   // How each sample's dense range is re-evaluated, chosen after the dense
   // stage from its FP32 rounding estimate (the dense stage's own sum of
   // |d|^2 |h|^2 w^2) and its splines' error estimate (k_hd): not at all, in
   // float-float from the same splines (rounding: k_dense_ff), or exactly
   // (spline error: k_exact<3>).
   int32_t* rkind;           // [B] kRefineNone, kRefineFF or kRefineExact
-  double* fpart;            // [B][nblk_dense] float-float dense-range partials
+  int32_t nblk_ff;          // float-float partial sums per sample
+  double* fpart;            // [B][nblk_ff] float-float dense-range partials
   // Float-float copies of the FP64 inputs of one bin for k_dense_ff, six rows
   // per detector: d_A, d_E, d_T (re hi, re lo, im hi, im lo; scaled data),
   // (w_A hi, lo, w_E hi, lo), (w_T hi, lo, P re hi, lo), (P im hi, lo, 0, 0)
@@ -230,7 +234,20 @@ __device__ __forceinline__ bool in_zero_window(const MixedDev& M, int d, int64_t
 }
 constexpr double kSpikeRatio = 8.0;
 constexpr int kMomStride = 21;  // moments per bin (and interval) of wmom / wtot
-constexpr int kRefineBlocks = 32;  // blocks per sample of the exact re-evaluation
+// The exact re-evaluation: a listed sample's bins go to rblocks parts of at
+// least kRefineBins bins, a partial sum each, and the parts of all listed
+// samples to the blocks that the chip holds.  (A few samples are listed, of up
+// to 10^5 bins: with 32 blocks each they left most of the SMs idle.)
+constexpr int kRefineBins = 512;
+constexpr int kRefinePartsMax = 256, kRefinePartsMin = 32;
+constexpr int kSampleWarps = 4;  // samples per block of the kernels with a warp per sample
+
+// the sum over a warp, in a fixed order, in every lane
+__device__ __forceinline__ double warp_sum(double x) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
 
 // Error-free transformation: s + e == a + b exactly (Knuth's two-sum).
 __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
@@ -258,6 +275,7 @@ struct MixedBuffers {
   // the gradient pass of the dense stage stages its run inputs through shared
   // memory when they exceed half of L2 (they then stream from DRAM)
   bool stage_grad = false;
+  int64_t exact_grid = 1, ff_grid = 1;  // blocks of the re-evaluations that the device holds
   cudaEvent_t ev_nodes = nullptr, ev_tfit = nullptr, ev_dense = nullptr, ev_tadj = nullptr, ev_hd = nullptr, ev_pfit = nullptr,
               ev_kink = nullptr, ev_xgrad = nullptr;
   std::vector<int32_t> zbin_host;  // the zero windows' bins ([n_det][kZeroMax]), for the work report
@@ -824,125 +842,134 @@ __global__ void __launch_bounds__(kSparseThreads, 3) k_sparse_bwd_split(PlanDev 
 // live bin; xbin: bins below the first interval whose yearly orbital phase
 // advance omega |t(f_{j+1}) - t(f_j)| is at most kOrbitPhaseMax (that advance
 // falls monotonically with f over the inspiral, so a bisection finds it).
-// kPart 0 writes nsp and nch (needed by the sparse stage), kPart 1 xbin (needed
-// from the exact bins and the run anchors on), so the bisection can run on the
-// side stream.
-template <int kPart>
+// k_mixed_ranges writes nsp and nch (needed by the sparse stage),
+// k_exact_ranges xbin (needed from the exact bins and the run anchors on), so
+// the bisection can run on the side stream.
+__device__ __forceinline__ void range_counts(const MixedDev& M, int64_t kc, int& ns, int& nc) {
+  const int64_t last = kc - 1;
+  int lo = 0, hi = M.nchunks - 1;  // last run whose first bin is <= last
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (M.ch_begin[mid] <= last) lo = mid; else hi = mid - 1;
+  }
+  nc = lo + 1;
+  ns = min(max(M.ch_iv[lo] + 1, 3), M.J - 1);
+}
+
 __global__ void k_mixed_ranges(PlanDev P, MixedDev M, const SampleBlock<double>* __restrict__ blocks, int64_t B) {
-  // kPart 0: one thread per virtual sample v; kPart 1: one thread per sample
+  // kPart 0: one thread per virtual sample v
   const int nm = M.n_modes;
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= (kPart == 0 ? B * nm : B)) return;
-  const int64_t s = kPart == 0 ? t / nm : t;
-  const int kmode = kPart == 0 ? (int)(t % nm) : 0;
+  if (t < 2) M.rcount[t] = 0;  // this call's re-evaluation lists
+  if (t >= B * nm) return;
+  const int64_t s = t / nm;
+  const int kmode = (int)(t % nm);
   const SampleBlock<double>& b = blocks[s];
   const PhenomHMCoef<double>* hm = M.hm ? M.hm + s : nullptr;
   // the range's last live bin: the sample's cut, and for mode k of a
   // multi-mode model its mapped Mf = 0.2 (the mode's own cut)
   int64_t kc = b.status == kSampleOk ? b.kcut : 0;
-  if (kPart == 0) {
-    // the model's (the mode's) amplitude kink point: PhenomD's f_peak, or
-    // where the mode's amplitude map turns linear at its mapped f_peak
-    const double mfpk = (hm && kmode > 0) ? hm->md[kmode].frA : b.wf.fpeak;
-    const FF tcf = ff_from(b.tc), msf = ff_from(b.wf.Msec), fpf = ff_from(mfpk);
-    M.sff[2 * t] = make_float4(tcf.hi, tcf.lo, msf.hi, msf.lo);
-    M.sff[2 * t + 1] = make_float4(fpf.hi, fpf.lo, 0.0f, 0.0f);
-    // f t_c = (k0 + k) c, c = f_step t_c: its fraction is (k0 + k) frac(c) mod 1
-    const double cyc = M.f_step * b.tc;
-    const double rs = (cyc - floor(cyc)) * 18446744073709551616.0;  // 2^64
-    M.cfrac[t] = (rs >= 0.0 && rs < 18446744073709551616.0) ? (unsigned long long)rs : 0ull;
-    if (hm && kc > 0) {
-      // first bin whose mapped frequency passes Mf = 0.2 (the linear map, as
-      // the mode's model evaluates it past its amplitude corner)
-      const double Rk = hm->md[kmode].Rholm;
-      int64_t lo = 0, hi = kc;
-      while (lo < hi) {
-        const int64_t mid = (lo + hi) >> 1;
-        const double Mf = b.wf.Msec * ((double)(P.k0 + mid) * P.f_step);
-        if ((kmode == 0 ? Mf : Rk * Mf) <= kMfCut) lo = mid + 1; else hi = mid;
-      }
-      kc = lo;
-    }
-    M.vcut[t] = (int32_t)kc;
-    if (M.pkink) {
-      // the phase's second-derivative jumps at the mode's phase-map corners:
-      // one-sided second differences of dPsi/dMf, 1e-6 of Mf_c apart
-      float4* pk = M.pkink + 2 * t;
-      for (int c = 0; c < 2; ++c) {
-        double jh = 0.0, mfc = 1.0;
-        if (b.status == kSampleOk && hm) {
-          const HMMode<double>& md = hm->md[kmode];
-          const int m = kHMlm[kmode][1];
-          mfc = c == 0 ? md.fiP : md.frP;
-          const double e = 1e-6 * mfc;
-          auto dps = [&](double x) {
-            double ps, dp;
-            hm_phase<double>(b.wf, md, m, x, ps, dp);
-            return dp;
-          };
-          const double right = (dps(mfc + 2.0 * e) - dps(mfc + e)) / e;
-          const double left = (dps(mfc - e) - dps(mfc - 2.0 * e)) / e;
-          jh = 0.5 * (right - left);
-        }
-        const FF a = ff_from(mfc), q = ff_from(jh);
-        pk[c] = make_float4(a.hi, a.lo, q.hi, q.lo);
-      }
-    }
-  }
-  int ns = 0, nc = 0, xb = 0;
-  if (kc > 0) {
-    const int64_t last = kc - 1;
-    int lo = 0, hi = M.nchunks - 1;  // last run whose first bin is <= last
+  // the model's (the mode's) amplitude kink point: PhenomD's f_peak, or
+  // where the mode's amplitude map turns linear at its mapped f_peak
+  const double mfpk = (hm && kmode > 0) ? hm->md[kmode].frA : b.wf.fpeak;
+  const FF tcf = ff_from(b.tc), msf = ff_from(b.wf.Msec), fpf = ff_from(mfpk);
+  M.sff[2 * t] = make_float4(tcf.hi, tcf.lo, msf.hi, msf.lo);
+  M.sff[2 * t + 1] = make_float4(fpf.hi, fpf.lo, 0.0f, 0.0f);
+  // f t_c = (k0 + k) c, c = f_step t_c: its fraction is (k0 + k) frac(c) mod 1
+  const double cyc = M.f_step * b.tc;
+  const double rs = (cyc - floor(cyc)) * 18446744073709551616.0;  // 2^64
+  M.cfrac[t] = (rs >= 0.0 && rs < 18446744073709551616.0) ? (unsigned long long)rs : 0ull;
+  if (hm && kc > 0) {
+    // first bin whose mapped frequency passes Mf = 0.2 (the linear map, as
+    // the mode's model evaluates it past its amplitude corner)
+    const double Rk = hm->md[kmode].Rholm;
+    int64_t lo = 0, hi = kc;
     while (lo < hi) {
-      int mid = (lo + hi + 1) >> 1;
-      if (M.ch_begin[mid] <= last) lo = mid; else hi = mid - 1;
+      const int64_t mid = (lo + hi) >> 1;
+      const double Mf = b.wf.Msec * ((double)(P.k0 + mid) * P.f_step);
+      if ((kmode == 0 ? Mf : Rk * Mf) <= kMfCut) lo = mid + 1; else hi = mid;
     }
-    nc = lo + 1;
-    ns = M.ch_iv[lo] + 1;
-    if (ns < 3) ns = 3;
-    if (ns > M.J - 1) ns = M.J - 1;
-    if (kPart == 0) {
-      M.nsp[t] = ns;
-      M.nch[t] = nc;
-      return;
-    }
-    for (int d = 0; d < M.n_det; ++d) {
-      int xbd = 0;
-      // the exact range: the largest over the modes (each mode's own t(f))
-      for (int k = 0; k < nm; ++k) {
-        auto tfk = [&](int j) {
-          double a, ps, tt;
-          const double Mf = b.wf.Msec * M.node_f[j];
-          if (hm)
-            phenomhm_eval<double>(b.wf, *hm, k, Mf, a, ps, tt, nullptr);
-          else
-            phenomd_eval<double>(b.wf, Mf, a, ps, tt);
-          return tt;
-        };
-        auto unresolved = [&](int j) { return M.omega[d] * fabs(tfk(j + 1) - tfk(j)) > kOrbitPhaseMax; };
-        if (unresolved(0)) {
-          int lo2 = 0, hi2 = ns - 1;  // last unresolved interval
-          while (lo2 < hi2) {
-            int mid = (lo2 + hi2 + 1) >> 1;
-            if (unresolved(mid)) lo2 = mid; else hi2 = mid - 1;
-          }
-          const int64_t first = M.iv_first[lo2 + 1];
-          const int x = (int)(first < kc ? first : kc);
-          xbd = x > xbd ? x : xbd;
-        }
-      }
-      for (int k = 0; k < nm; ++k) M.xbind[(s * nm + k) * M.n_det + d] = xbd;
-      xb = xbd > xb ? xbd : xb;
-    }
-  } else if (kPart == 1) {
-    for (int d = 0; d < M.n_det; ++d)
-      for (int k = 0; k < nm; ++k) M.xbind[(s * nm + k) * M.n_det + d] = 0;
+    kc = lo;
   }
-  if (kPart == 0) {
-    M.nsp[t] = ns;
-    M.nch[t] = nc;
-  } else {
-    for (int k = 0; k < nm; ++k) M.xbin[s * nm + k] = xb;
+  M.vcut[t] = (int32_t)kc;
+  if (M.pkink) {
+    // the phase's second-derivative jumps at the mode's phase-map corners:
+    // one-sided second differences of dPsi/dMf, 1e-6 of Mf_c apart
+    float4* pk = M.pkink + 2 * t;
+    for (int c = 0; c < 2; ++c) {
+      double jh = 0.0, mfc = 1.0;
+      if (b.status == kSampleOk && hm) {
+        const HMMode<double>& md = hm->md[kmode];
+        const int m = kHMlm[kmode][1];
+        mfc = c == 0 ? md.fiP : md.frP;
+        const double e = 1e-6 * mfc;
+        auto dps = [&](double x) {
+          double ps, dp;
+          hm_phase<double>(b.wf, md, m, x, ps, dp);
+          return dp;
+        };
+        const double right = (dps(mfc + 2.0 * e) - dps(mfc + e)) / e;
+        const double left = (dps(mfc - e) - dps(mfc - 2.0 * e)) / e;
+        jh = 0.5 * (right - left);
+      }
+      const FF a = ff_from(mfc), q = ff_from(jh);
+      pk[c] = make_float4(a.hi, a.lo, q.hi, q.lo);
+    }
+  }
+  int ns = 0, nc = 0;
+  if (kc > 0) range_counts(M, kc, ns, nc);
+  M.nsp[t] = ns;
+  M.nch[t] = nc;
+}
+
+// xbin, xbind: a pair of threads per (sample, mode, detector), one for t(f) at
+// either end of the probed interval.  The bisection is a serial chain of FP64
+// model evaluations (64 cycles per warp instruction whatever its active
+// lanes): one thread per sample took 1.35 ms for six modes on three detectors
+// and 237 us for one mode on three, and the dense stage waits for it.
+__global__ void k_exact_ranges(PlanDev P, MixedDev M, const SampleBlock<double>* __restrict__ blocks, int64_t B,
+                               int group) {
+  __shared__ int xmax[64][PES_MAX_DETECTORS];  // [sample of the block]
+  const int nm = M.n_modes, sub = threadIdx.x % group, g = threadIdx.x / group;
+  const int64_t s = blockIdx.x * (int64_t)(blockDim.x / group) + g;
+  if (sub < M.n_det) xmax[g][sub] = 0;
+  __syncthreads();
+  const int k = (sub >> 1) / M.n_det, d = (sub >> 1) % M.n_det, side = sub & 1;
+  const bool mine = s < B && k < nm && blocks[s].status == kSampleOk && blocks[s].kcut > 0;
+  const unsigned pair = 3u << (threadIdx.x & 30);
+  if (mine) {  // the same for both threads of a pair
+    const SampleBlock<double>& b = blocks[s];
+    const PhenomHMCoef<double>* hm = M.hm ? M.hm + s : nullptr;
+    const int64_t kc = b.kcut;
+    int ns, nc;
+    range_counts(M, kc, ns, nc);
+    auto unresolved = [&](int j) {
+      double a, ps, tt;
+      const double Mf = b.wf.Msec * M.node_f[j + side];
+      if (hm)
+        phenomhm_eval<double>(b.wf, *hm, k, Mf, a, ps, tt, nullptr);
+      else
+        phenomd_eval<double>(b.wf, Mf, a, ps, tt);
+      return M.omega[d] * fabs(__shfl_xor_sync(pair, tt, 1) - tt) > kOrbitPhaseMax;
+    };
+    if (unresolved(0)) {
+      int lo = 0, hi = ns - 1;  // last unresolved interval
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (unresolved(mid)) lo = mid; else hi = mid - 1;
+      }
+      const int64_t first = M.iv_first[lo + 1];
+      // the exact range: the largest over the modes (each mode's own t(f))
+      if (side == 0) atomicMax(&xmax[g][d], (int)(first < kc ? first : kc));
+    }
+  }
+  __syncthreads();
+  if (s >= B) return;
+  if (side == 0 && k < nm) M.xbind[(s * nm + k) * M.n_det + d] = xmax[g][d];
+  if (side == 0 && k < nm && d == 0) {
+    int xb = 0;
+    for (int e = 0; e < M.n_det; ++e) xb = max(xb, xmax[g][e]);
+    M.xbin[s * nm + k] = xb;
   }
 }
 
@@ -1838,14 +1865,20 @@ constexpr double kSplineRel = 0.01;
 constexpr double kModelRelHM = 2e-9;
 constexpr double kBar = 1e-2;
 
-// one thread per sample, after the dense stage (its rounding sums) and k_hd
-__global__ void k_refine_select(PlanDev P, MixedDev M, const SampleBlock<double>* __restrict__ blocks, int64_t B) {
-  const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// One warp per sample, after the dense stage (its rounding sums) and k_hd; the
+// samples to re-evaluate go on the lists that the re-evaluations share out over
+// the chip.
+__global__ void __launch_bounds__(kSampleWarps * 32) k_refine_select(PlanDev P, MixedDev M,
+                                                                     const SampleBlock<double>* __restrict__ blocks,
+                                                                     int64_t B) {
+  const int lane = threadIdx.x & 31;
+  const int64_t s = blockIdx.x * (int64_t)kSampleWarps + (threadIdx.x >> 5);
   if (s >= B) return;
   int kind = kRefineNone;
   if (blocks[s].status == kSampleOk) {
     double sq = 0.0, eha = 0.0, hh = 0.0;
-    for (int k = 0; k < M.nblk_dense; ++k) sq += M.part[((size_t)s * M.nblk_dense + k) * kPartW + 3];
+    for (int k = lane; k < M.nblk_dense; k += 32) sq += M.part[((size_t)s * M.nblk_dense + k) * kPartW + 3];
+    sq = warp_sum(sq);
     for (int k = 0; k < M.n_modes; ++k)
       for (int d = 0; d < M.n_det; ++d) {
         const double* hv = M.hd + (((size_t)s * M.n_modes + k) * M.n_det + d) * kHdOut;
@@ -1859,7 +1892,12 @@ __global__ void k_refine_select(PlanDev P, MixedDev M, const SampleBlock<double>
     if (M.refine_all || er + es > kRefineTarget || loud)
       kind = (es > kRefineTarget || loud) ? kRefineExact : kRefineFF;
   }
+  if (lane != 0) return;
   M.rkind[s] = kind;
+  if (kind != kRefineNone) {
+    const int l = kind == kRefineExact ? 1 : 0;
+    M.rlist[(size_t)l * M.list_cap + atomicAdd(&M.rcount[l], 1)] = (int)s;
+  }
 }
 
 // Bins [0, xbind[s][d]) of each detector evaluated directly (FP64 model and residual against the
@@ -1869,7 +1907,8 @@ __global__ void k_refine_select(PlanDev P, MixedDev M, const SampleBlock<double>
 // k_refine_select sends to the exact re-evaluation of their dense range
 // (without the T-channel zero windows); 4: lnL partials of the window bins
 // in [xbind[s][d], kcut) (their gradient: k_zero_grad).
-// grid (xblocks, rblocks or zblocks, B); threads stride over the bins.  The
+// grid (xblocks or zblocks, B), kMode 3: as many blocks as the chip holds, over
+// the parts of the listed samples; threads stride over the bins.  The
 // value passes are held to 168 registers (3 blocks per SM instead of 2: the
 // bench step 1.5% faster).
 template <int kMode, class T>
@@ -1889,11 +1928,23 @@ __global__ void __launch_bounds__(kExactThreads, kMode == 1 ? 1 : 3) k_exact(Pla
   __shared__ double red[kExactThreads / 32][NV];
   __shared__ PhenomHMCoef<double> hmd;  // multi-mode plans (value passes)
   __shared__ PhenomHMCoef<FF> hmf;
-  const int s = blockIdx.y;
   const int nm = M.n_modes;
+  // kRefine: the parts of the listed samples, shared out over the grid
+  for (int item = blockIdx.x; !kRefine || item < M.rcount[1] * M.rblocks; item += gridDim.x) {
+  const int s = kRefine ? M.rlist[M.list_cap + item / M.rblocks] : blockIdx.y;
+  const int part = kRefine ? item % M.rblocks : blockIdx.x, parts = kRefine ? M.rblocks : gridDim.x;
   const int xb = M.xbin[(size_t)s * nm];
   if (!kRefine && !kZero && xb == 0) return;  // uniform per block; the finalizers skip such samples
-  if (kRefine && (blocks[s].status != kSampleOk || M.rkind[s] != kRefineExact)) return;
+  if constexpr (kRefine) {
+    int most = 0;
+    for (int d = 0; d < M.n_det; ++d)
+      most = max(most, (int)blocks[s].kcut - M.xbind[(size_t)s * nm * M.n_det + d]);
+    if (part * kExactThreads >= most) {  // no bins in this part (uniform)
+      if (threadIdx.x == 0) M.rpart[(size_t)s * parts + part] = 0.0;
+      continue;
+    }
+    __syncthreads();  // the previous part's reads of the shared block
+  }
   load_block(blocks, s, sb);
   if (kFF && M.hm) load_hm(M.hm, s, hmd);
   __syncthreads();
@@ -1913,7 +1964,7 @@ __global__ void __launch_bounds__(kExactThreads, kMode == 1 ? 1 : 3) k_exact(Pla
       const int xbd = M.xbind[(size_t)s * nm * M.n_det + d];
       const int i0 = kRefine ? xbd : 0, i1 = kRefine ? (int)sb.kcut : xbd;
       const int n_it = kZero ? M.nzb[d] : i1 - i0;
-      for (int it = blockIdx.x * kExactThreads + threadIdx.x; it < n_it; it += gridDim.x * kExactThreads) {
+      for (int it = part * kExactThreads + threadIdx.x; it < n_it; it += parts * kExactThreads) {
         int i = i0 + it;
         if constexpr (kZero) {
           i = M.zbin[(size_t)d * kZeroMax + it];
@@ -2046,13 +2097,15 @@ __global__ void __launch_bounds__(kExactThreads, kMode == 1 ? 1 : 3) k_exact(Pla
 #pragma unroll
     for (int w = 0; w < kExactThreads / 32; ++w) x += red[w][threadIdx.x];
     if (kMode == 0)
-      M.xpart[(size_t)s * gridDim.x + blockIdx.x] = x;
+      M.xpart[(size_t)s * parts + part] = x;
     else if (kMode == 3)
-      M.rpart[(size_t)s * gridDim.x + blockIdx.x] = x;
+      M.rpart[(size_t)s * parts + part] = x;
     else if (kMode == 4)
-      M.zpart[(size_t)s * gridDim.x + blockIdx.x] = x;
+      M.zpart[(size_t)s * parts + part] = x;
     else
-      M.xgpart[((size_t)s * gridDim.x + blockIdx.x) * 11 + threadIdx.x] = x;
+      M.xgpart[((size_t)s * parts + part) * 11 + threadIdx.x] = x;
+  }
+  if (!kRefine) break;
   }
 }
 
@@ -2881,50 +2934,54 @@ __global__ void __launch_bounds__(kMixThreads, 5) k_dense_mixed(PlanDev P, Mixed
 // coefficients to the residual |d - h|^2 w in float-float against
 // float-float copies of the FP64 data, weights and prefactor.  The per-bin
 // rounding falls from about 2e-7 of the terms to below 1e-13, so what is
-// left of the error is the splines' own.  Same grid and run groups as
-// k_dense_mixed; lane l of a warp first takes the phase anchor of the
-// group's run l of every mode (shared memory), then each run takes a bin
-// per lane.  Partials: fpart [B][nblk_dense].
+// left of the error is the splines' own.  As many blocks as the chip holds
+// share the listed samples' groups of 32 runs; a block's threads first take
+// the groups' phase anchors (run, mode, detector), then its warps every fourth
+// run, a bin per lane (32 runs per warp left a call of 16 samples with less
+// than one warp per SM partition).  Partials: fpart [B][nblk_ff].
 template <int kNM>
 __global__ void __launch_bounds__(kMixThreads) k_dense_ff(PlanDev P, MixedDev M,
                                                           const SampleBlock<double>* __restrict__ blocks) {
-  __shared__ float4 anc[kMixThreads / 32][kNM][kChunkMax][2];  // ph0, ph1 | ph2, ph3 (hi, lo pairs)
-  __shared__ int ancq[kMixThreads / 32][kNM][kChunkMax];        // the straddled phase corner, -1 when none
+  // phase anchors of the block's runs: ph0, ph1 | ph2, ph3 (hi, lo pairs), and
+  // the straddled phase corner (-1 when none)
+  __shared__ float4 anc[PES_MAX_DETECTORS][kNM][kChunkMax][2];
+  __shared__ int ancq[PES_MAX_DETECTORS][kNM][kChunkMax];
   __shared__ double red[kMixThreads / 32];
-  const int s = blockIdx.y;
-  if (M.rkind[s] != kRefineFF) return;  // uniform per block
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int first = (blockIdx.x * (kMixThreads / 32) + wid) * kChunkMax;
-  int nc = M.nch[(size_t)s * kNM];
+  for (int item = blockIdx.x; item < M.rcount[0] * M.nblk_ff; item += gridDim.x) {
+    const int s = M.rlist[item / M.nblk_ff], blk = item % M.nblk_ff;
+    const int first = blk * kChunkMax;
+    int nc = M.nch[(size_t)s * kNM];
 #pragma unroll
-  for (int k = 1; k < kNM; ++k) nc = max(nc, M.nch[(size_t)s * kNM + k]);
-  const int64_t kcut = blocks[s].kcut;
-  FF acc = ff_make(0.0f, 0.0f);
-  if (first < nc) {
+    for (int k = 1; k < kNM; ++k) nc = max(nc, M.nch[(size_t)s * kNM + k]);
+    const int64_t kcut = blocks[s].kcut;
+    if (first >= nc) {  // uniform
+      if (threadIdx.x == 0) M.fpart[(size_t)s * M.nblk_ff + blk] = 0.0;
+      continue;
+    }
     const int last = min(nc, first + kChunkMax);
+    for (int q = threadIdx.x; q < M.n_det * kNM * kChunkMax; q += kMixThreads) {
+      const int r = q % kChunkMax, k = q / kChunkMax % kNM, d = q / (kChunkMax * kNM);
+      const int c = first + r, v = s * kNM + k;
+      const size_t sdk = ((size_t)s * kNM + k) * M.n_det + d;
+      float4 a0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), a1 = a0;
+      int qk = -1;
+      if (c < M.nch[v] && M.ch_begin[c] >= M.xbind[sdk]) {
+        const AnchorFF A = run_anchor_ff(P, M, v, sdk, c, M.ch_begin[c], M.ch_iv[c]);
+        a0 = make_float4(A.ph0.hi, A.ph0.lo, A.ph1.hi, A.ph1.lo);
+        a1 = make_float4(A.ph2.hi, A.ph2.lo, A.ph3.hi, A.ph3.lo);
+        qk = A.qk;
+      }
+      anc[d][k][r][0] = a0;
+      anc[d][k][r][1] = a1;
+      ancq[d][k][r] = qk;
+    }
+    __syncthreads();
+    FF acc = ff_make(0.0f, 0.0f);
     for (int d = 0; d < M.n_det; ++d) {
       const size_t sd = (size_t)s * kNM * M.n_det + d;  // (virtual sample of mode 0, detector)
       const int xb = M.xbind[sd];
-      {
-        const int c = first + lane;
-#pragma unroll 1
-        for (int k = 0; k < kNM; ++k) {
-          const int v = s * kNM + k;
-          float4 a0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), a1 = a0;
-          int qk = -1;
-          if (c < M.nch[v] && M.ch_begin[c] >= xb) {
-            const AnchorFF A = run_anchor_ff(P, M, v, sd + (size_t)k * M.n_det, c, M.ch_begin[c], M.ch_iv[c]);
-            a0 = make_float4(A.ph0.hi, A.ph0.lo, A.ph1.hi, A.ph1.lo);
-            a1 = make_float4(A.ph2.hi, A.ph2.lo, A.ph3.hi, A.ph3.lo);
-            qk = A.qk;
-          }
-          anc[wid][k][lane][0] = a0;
-          anc[wid][k][lane][1] = a1;
-          ancq[wid][k][lane] = qk;
-        }
-      }
-      __syncwarp();
-      for (int c = first; c < last; ++c) {
+      for (int c = first + wid; c < last; c += kMixThreads / 32) {
         const int kb = M.ch_begin[c];
         if (kb < xb) continue;  // exact bins
         const int j = M.ch_iv[c];
@@ -2942,14 +2999,14 @@ __global__ void __launch_bounds__(kMixThreads) k_dense_ff(PlanDev P, MixedDev M,
           const int v = s * kNM + k;
           if (kNM > 1 && (c >= M.nch[v] || i >= M.vcut[v])) continue;  // past the mode's range
           const size_t sdk = sd + (size_t)k * M.n_det;
-          const float4 a0 = anc[wid][k][c - first][0], a1 = anc[wid][k][c - first][1];
+          const float4 a0 = anc[d][k][c - first][0], a1 = anc[d][k][c - first][1];
           FF ph = ff_make(a0.x, a0.y) + ff_mulf(ff_make(a0.z, a0.w), u);
           ph = ph + ff_mulf(ff_make(a1.x, a1.y), u * u);  // u^2, u^3 < 2^15: exact
           ph = ph + ff_mulf(ff_make(a1.z, a1.w), u * u * u);
           const float4 sa = M.sff[2 * v];
           const FF msf = ff_make(sa.z, sa.w);
           if (kNM > 1) {
-            const int qk = ancq[wid][k][c - first];
+            const int qk = ancq[d][k][c - first];
             if (qk >= 0) {
               const float4 k4 = M.pkink[2 * v + qk];
               const FF xq = msf * f - ff_make(k4.x, k4.y);
@@ -3013,23 +3070,22 @@ __global__ void __launch_bounds__(kMixThreads) k_dense_ff(PlanDev P, MixedDev M,
           acc = acc + (er * er + ei * ei) * wch[ch];
         }
       }
-      __syncwarp();  // the next detector's anchors overwrite this one's
     }
-  }
-  // lanes and warps in float-float, the block partial in FP64
+    // lanes and warps in float-float, the block partial in FP64
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float oh = __shfl_down_sync(0xffffffffu, acc.hi, o);
-    const float ol = __shfl_down_sync(0xffffffffu, acc.lo, o);
-    acc = acc + ff_make(oh, ol);
-  }
-  if (lane == 0) red[wid] = ff_to(acc);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double x = 0.0;
+    for (int o = 16; o > 0; o >>= 1) {
+      const float oh = __shfl_down_sync(0xffffffffu, acc.hi, o);
+      const float ol = __shfl_down_sync(0xffffffffu, acc.lo, o);
+      acc = acc + ff_make(oh, ol);
+    }
+    if (lane == 0) red[wid] = ff_to(acc);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double x = 0.0;
 #pragma unroll
-    for (int w = 0; w < kMixThreads / 32; ++w) x += red[w];
-    M.fpart[(size_t)s * M.nblk_dense + blockIdx.x] = x;
+      for (int w = 0; w < kMixThreads / 32; ++w) x += red[w];
+      M.fpart[(size_t)s * M.nblk_ff + blk] = x;
+    }
   }
 }
 
@@ -3217,93 +3273,85 @@ __global__ void __launch_bounds__(kHdThreads) k_hd(PlanDev P, MixedDev M,
   }
 }
 
-__global__ void k_mixed_finalize(PlanDev P, MixedDev M, const SampleBlock<double>* __restrict__ blocks, int64_t B,
-                                 double* __restrict__ lnl, int32_t* __restrict__ status) {
-  int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// One warp per sample, its lanes over the partial sums (one thread per sample
+// took 75 us, the gradient's sums 102 us, on three detectors).
+__global__ void __launch_bounds__(kSampleWarps * 32) k_mixed_finalize(PlanDev P, MixedDev M,
+                                                                      const SampleBlock<double>* __restrict__ blocks,
+                                                                      int64_t B, double* __restrict__ lnl,
+                                                                      int32_t* __restrict__ status) {
+  const int lane = threadIdx.x & 31;
+  const int64_t s = blockIdx.x * (int64_t)kSampleWarps + (threadIdx.x >> 5);
   if (s >= B) return;
   const SampleBlock<double>& b = blocks[s];
   if (b.status != kSampleOk) {
-    lnl[s] = -INFINITY;
-    if (status) status[s] = b.status;
+    if (lane == 0) {
+      lnl[s] = -INFINITY;
+      if (status) status[s] = b.status;
+    }
     return;
   }
-  // dense bins: the direct sum of |d - h|^2 w, or the split form for templates
-  // far from the data (residual above 2 sqrt(<h|h> <d|d>)), where the FP32
-  // rounding of the model enters only the cross term
-  double R = 0.0, X = 0.0, H = 0.0, Dd = 0.0, Cm = 0.0;
-  for (int k = 0; k < M.nblk_dense; ++k) {
-    R += M.part[((size_t)s * M.nblk_dense + k) * kPartW];
-    X += M.part[((size_t)s * M.nblk_dense + k) * kPartW + 1];
-    Cm += M.part[((size_t)s * M.nblk_dense + k) * kPartW + 2];
-  }
-  if (M.n_modes > 1) {
-    // multi-mode plans: the split form for far templates with sum |h|^2 w =
-    // the modes' own sums (exact, from their splines) + their cross terms
-    // (dense stage)
+  double acc;
+  if (M.rkind[s] == kRefineExact) {  // the exact re-evaluation of the dense range
+    acc = 0.0;
+    for (int k = lane; k < M.rblocks; k += 32) acc += M.rpart[(size_t)s * M.rblocks + k];
+  } else if (M.rkind[s] == kRefineFF) {  // the float-float one
+    acc = 0.0;
+    for (int k = lane; k < M.nblk_ff; k += 32) acc += M.fpart[(size_t)s * M.nblk_ff + k];
+  } else {
+    // dense bins: the direct sum of |d - h|^2 w, or the split form for templates
+    // far from the data (residual above 2 sqrt(<h|h> <d|d>)), where the FP32
+    // rounding of the model enters only the cross term
+    double R = 0.0, X = 0.0, Cm = 0.0, H = 0.0, Dd = 0.0;
+    for (int k = lane; k < M.nblk_dense; k += 32) {
+      const double* v = M.part + ((size_t)s * M.nblk_dense + k) * kPartW;
+      R += v[0];
+      X += v[1];
+      Cm += v[2];
+    }
+    R = warp_sum(R);
+    X = warp_sum(X);
+    // sum |h|^2 w: the modes' own sums from their splines, corrected by the
+    // midpoint estimate of their error, and (several modes) their cross terms
+    // from the dense stage
+    if (M.n_modes > 1) H = warp_sum(Cm);
     for (int k = 0; k < M.n_modes; ++k)
       for (int d = 0; d < M.n_det; ++d) {
         const double* hv = M.hd + (((size_t)s * M.n_modes + k) * M.n_det + d) * kHdOut;
         H += hv[0] + hv[3];
+        if (k == 0) Dd += hv[1];
       }
-    for (int d = 0; d < M.n_det; ++d) Dd += M.hd[((size_t)s * M.n_modes * M.n_det + d) * kHdOut + 1];
-    const double Ht = H + Cm;
-    double acc = (R > 2.0 * sqrt(fmax(Ht, 0.0) * Dd)) ? (Dd + X) + Ht : R;
-    if (M.rkind[s] == kRefineExact) {  // the exact re-evaluation of the dense range
-      acc = 0.0;
-      for (int k = 0; k < M.rblocks; ++k) acc += M.rpart[(size_t)s * M.rblocks + k];
-    } else if (M.rkind[s] == kRefineFF) {  // the float-float one
-      acc = 0.0;
-      for (int k = 0; k < M.nblk_dense; ++k) acc += M.fpart[(size_t)s * M.nblk_dense + k];
-    }
-    if (M.xbin[s * M.n_modes] > 0)
-      for (int k = 0; k < M.xblocks; ++k) acc += M.xpart[(size_t)s * M.xblocks + k];
-    for (int k = 0; k < M.zblocks; ++k) acc += M.zpart[(size_t)s * M.zblocks + k];
-    const double v = -2.0 * P.df * (acc + P.suffix[b.kcut]);
-    lnl[s] = v;
-    if (status) status[s] = isfinite(v) ? kSampleOk : kSampleNonFinite;
-    return;
+    acc = (R > 2.0 * sqrt((M.n_modes > 1 ? fmax(H, 0.0) : H) * Dd)) ? (Dd + X) + H : R;
+    if (lane != 0) acc = 0.0;
   }
-  for (int d = 0; d < M.n_det; ++d) {
-    // sum |h|^2 w from the splines, corrected by the midpoint estimate of their error
-    H += M.hd[((size_t)s * M.n_det + d) * kHdOut] + M.hd[((size_t)s * M.n_det + d) * kHdOut + 3];
-    Dd += M.hd[((size_t)s * M.n_det + d) * kHdOut + 1];
-  }
-  double acc = (R > 2.0 * sqrt(H * Dd)) ? (Dd + X) + H : R;
-  if (M.rkind[s] == kRefineExact) {  // the exact re-evaluation of the dense range
-    acc = 0.0;
-    for (int k = 0; k < M.rblocks; ++k) acc += M.rpart[(size_t)s * M.rblocks + k];
-  } else if (M.rkind[s] == kRefineFF) {  // the float-float one
-    acc = 0.0;
-    for (int k = 0; k < M.nblk_dense; ++k) acc += M.fpart[(size_t)s * M.nblk_dense + k];
-  }
-  if (M.xbin[s] > 0)
-    for (int k = 0; k < M.xblocks; ++k) acc += M.xpart[(size_t)s * M.xblocks + k];
-  for (int k = 0; k < M.zblocks; ++k) acc += M.zpart[(size_t)s * M.zblocks + k];
+  if (M.xbin[s * M.n_modes] > 0)
+    for (int k = lane; k < M.xblocks; k += 32) acc += M.xpart[(size_t)s * M.xblocks + k];
+  for (int k = lane; k < M.zblocks; k += 32) acc += M.zpart[(size_t)s * M.zblocks + k];
+  acc = warp_sum(acc);
+  if (lane != 0) return;
   const double v = -2.0 * P.df * (acc + P.suffix[b.kcut]);
   lnl[s] = v;
   if (status) status[s] = isfinite(v) ? kSampleOk : kSampleNonFinite;
 }
 
-__global__ void k_mixed_grad_finalize(MixedDev M, int64_t B, double xscale, double* __restrict__ grad) {
-  int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (s >= B) return;
-  const bool ok = reinterpret_cast<const SampleBlock<GradScalar>*>(M.gblocks)[s].status == kSampleOk;
-  const bool exact = M.xbin[s] > 0;
-  for (int p = 0; p < 11; ++p) {
-    double acc = 0.0;
-    if (ok) {
-      for (int d = 0; d < M.n_det; ++d) {
-        for (int b = 0; b < M.nblk_sparse; ++b) acc += M.gpart[(((size_t)s * M.n_det + d) * M.nblk_sparse + b) * 11 + p];
-        if (p == 10) acc += M.gdir[(size_t)s * M.n_det + d];
-      }
-      double x = 0.0;
-      if (exact)
-        for (int b = 0; b < M.xblocks; ++b) x += M.xgpart[((size_t)s * M.xblocks + b) * 11 + p];
-      for (int b = 0; b < M.zblocks; ++b) x += M.zgpart[((size_t)s * M.zblocks + b) * 11 + p];
-      acc += xscale * x;
-    }
-    grad[11 * s + p] = acc;
+// one warp per (sample, parameter)
+__global__ void __launch_bounds__(kSampleWarps * 32) k_mixed_grad_finalize(MixedDev M, int64_t B, double xscale,
+                                                                           double* __restrict__ grad) {
+  const int lane = threadIdx.x & 31;
+  const int64_t t = blockIdx.x * (int64_t)kSampleWarps + (threadIdx.x >> 5);
+  if (t >= 11 * B) return;
+  const int64_t s = t / 11;
+  const int p = (int)(t % 11);
+  double acc = 0.0, x = 0.0;
+  if (reinterpret_cast<const SampleBlock<GradScalar>*>(M.gblocks)[s].status == kSampleOk) {
+    const int nb = M.n_det * M.nblk_sparse;
+    for (int b = lane; b < nb; b += 32) acc += M.gpart[((size_t)s * nb + b) * 11 + p];
+    if (p == 10 && lane < M.n_det) acc += M.gdir[(size_t)s * M.n_det + lane];
+    if (M.xbin[s] > 0)
+      for (int b = lane; b < M.xblocks; b += 32) x += M.xgpart[((size_t)s * M.xblocks + b) * 11 + p];
+    for (int b = lane; b < M.zblocks; b += 32) x += M.zgpart[((size_t)s * M.zblocks + b) * 11 + p];
+    acc = warp_sum(acc + xscale * x);
   }
+  if (lane == 0) grad[11 * s + p] = acc;
 }
 
 // ------------------------------------------------------------------ data ingestion
@@ -3456,6 +3504,17 @@ int mixed_create(PesPlan* p) {
   PES_CHECK_CUDA(cudaEventCreateWithFlags(&mb->join, cudaEventDisableTiming));
   PES_CHECK_CUDA(cudaEventCreateWithFlags(&mb->xready, cudaEventDisableTiming));
   PES_CHECK_CUDA(cudaStreamCreateWithFlags(&mb->aux, cudaStreamNonBlocking));
+  {
+    int sms = 0, per = 0;
+    PES_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device));
+    PES_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_exact<3, double>, kExactThreads, 0));
+    mb->exact_grid = (int64_t)sms * std::max(per, 1);
+    if (p->desc.approximant == PES_APPROX_PHENOMHM)
+      PES_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_dense_ff<kHMModes>, kMixThreads, 0));
+    else
+      PES_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_dense_ff<1>, kMixThreads, 0));
+    mb->ff_grid = (int64_t)sms * std::max(per, 1);
+  }
   for (cudaEvent_t* e : {&mb->ev_nodes, &mb->ev_tfit, &mb->ev_dense, &mb->ev_tadj, &mb->ev_hd, &mb->ev_pfit,
                          &mb->ev_kink, &mb->ev_xgrad})
     PES_CHECK_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
@@ -3534,6 +3593,8 @@ int mixed_create(PesPlan* p) {
   }
   M.nchunks = (int32_t)cb.size();
   M.nblk_dense = (int32_t)ceil_div(M.nchunks, (long long)kChunkMax * (kMixThreads / 32));
+  M.nblk_ff = (int32_t)ceil_div(M.nchunks, (long long)kChunkMax);
+  M.rblocks = (int32_t)std::min<int64_t>(kRefinePartsMax, std::max<int64_t>(kRefinePartsMin, n / kRefineBins));
   M.nblk_sparse = (int32_t)ceil_div(J, kSparseThreads);
   int rc = PES_OK;
   double *node_f = nullptr, *scr, *part, *gpart, *gdir;
@@ -3551,7 +3612,7 @@ int mixed_create(PesPlan* p) {
   double *xpart, *xgpart;
   FF *wmom, *wtot;
   double *dsuf, *wrow, *hdv, *rpart, *fpart;
-  int32_t* rkind;
+  int32_t *rkind, *rcount, *rlist;
   float4* xff;
   float* cgb;
   float2* mid_ff;
@@ -3587,8 +3648,9 @@ int mixed_create(PesPlan* p) {
       (rc = alloc(mb, &cgb, sd * J * 6)) || (rc = alloc(mb, &hdv, sd * kHdOut)) ||
       (rc = alloc(mb, &mid_ff, J)) || (rc = alloc(mb, &tdm_ff, (size_t)nd * J)) || (rc = alloc(mb, &ymv, sd * 7 * J)) ||
       (rc = alloc(mb, &cbump, sd * J * 2)) || (rc = alloc(mb, &wspk, (size_t)nd * J)) ||
-      (rc = alloc(mb, &rpart, (size_t)B * kRefineBlocks)) || (rc = alloc(mb, &rkind, (size_t)B)) ||
-      (rc = alloc(mb, &fpart, (size_t)B * M.nblk_dense)) || (rc = alloc(mb, &xff, (size_t)nd * 6 * n)) ||
+      (rc = alloc(mb, &rpart, (size_t)B * M.rblocks)) || (rc = alloc(mb, &rkind, (size_t)B)) ||
+      (rc = alloc(mb, &rcount, 2)) || (rc = alloc(mb, &rlist, (size_t)2 * B)) ||
+      (rc = alloc(mb, &fpart, (size_t)B * M.nblk_ff)) || (rc = alloc(mb, &xff, (size_t)nd * 6 * n)) ||
       (rc = alloc(mb, &gpart, gsd * M.nblk_sparse * 11)) || (rc = alloc(mb, &gdir, gsd)) ||
       (rc = alloc(mb, &gblk, (size_t)B)) || (rc = alloc(mb, &kR, sd * 6)) || (rc = alloc(mb, &kC, sd * 6)) ||
       (rc = alloc(mb, &kF, sd * 16)) || (rc = alloc(mb, &kM, gsd * 12)) || (rc = alloc(mb, &xbin, V)) || (rc = alloc(mb, &xbind, sd)) ||
@@ -3732,7 +3794,9 @@ int mixed_create(PesPlan* p) {
   M.wspike = wspk;
   PES_CHECK_CUDA(cudaMemset(wspk, 0, sizeof(int32_t) * nd * J));
   M.rpart = rpart;
-  M.rblocks = kRefineBlocks;
+  M.rcount = rcount;
+  M.rlist = rlist;
+  M.list_cap = (int32_t)B;
   M.refine_all = 0;
   M.rkind = rkind;
   M.fpart = fpart;
@@ -3857,6 +3921,15 @@ int mixed_ingest(PesPlan* p, int det, const double* data, const double* psd, cud
 }
 
 // The value set-up: IMRPhenomD plans in the plain order (phenomd_setup_serial).
+// blocks of sample_threads threads, or of one sample's group where that is larger
+static void launch_exact_ranges(PesPlan* p, const SampleBlock<double>* blocks, int64_t B, cudaStream_t st) {
+  const MixedDev& M = p->mixed->dev;
+  int group = 2;
+  while (group < 2 * M.n_modes * M.n_det) group *= 2;
+  const int threads = std::max(group, std::min(p->sample_threads, 64) / group * group);
+  k_exact_ranges<<<ceil_div(B, threads / group), threads, 0, st>>>(p->dev, M, blocks, B, group);
+}
+
 static void launch_setup(PesPlan* p, const double* theta, int64_t B, SampleBlock<double>* blocks, cudaStream_t st) {
   if (p->desc.approximant == PES_APPROX_PHENOMHM)
     k_setup<double><<<setup_blocks(B), 64, 0, st>>>(p->dev, theta, B, 0, blocks, hm_blocks<double>(p));
@@ -3872,8 +3945,8 @@ int mixed_model(PesPlan* p, const double* theta_dev, double* out, cudaStream_t s
   launch_setup(p, theta_dev, 1, blocks, st);
   PES_CHECK_LAUNCH();
   const unsigned nm = (unsigned)M.n_modes;
-  k_mixed_ranges<0><<<1, 64, 0, st>>>(p->dev, M, blocks, 1);
-  k_mixed_ranges<1><<<1, 64, 0, st>>>(p->dev, M, blocks, 1);
+  k_mixed_ranges<<<1, 64, 0, st>>>(p->dev, M, blocks, 1);
+  launch_exact_ranges(p, blocks, 1, st);
   PES_CHECK_LAUNCH();
   k_kink<<<1, 64, 0, st>>>(p->dev, M, G, blocks, 1);
   PES_CHECK_LAUNCH();
@@ -3948,7 +4021,7 @@ int mixed_lnl(PesPlan* p, const double* theta, int64_t B, double* lnl, double* g
   PES_CHECK_LAUNCH();
   {
     ProfScope ps(p, kKOther, st);
-    k_mixed_ranges<0><<<ceil_div(V, 64), 64, 0, st>>>(p->dev, M, blocks, B);
+    k_mixed_ranges<<<ceil_div(V, 64), 64, 0, st>>>(p->dev, M, blocks, B);
   }
   PES_CHECK_LAUNCH();
   // side stream: the exact-bin range, the exact bins and the gradient set-up they need
@@ -3957,7 +4030,7 @@ int mixed_lnl(PesPlan* p, const double* theta, int64_t B, double* lnl, double* g
   PES_CHECK_CUDA(cudaStreamWaitEvent(side, p->mixed->fork, 0));
   {
     ProfScope ps(p, kKOther, side);
-    k_mixed_ranges<1><<<ceil_div(B, p->sample_threads), p->sample_threads, 0, side>>>(p->dev, M, blocks, B);
+    launch_exact_ranges(p, blocks, B, side);
   }
   PES_CHECK_LAUNCH();
   PES_CHECK_CUDA(cudaEventRecord(p->mixed->xready, side));
@@ -4053,20 +4126,22 @@ int mixed_lnl(PesPlan* p, const double* theta, int64_t B, double* lnl, double* g
     PES_CHECK_CUDA(cudaStreamWaitEvent(side, p->mixed->ev_dense, 0));
     {
       ProfScope ps(p, kKOther, side);
-      k_refine_select<<<ceil_div(B, 64), 64, 0, side>>>(p->dev, M, blocks, B);
+      k_refine_select<<<ceil_div(B, kSampleWarps), kSampleWarps * 32, 0, side>>>(p->dev, M, blocks, B);
     }
     PES_CHECK_LAUNCH();
     {
       ProfScope ps(p, kKDenseFp64, side);
-      k_exact<3, double><<<dim3(M.rblocks, (unsigned)B), kExactThreads, 0, side>>>(p->dev, M, G, blocks, nullptr);
+      k_exact<3, double><<<(unsigned)std::min<int64_t>(p->mixed->exact_grid, B * M.rblocks), kExactThreads, 0, side>>>(
+          p->dev, M, G, blocks, nullptr);
     }
     PES_CHECK_LAUNCH();
     {
       ProfScope ps(p, kKOther, side);
+      const unsigned ffgrid = (unsigned)std::min<int64_t>(p->mixed->ff_grid, B * M.nblk_ff);
       if (multi)
-        k_dense_ff<kHMModes><<<dim3(M.nblk_dense, (unsigned)B), kMixThreads, 0, side>>>(p->dev, M, blocks);
+        k_dense_ff<kHMModes><<<ffgrid, kMixThreads, 0, side>>>(p->dev, M, blocks);
       else
-        k_dense_ff<1><<<dim3(M.nblk_dense, (unsigned)B), kMixThreads, 0, side>>>(p->dev, M, blocks);
+        k_dense_ff<1><<<ffgrid, kMixThreads, 0, side>>>(p->dev, M, blocks);
     }
     PES_CHECK_LAUNCH();
     PES_CHECK_CUDA(cudaEventRecord(p->mixed->join, side));
@@ -4109,7 +4184,7 @@ int mixed_lnl(PesPlan* p, const double* theta, int64_t B, double* lnl, double* g
     PES_CHECK_CUDA(cudaStreamWaitEvent(st, p->mixed->ev_hd, 0));
     {
       ProfScope ps(p, kKFinalize, st);
-      k_mixed_finalize<<<ceil_div(B, 64), 64, 0, st>>>(p->dev, M, blocks, B, lnl, status);
+      k_mixed_finalize<<<ceil_div(B, kSampleWarps), kSampleWarps * 32, 0, st>>>(p->dev, M, blocks, B, lnl, status);
     }
     PES_CHECK_LAUNCH();
     return PES_OK;
@@ -4162,7 +4237,7 @@ int mixed_lnl(PesPlan* p, const double* theta, int64_t B, double* lnl, double* g
   }
   {
     ProfScope ps(p, kKFinalize, st);
-    k_mixed_grad_finalize<<<ceil_div(B, 64), 64, 0, st>>>(M, B, -2.0 * p->dev.df, grad);
+    k_mixed_grad_finalize<<<ceil_div(11 * B, kSampleWarps), kSampleWarps * 32, 0, st>>>(M, B, -2.0 * p->dev.df, grad);
   }
   PES_CHECK_LAUNCH();
   return PES_OK;
