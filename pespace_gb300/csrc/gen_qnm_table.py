@@ -166,7 +166,6 @@ def main(out_path):
         "// Generated by gen_qnm_table.py (Leaver's continued fractions); do not edit.",
         "// Kerr quasi-normal modes (s = -2, n = 0): M omega = re - i im on a grid",
         "// uniform in u = sqrt(1 - a), with natural-spline second derivatives.",
-        "#pragma once",
         "",
         f"#define PES_QNM_MODES {len(MODES)}",
         f"#define PES_QNM_NODES {N_NODES}",

@@ -337,6 +337,17 @@ PES_HD void tdi_channels(const Cx<double>& D, const Cx<double>& P, int orth, con
 // (negative a: the retrograde continuation).  a is clamped to +-PES_QNM_A_MAX.
 #define PES_QNM_STORAGE __device__ static const
 #include "pes_qnm_table.h"
+#undef PES_QNM_STORAGE
+// The tables of the set-up exist on the host too: the plugins set one sample up there.
+namespace host_tables {
+#define PES_QNM_STORAGE static const
+#include "pes_qnm_table.h"
+}  // namespace host_tables
+#ifdef __CUDA_ARCH__
+#define PES_ON_SIDE(device, host) device
+#else
+#define PES_ON_SIDE(device, host) host
+#endif
 
 template <class T>
 PES_HD void qnm_interp(int mode, const T& a, T& wR, T& wI) {
@@ -350,10 +361,10 @@ PES_HD void qnm_interp(int mode, const T& a, T& wR, T& wI) {
   const T t = (u - (PES_QNM_U0 + i * h)) / h;
   const T s = 1.0 - t;
   const T cA = (s * s * s - s) * (h * h / 6.0), cB = (t * t * t - t) * (h * h / 6.0);
-  const double* re = kQnmTable[mode][0];
-  const double* re2 = kQnmTable[mode][1];
-  const double* im = kQnmTable[mode][2];
-  const double* im2 = kQnmTable[mode][3];
+  const double* re = PES_ON_SIDE(kQnmTable, host_tables::kQnmTable)[mode][0];
+  const double* re2 = PES_ON_SIDE(kQnmTable, host_tables::kQnmTable)[mode][1];
+  const double* im = PES_ON_SIDE(kQnmTable, host_tables::kQnmTable)[mode][2];
+  const double* im2 = PES_ON_SIDE(kQnmTable, host_tables::kQnmTable)[mode][3];
   wR = s * re[i] + t * re[i + 1] + cA * re2[i] + cB * re2[i + 1];
   wI = s * im[i] + t * im[i + 1] + cA * im2[i] + cB * im2[i + 1];
 }
@@ -368,27 +379,29 @@ constexpr double kMfCut = 0.2;         // PhenomD is zero above Mf = 0.2
 // xi = chi_PN - 1.
 enum { kFV2, kFG1, kFG2, kFG3, kFS1, kFS2, kFS3, kFS4, kFB1, kFB2, kFB3, kFA1, kFA2, kFA3, kFA4, kFA5,
        kFR1, kFR2, kFR3, kFCount };
-__device__ static const double kPhenomFits[kFCount][11] = {
-  {0.8149838730507785, 2.5747553517454658, 1.1610198035496786, -2.3627771785551537, 6.771038707057573, 0.7570782938606834, -2.7256896890432474, 7.1140380397149965, 0.1766934149293479, -0.7978690983168183, 2.1162391502005153},
-  {0.006927402739328343, 0.03020474290328911, 0.006308024337706171, -0.12074130661131138, 0.26271598905781324, 0.0034151773647198794, -0.10779338611188374, 0.27098966966891747, 0.0007374185938559283, -0.02749621038376281, 0.0733150789135702},
-  {1.010344404799477, 0.0008993122007234548, 0.283949116804459, -4.049752962958005, 13.207828172665366, 0.10396278486805426, -7.025059158961947, 24.784892370130475, 0.03093202475605892, -2.6924023896851663, 9.609374464684983},
-  {1.3081615607036106, -0.005537729694807678, -0.06782917938621007, -0.6689834970767117, 3.403147966134083, -0.05296577374411866, -0.9923793203111362, 4.820681208409587, -0.006134139870393713, -0.38429253308696365, 1.7561754421985984},
-  {2096.551999295543, 1463.7493168261553, 1312.5493286098522, 18307.330017082117, -43534.1440746107, -833.2889543511114, 32047.31997183187, -108609.45037520859, 452.25136398112204, 8353.439546391714, -44531.3250037322},
-  {-10114.056472621156, -44631.01109458185, -6541.308761668722, -266959.23419307504, 686328.3229317984, 3405.6372187679685, -437507.7208209015, 1.6318171307344697e6, -7462.648563007646, -114585.25177153319, 674402.4689098676},
-  {22933.658273436497, 230960.00814979506, 14961.083974183695, 1.1940181342318142e6, -3.1042239693052764e6, -3038.166617199259, 1.8720322849093592e6, -7.309145012085539e6, 42738.22871475411, 467502.018616601, -3.064853498512499e6},
-  {-14621.71522218357, -377812.8579387104, -9608.682631509726, -1.7108925257214056e6, 4.332924601416521e6, -22366.683262266528, -2.5019716386377467e6, 1.0274495902259542e7, -85360.30079034246, -570025.3441737515, 4.396844346849777e6},
-  {97.89747327985583, -42.659730877489224, 153.48421037904913, -1417.0620760768954, 2752.8614143665027, 138.7406469558649, -1433.6585075135881, 2857.7418952430758, 41.025109467376126, -423.680737974639, 850.3594335657173},
-  {-3.282701958759534, -9.051384468245866, -12.415449742258042, 55.4716447709787, -106.05109938966335, -11.953044553690658, 76.80704618365418, -155.33172948098394, -3.4129261592393263, 25.572377569952536, -54.408036707740465},
-  {-0.000025156429818799565, 0.000019750256942201327, -0.000018370671469295915, 0.000021886317041311973, 0.00008250240316860033, 7.157371250566708e-6, -0.000055780000112270685, 0.00019142082884072178, 5.447166261464217e-6, -0.00003220610095021982, 0.00007974016714984341},
-  {43.31514709695348, 638.6332679188081, -32.85768747216059, 2415.8938269370315, -5766.875169379177, -61.85459307173841, 2953.967762459948, -8986.29057591497, -21.571435779762044, 981.2158224673428, -3239.5664895930286},
-  {-0.07020209449091723, -0.16269798450687084, -0.1872514685185499, 1.138313650449945, -2.8334196304430046, -0.17137955686840617, 1.7197549338119527, -4.539717148261272, -0.049983437357548705, 0.6062072055948309, -1.682769616644546},
-  {9.5988072383479, -397.05438595557433, 16.202126189517813, -1574.8286986717037, 3600.3410843831093, 27.092429659075467, -1786.482357315139, 5152.919378666511, 11.175710130033895, -577.7999423177481, 1808.730762932043},
-  {-0.02989487384493607, 1.4022106448583738, -0.07356049468633846, 0.8337006542278661, 0.2240008282397391, -0.055202870001177226, 0.5667186343606578, 0.7186931973380503, -0.015507437354325743, 0.15750322779277187, 0.21076815715176228},
-  {0.9974408278363099, -0.007884449714907203, -0.059046901195591035, 1.3958712396764088, -4.516631601676276, -0.05585343136869692, 1.7516580039343603, -5.990208965347804, -0.017945336522161195, 0.5965097794825992, -2.0608879367971804},
-  {3931.8979897196614, -17395.758706812805, 3132.375545898835, 343965.86092361377, -1.2162565819981997e6, -70698.00600428853, 1.383907177859705e6, -3.9662761890979446e6, -60017.52423652596, 803515.1181825735, -2.091710365941658e6},
-  {-40105.47653771657, 112253.0169706701, 23561.696065836168, -3.476180699403351e6, 1.137593670849482e7, 754313.1127166454, -1.308476044625268e7, 3.6444584853928134e7, 596226.612472288, -7.4277901143564405e6, 1.8928977514040343e7},
-  {83208.35471266537, -191237.7264145924, -210916.2454782992, 8.71797508352568e6, -2.6914942420669552e7, -1.9889806527362722e6, 3.0888029960154563e7, -8.390870279256162e7, -1.4535031953446497e6, 1.7063528990822166e7, -4.2748659731120914e7},
-};
+#define PES_PHENOM_FITS { \
+  {0.8149838730507785, 2.5747553517454658, 1.1610198035496786, -2.3627771785551537, 6.771038707057573, 0.7570782938606834, -2.7256896890432474, 7.1140380397149965, 0.1766934149293479, -0.7978690983168183, 2.1162391502005153}, \
+  {0.006927402739328343, 0.03020474290328911, 0.006308024337706171, -0.12074130661131138, 0.26271598905781324, 0.0034151773647198794, -0.10779338611188374, 0.27098966966891747, 0.0007374185938559283, -0.02749621038376281, 0.0733150789135702}, \
+  {1.010344404799477, 0.0008993122007234548, 0.283949116804459, -4.049752962958005, 13.207828172665366, 0.10396278486805426, -7.025059158961947, 24.784892370130475, 0.03093202475605892, -2.6924023896851663, 9.609374464684983}, \
+  {1.3081615607036106, -0.005537729694807678, -0.06782917938621007, -0.6689834970767117, 3.403147966134083, -0.05296577374411866, -0.9923793203111362, 4.820681208409587, -0.006134139870393713, -0.38429253308696365, 1.7561754421985984}, \
+  {2096.551999295543, 1463.7493168261553, 1312.5493286098522, 18307.330017082117, -43534.1440746107, -833.2889543511114, 32047.31997183187, -108609.45037520859, 452.25136398112204, 8353.439546391714, -44531.3250037322}, \
+  {-10114.056472621156, -44631.01109458185, -6541.308761668722, -266959.23419307504, 686328.3229317984, 3405.6372187679685, -437507.7208209015, 1.6318171307344697e6, -7462.648563007646, -114585.25177153319, 674402.4689098676}, \
+  {22933.658273436497, 230960.00814979506, 14961.083974183695, 1.1940181342318142e6, -3.1042239693052764e6, -3038.166617199259, 1.8720322849093592e6, -7.309145012085539e6, 42738.22871475411, 467502.018616601, -3.064853498512499e6}, \
+  {-14621.71522218357, -377812.8579387104, -9608.682631509726, -1.7108925257214056e6, 4.332924601416521e6, -22366.683262266528, -2.5019716386377467e6, 1.0274495902259542e7, -85360.30079034246, -570025.3441737515, 4.396844346849777e6}, \
+  {97.89747327985583, -42.659730877489224, 153.48421037904913, -1417.0620760768954, 2752.8614143665027, 138.7406469558649, -1433.6585075135881, 2857.7418952430758, 41.025109467376126, -423.680737974639, 850.3594335657173}, \
+  {-3.282701958759534, -9.051384468245866, -12.415449742258042, 55.4716447709787, -106.05109938966335, -11.953044553690658, 76.80704618365418, -155.33172948098394, -3.4129261592393263, 25.572377569952536, -54.408036707740465}, \
+  {-0.000025156429818799565, 0.000019750256942201327, -0.000018370671469295915, 0.000021886317041311973, 0.00008250240316860033, 7.157371250566708e-6, -0.000055780000112270685, 0.00019142082884072178, 5.447166261464217e-6, -0.00003220610095021982, 0.00007974016714984341}, \
+  {43.31514709695348, 638.6332679188081, -32.85768747216059, 2415.8938269370315, -5766.875169379177, -61.85459307173841, 2953.967762459948, -8986.29057591497, -21.571435779762044, 981.2158224673428, -3239.5664895930286}, \
+  {-0.07020209449091723, -0.16269798450687084, -0.1872514685185499, 1.138313650449945, -2.8334196304430046, -0.17137955686840617, 1.7197549338119527, -4.539717148261272, -0.049983437357548705, 0.6062072055948309, -1.682769616644546}, \
+  {9.5988072383479, -397.05438595557433, 16.202126189517813, -1574.8286986717037, 3600.3410843831093, 27.092429659075467, -1786.482357315139, 5152.919378666511, 11.175710130033895, -577.7999423177481, 1808.730762932043}, \
+  {-0.02989487384493607, 1.4022106448583738, -0.07356049468633846, 0.8337006542278661, 0.2240008282397391, -0.055202870001177226, 0.5667186343606578, 0.7186931973380503, -0.015507437354325743, 0.15750322779277187, 0.21076815715176228}, \
+  {0.9974408278363099, -0.007884449714907203, -0.059046901195591035, 1.3958712396764088, -4.516631601676276, -0.05585343136869692, 1.7516580039343603, -5.990208965347804, -0.017945336522161195, 0.5965097794825992, -2.0608879367971804}, \
+  {3931.8979897196614, -17395.758706812805, 3132.375545898835, 343965.86092361377, -1.2162565819981997e6, -70698.00600428853, 1.383907177859705e6, -3.9662761890979446e6, -60017.52423652596, 803515.1181825735, -2.091710365941658e6}, \
+  {-40105.47653771657, 112253.0169706701, 23561.696065836168, -3.476180699403351e6, 1.137593670849482e7, 754313.1127166454, -1.308476044625268e7, 3.6444584853928134e7, 596226.612472288, -7.4277901143564405e6, 1.8928977514040343e7}, \
+  {83208.35471266537, -191237.7264145924, -210916.2454782992, 8.71797508352568e6, -2.6914942420669552e7, -1.9889806527362722e6, 3.0888029960154563e7, -8.390870279256162e7, -1.4535031953446497e6, 1.7063528990822166e7, -4.2748659731120914e7}, \
+}
+__device__ static const double kPhenomFits[kFCount][11] = PES_PHENOM_FITS;
+static const double kPhenomFitsHost[kFCount][11] = PES_PHENOM_FITS;
 
 // Per-sample coefficient block.  Psi is the full phase in h22 = A e^{-i Psi}
 // (time and phase alignment folded in); tf = dPsi/df / (2 pi) in seconds.
@@ -411,7 +424,7 @@ struct PhenomDCoef {
 
 // One coefficient fit and its partial derivatives: out = (value, d/d eta, d/d xi).
 PES_HD void phenom_fit_row(int w, double eta, double xi, double out[3]) {
-  const double* c = kPhenomFits[w];
+  const double* c = PES_ON_SIDE(kPhenomFits, kPhenomFitsHost)[w];
   const double a0 = c[2] + eta * (c[3] + eta * c[4]), a1 = c[5] + eta * (c[6] + eta * c[7]),
                a2 = c[8] + eta * (c[9] + eta * c[10]);
   out[0] = c[0] + c[1] * eta + xi * (a0 + xi * (a1 + xi * a2));
@@ -776,7 +789,7 @@ PES_HD void phenomd_setup(const T* th, double f_ref, double (*rows)[3], int lane
 
 template <class T>
 PES_HD T phenom_fit(int w, const T& eta, const T& xi) {
-  const double* c = kPhenomFits[w];
+  const double* c = PES_ON_SIDE(kPhenomFits, kPhenomFitsHost)[w];
   T eta2 = eta * eta;
   return c[0] + c[1] * eta + xi * (c[2] + c[3] * eta + c[4] * eta2) +
          xi * xi * ((c[5] + c[6] * eta + c[7] * eta2) + xi * (c[8] + c[9] * eta + c[10] * eta2));
@@ -1094,8 +1107,11 @@ PES_HD void phenomd_setup_serial(const T* th, double f_ref, double (*rows)[3], i
 // Polarisations: hp = sum P_lm h_lm, hc = i sum C_lm h_lm (s = -2 spherical
 // harmonics at azimuth 0; (2,2) gives (1 + cos^2 i)/2 and -cos i).
 constexpr int kHMModes = 6;
-__device__ __constant__ static const int kHMlm[kHMModes][3] = {  // l, m, quarter turns of H_lm
-    {2, 2, 0}, {2, 1, 1}, {3, 3, 3}, {3, 2, 0}, {4, 4, 2}, {4, 3, 3}};
+// l, m, quarter turns of H_lm
+#define PES_HM_LM { \
+    {2, 2, 0}, {2, 1, 1}, {3, 3, 3}, {3, 2, 0}, {4, 4, 2}, {4, 3, 3}}
+__device__ __constant__ static const int kHMlm[kHMModes][3] = PES_HM_LM;
+static const int kHMlmHost[kHMModes][3] = PES_HM_LM;
 
 template <class T>
 struct HMMode {
@@ -1129,22 +1145,24 @@ struct PhenomHMCoef {
 // Prefactors of the s = -2 harmonics' sums over k = 0, 1, 2 for (l, m) and
 // (l, -m) of each mode: sqrt((2l+1)/4pi) (-1)^k sqrt((l+m)! (l-m)! (l+2)! (l-2)!)
 // / ((l+m-k)! (l-2-k)! k! (k+2-m)!), 0 where a factorial has no value.
-__device__ static const double kHMHarm[kHMModes][2][3] = {
-    {{0.63078313050504, 0.0, 0.0}, {0.63078313050504, 0.0, 0.0}},
-    {{1.26156626101008, 0.0, 0.0}, {1.26156626101008, 0.0, 0.0}},
-    {{0.0, -1.8281831978578629, 0.0}, {1.8281831978578629, 0.0, 0.0}},
-    {{0.7463526651802308, -3.731763325901154, 0.0}, {3.731763325901154, -0.7463526651802308, 0.0}},
-    {{0.0, 0.0, 4.478115991081385}, {4.478115991081385, 0.0, 0.0}},
-    {{0.0, -3.166506184233564, 9.499518552700692}, {9.499518552700692, -3.166506184233564, 0.0}}};
+#define PES_HM_HARM { \
+    {{0.63078313050504, 0.0, 0.0}, {0.63078313050504, 0.0, 0.0}}, \
+    {{1.26156626101008, 0.0, 0.0}, {1.26156626101008, 0.0, 0.0}}, \
+    {{0.0, -1.8281831978578629, 0.0}, {1.8281831978578629, 0.0, 0.0}}, \
+    {{0.7463526651802308, -3.731763325901154, 0.0}, {3.731763325901154, -0.7463526651802308, 0.0}}, \
+    {{0.0, 0.0, 4.478115991081385}, {4.478115991081385, 0.0, 0.0}}, \
+    {{0.0, -3.166506184233564, 9.499518552700692}, {9.499518552700692, -3.166506184233564, 0.0}}}
+__device__ static const double kHMHarm[kHMModes][2][3] = PES_HM_HARM;
+static const double kHMHarmHost[kHMModes][2][3] = PES_HM_HARM;
 
 // s = -2 spherical harmonic at azimuth 0 of mode `mode` (sgn 0) or of its -m
 // (sgn 1) from ch = cos(iota / 2), sh = sin(iota / 2): sqrt((2l+1)/4pi) d^l_{m,2}
 template <class T>
 PES_HD T hm_sylm(int mode, int sgn, const T& ch, const T& sh) {
-  const int l = kHMlm[mode][0], m = sgn ? -kHMlm[mode][1] : kHMlm[mode][1];
+  const int l = PES_ON_SIDE(kHMlm, kHMlmHost)[mode][0], m = sgn ? -PES_ON_SIDE(kHMlm, kHMlmHost)[mode][1] : PES_ON_SIDE(kHMlm, kHMlmHost)[mode][1];
   T sum = lift<T>(0.0);
   for (int k = 0; k < 3; ++k) {
-    const double c = kHMHarm[mode][sgn][k];
+    const double c = PES_ON_SIDE(kHMHarm, kHMHarmHost)[mode][sgn][k];
     if (c == 0.0) continue;
     T term = lift<T>(c);
     for (int e = 0; e < 2 * l + m - 2 * k - 2; ++e) term = term * ch;
@@ -1239,7 +1257,7 @@ template <class T>
 PES_HD void phenomhm_eval(const PhenomDCoef<T>& c, const PhenomHMCoef<T>& h, int k, const T& Mf, T& amp, T& psi,
                           T& tf, T* f22_out) {
   const HMMode<T>& md = h.md[k];
-  const int m = kHMlm[k][1];
+  const int m = PES_ON_SIDE(kHMlm, kHMlmHost)[k][1];
   const T f22 = k == 0 ? Mf : hm_amp_map<T>(md, m, Mf);
   if (f22_out) *f22_out = f22;
   const T u = dcbrt(f22);
@@ -1271,7 +1289,7 @@ PES_HD void hm_kink(const PhenomDCoef<T>& c, const PhenomHMCoef<T>& h, int k, T&
     return;
   }
   const HMMode<T>& md = h.md[k];
-  const double m = kHMlm[k][1];
+  const double m = PES_ON_SIDE(kHMlm, kHMlmHost)[k][1];
   const T fp = md.fpeak, x = fp - c.fRD, a = md.g3fDMeff;
   const T D = x * x + a * a;
   const T A = c.g1 * a / D * dexp(-c.g2 * x / a);
@@ -1308,11 +1326,11 @@ template <class T, int kRole = 3>
 PES_HD void phenomhm_mode(const T* th, const PhenomDCoef<T>& c, int k, HMMode<T>& md) {
   const T one = lift<T>(1.0);
   constexpr double nrm = 0.31539156525252;  // 2 sqrt(5/(64 pi))
-  const int l = kHMlm[k][0], m = kHMlm[k][1];
+  const int l = PES_ON_SIDE(kHMlm, kHMlmHost)[k][0], m = PES_ON_SIDE(kHMlm, kHMlmHost)[k][1];
   md.tm = lift<T>(2.0 / m);
   md.hm = lift<T>(0.5 * m);
   md.tpm = lift<T>(2.0 * kPi / m);
-  md.qt = lift<T>(kHMlm[k][2] * (0.5 * kPi));
+  md.qt = lift<T>(PES_ON_SIDE(kHMlm, kHMlmHost)[k][2] * (0.5 * kPi));
   const T ch = dsqrt(0.5 * (1.0 + th[5])), sh = dsqrt(0.5 * (1.0 - th[5]));
   const T Yp = hm_sylm<T>(k, 0, ch, sh), Ym = hm_sylm<T>(k, 1, ch, sh);
   const double sg = (l & 1) ? -1.0 : 1.0;

@@ -1,12 +1,13 @@
 // Granular drop-in entry points: one per reference plugin method (orbit
 // vectors, single-link response, TDI combination, Whittle likelihood) plus the
-// IMRPhenomD waveform producer.  FP64 throughout, one thread per frequency.
+// IMRPhenomD / IMRPhenomHM waveform producers.  FP64 throughout, one thread per frequency.
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <mutex>
 
 #include "pes_abi_common.cuh"
+#include "pes_freq.cuh"
 #include "pes_physics.cuh"
 
 namespace pes {
@@ -36,26 +37,156 @@ __global__ void k_orbit_vectors(PesOrbit o, const double* __restrict__ t, int64_
     }
 }
 
-__global__ void k_response_links(PesOrbit o, Polar<double> pol, const double* __restrict__ freqs, int64_t n,
-                                 int nmodes, const double2* __restrict__ hp, const double2* __restrict__ hc,
-                                 const double* __restrict__ tf, double tc, double2* __restrict__ links) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double f = freqs[i];
-  // antenna.py:435: exp(-2 pi i f tc)
-  Cx<double> ts;
-  dsincos(-2.0 * kPi * f * tc, &ts.im, &ts.re);
-  Cx<double> acc[6];
-  for (int m = 0; m < nmodes; ++m) {
-    double2 a = hp[m * n + i], b = hc[m * n + i];
-    Cx<double> p = cmul(cx(a.x, a.y), ts), c = cmul(cx(b.x, b.y), ts);
-    Cx<double> L[6];
-    single_links<double>(o, f, p, c, tf[m * n + i] + tc, pol, L);
-#pragma unroll
-    for (int l = 0; l < 6; ++l) acc[l] = (m == 0) ? L[l] : acc[l] + L[l];
+// The response's trigonometric polynomials in the orbital angle, [1, c1, s1, c2,
+// s2], of one source and detector (the value part of RespTab, from the orbit's
+// closed form on the host): the arms of links 12 and 23 along the polarisation
+// axes, the delays k.(x - x0) of nodes 1 and 2, and k.x0.
+struct LinkArg {
+  double np[2][5], nq[2][5], y[2][5], k0[2];
+  double om[2], ph[2];  // revolution, rotation: rate and initial angle
+  double arm_sec, tc;
+  int32_t helio;
+  int32_t pad;
+};
+
+static void link_arg(const PesOrbit& ob, double lam, double beta, double psi, double tc, LinkArg& o) {
+  const double sl = std::sin(lam), cl = std::cos(lam), sb = std::sin(beta), cb = std::cos(beta);
+  const double sp = std::sin(psi), cp = std::cos(psi);
+  const double p[3] = {sl * cp - cl * sb * sp, -cl * cp - sl * sb * sp, cb * sp};
+  const double q[3] = {-sl * sp - cl * sb * cp, cl * sp - sl * sb * cp, cb * cp};
+  const double k[3] = {-(cb * cl), -(cb * sl), -sb};
+  double x[3][3][5] = {};  // [node][axis][term]
+  const double r = ob.r_sec;
+  for (int n = 0; n < 3; ++n) {
+    if (ob.kind == 0) {
+      const double ck = ob.ck[n], sk = ob.sk[n];
+      x[n][0][0] = -1.5 * r * ck;
+      x[n][0][3] = 0.5 * r * ck;
+      x[n][0][4] = 0.5 * r * sk;
+      x[n][1][0] = -1.5 * r * sk;
+      x[n][1][3] = -0.5 * r * sk;
+      x[n][1][4] = 0.5 * r * ck;
+      x[n][2][1] = -1.7320508075688772 * r * ck;
+      x[n][2][2] = -1.7320508075688772 * r * sk;
+    } else {
+      // angle + 2 pi n / 3: cos = c1 a - s1 b, sin = s1 a + c1 b
+      const double a = n == 0 ? 1.0 : -0.5, b = n == 0 ? 0.0 : (n == 1 ? 0.86602540378443865 : -0.86602540378443865);
+      const double S[3] = {ob.sbeta_ref * ob.clam_ref, ob.sbeta_ref * ob.slam_ref, -ob.cbeta_ref};
+      const double K[3] = {ob.slam_ref, -ob.clam_ref, 0.0};
+      for (int j = 0; j < 3; ++j) {
+        x[n][j][1] = r * (S[j] * b + K[j] * a);
+        x[n][j][2] = r * (S[j] * a - K[j] * b);
+      }
+    }
   }
+  const double iL = 1.0 / ob.arm_sec;
+  for (int n = 0; n < 2; ++n)
+    for (int t = 0; t < 5; ++t) {
+      double np = 0.0, nq = 0.0, y = 0.0;
+      for (int j = 0; j < 3; ++j) {
+        const double a = (x[n + 1][j][t] - x[n][j][t]) * iL;
+        np += a * p[j];
+        nq += a * q[j];
+        y += k[j] * x[n][j][t];
+      }
+      o.np[n][t] = np;
+      o.nq[n][t] = nq;
+      o.y[n][t] = y;
+    }
+  o.k0[0] = k[0] * kAUsec;
+  o.k0[1] = k[1] * kAUsec;
+  o.om[0] = ob.omega_revolution;
+  o.om[1] = ob.omega_rotation;
+  o.ph[0] = ob.revolution_initial;
+  o.ph[1] = ob.rotation_initial;
+  o.arm_sec = ob.arm_sec;
+  o.tc = tc;
+  o.helio = ob.kind == 0;
+  o.pad = 0;
+}
+
+constexpr int kLinkThreads = 128;
+
+// Six links of every bin, the modes summed.  FP64-bound: about 215 FP64
+// instructions per mode (the plain formulae with the library's sines took 514).
+__global__ void __launch_bounds__(kLinkThreads) k_response_links(const __grid_constant__ LinkArg a, const double* __restrict__ freqs,
+                                                        int64_t n, int nmodes, const double2* __restrict__ hp,
+                                                        const double2* __restrict__ hc, const double* __restrict__ tf,
+                                                        double2* __restrict__ links) {
+  __shared__ double2 tab[kTrig];
+  fill_trig(tab);
+  __syncthreads();
+  const int64_t i = blockIdx.x * (int64_t)kLinkThreads + threadIdx.x;
+  if (i < n) {
+    const double f = freqs[i], pif = kPi * f, w2 = 2.0 * kPi * f, aL = pif * a.arm_sec;
+    const int tier = sinc_tier(2.0 * fabs(aL));
+    // 2 pi f t_c, rounded as the plain formula's argument is, whole turns removed
+    double ptc;
+    {
+      const double p = w2 * a.tc, kf = fma(p, k64InvTwoPi, k64Magic) - k64Magic;
+      ptc = fma(-kf, k64TwoPiLo, fma(-kf, k64TwoPi, p));
+    }
+    double ar[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, ai[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll 1
+    for (int m = 0; m < nmodes; ++m) {
+      const double2 h1 = hp[m * n + i], h2 = hc[m * n + i];
+      const double t = tf[m * n + i];
+      // above its cut a mode is zero, and so are its links
+      if (h1.x == 0.0 && h1.y == 0.0 && h2.x == 0.0 && h2.y == 0.0 && isfinite(t)) continue;
+      const double T = t + a.tc;
+      double ca, sa, c1, s1, c2 = 0.0, s2 = 0.0;
+      sincos64(tab, fma(a.om[0], T, a.ph[0]), &sa, &ca);
+      c1 = ca;
+      s1 = sa;
+      if (a.helio) {
+        c2 = fma(c1, c1, -(s1 * s1));
+        s2 = 2.0 * (s1 * c1);
+      } else {
+        sincos64(tab, fma(a.om[1], T, a.ph[1]), &s1, &c1);
+      }
+      auto poly = [&](const double* Y) {
+        double v = fma(Y[1], c1, Y[2] * s1);
+        if (a.helio) v += fma(Y[3], c2, fma(Y[4], s2, Y[0]));
+        return v;
+      };
+      // -i a e^{-2 pi i f (t_c + k.x0)} times the polarisations
+      double sn, cs;
+      sincos64(tab, fma(w2, fma(a.k0[0], ca, a.k0[1] * sa), ptc), &sn, &cs);
+      sn *= aL;
+      cs *= aL;
+      const double pr_ = fma(h1.y, cs, -(h1.x * sn)), pi_ = -fma(h1.x, cs, h1.y * sn);
+      const double xr = 2.0 * fma(h2.y, cs, -(h2.x * sn)), xi = -2.0 * fma(h2.x, cs, h2.y * sn);
+      double th[3], np[3], nq[3];
 #pragma unroll
-  for (int l = 0; l < 6; ++l) links[l * n + i] = make_double2(acc[l].re, acc[l].im);
+      for (int k = 0; k < 2; ++k) {
+        th[k] = pif * poly(a.y[k]);
+        np[k] = poly(a.np[k]);
+        nq[k] = poly(a.nq[k]);
+      }
+      th[2] = -(th[0] + th[1]);
+      np[2] = np[0] + np[1];  // (its sign drops out of the patterns)
+      nq[2] = nq[0] + nq[1];
+#pragma unroll
+      for (int pr = 0; pr < 3; ++pr) {
+        const int k2 = (pr + 1) % 3;
+        const double Fp = fma(np[pr], np[pr], -(nq[pr] * nq[pr])), Fx = np[pr] * nq[pr];  // half of Fx
+        const double gr = fma(Fp, pr_, Fx * xr), gi = fma(Fp, pi_, Fx * xi);
+        double es, ec;
+        sincos64(tab, aL - th[(pr + 2) % 3], &es, &ec);  // a + th[pr] + th[k2]
+        const double br = fma(gr, ec, gi * es), bi = fma(gi, ec, -(gr * es));
+        const double dl = th[k2] - th[pr];
+        double sp, sm, d;
+        sinc64<false>(tab, tier, aL + dl, &sp, &d);
+        sinc64<false>(tab, tier, aL - dl, &sm, &d);
+        ar[2 * pr] = fma(sp, br, ar[2 * pr]);
+        ai[2 * pr] = fma(sp, bi, ai[2 * pr]);
+        ar[2 * pr + 1] = fma(sm, br, ar[2 * pr + 1]);
+        ai[2 * pr + 1] = fma(sm, bi, ai[2 * pr + 1]);
+      }
+    }
+#pragma unroll
+    for (int l = 0; l < 6; ++l) links[l * n + i] = make_double2(ar[l], ai[l]);
+  }
 }
 
 __global__ void k_tdi(const double* __restrict__ freqs, int64_t n, double arm, int gen20, int orth,
@@ -153,77 +284,291 @@ static int whittle_scratch(double** out) {
   return PES_OK;
 }
 
-struct ThetaArg {
-  double v[11];
+// IMRPhenomD / IMRPhenomHM modes on an array of frequencies.  The parameters are
+// the host's, so the host sets the sample up (a few microseconds; a set-up by
+// one warp of every block was a serial FP64 chain of 45 us and half of the work
+// of six modes on 150 000 bins) and passes each mode's coefficients, rescaled
+// to frequencies in Hz, as kernel arguments.  A thread takes one bin of every
+// mode: the powers and the logarithm of f are shared by the modes, and in the
+// inspiral a mode is two polynomials, a sine and a cosine.  Bound by the FP64
+// pipe: about 90 FP64 instructions per mode and 90 per bin; six modes go to two
+// threads, since the bins below the cut alone leave some SM partitions a warp
+// more than others.  (bilby's call on one detector, 125 410 bins: 519 -> 212 us
+// with the response below; six modes on three detectors, 149 850 bins: 4.70 -> 1.32 ms.)
+struct WaveMode {
+  // phase: inspiral f^{-5/3} sum pin_j f^{j/3} + (lg0 + lg1 f^{1/3}) ln(f)/3 below fj1;
+  // it0 + it1 f + it2 x^{-3} + it3 ln x, x = ap f + bp, to fj2;
+  // mr0 + mr1 f + mr2 / f + mr3 f^{3/4} + mr4 atan((f - f5) / fd) above
+  double pin[12], rin[12], lg0, lg1;  // rin_j = (j - 5) pin_j / (6 pi)
+  double it0, it1, it2, it3, ap, bp;
+  double mr0, mr1, mr2, mr3, mr4, f5, fd, ifd;
+  double fj1, fj2;
+  // amplitude: a0 f^{-7/6} (1 + sum ai_j f^{(j+2)/3}) below fa; a1 y^{-7/6} Ahat(y)
+  // at the mapped frequency y = sum y_j (f - fa)^j to fb; a2 f^{-7/6} Ahat(R f) above
+  double a0, a1, a2, ai[8], dl[5], y1, y2, y3, fa, fb, fpk, R;
+  double gm, w2, fr, gx, ymax;
+  // post-Newtonian ratio (b1 v + b2 v^2 + b3 v^3) / (1 + h2 v^2 + 2 pi v^3), v = cv f^{1/3}
+  // below fa, va (2 - exp(1 - f / fa))^{1/3} above
+  double b1, b2, b3, h2, cv, va, ifa;
+  double P, C;                        // hp = P h, hc = i C h
+};
+constexpr int kWaveThreads = 128;
+template <int kModes>
+struct WaveArg {
+  WaveMode md[kModes];
 };
 
-// h22 = A e^{-i Psi}; hp = pfac h22, hc = -i cfac h22; t(f) from dPsi/df.
-__global__ void k_phenomd(ThetaArg th, double f_ref, double f_cut, const double* __restrict__ freqs, int64_t n,
-                          double2* __restrict__ hp, double2* __restrict__ hc, double* __restrict__ tf) {
-  __shared__ PhenomDCoef<double> c;
-  __shared__ double rows[kFCount][3];
-  if (threadIdx.x < 32) {
-    PhenomDCoef<double> own;
-    phenomd_setup<double>(th.v, f_ref, rows, threadIdx.x, 32, 0xffffffffu, own);
-    if (threadIdx.x == 0) c = own;
-  }
-  __syncthreads();
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double f = freqs[i];
-  const double Mf = c.Msec * f;
-  if (f > f_cut || Mf > kMfCut) {
-    hp[i] = make_double2(0.0, 0.0);
-    hc[i] = make_double2(0.0, 0.0);
-    tf[i] = 0.0;
-    return;
-  }
-  double amp, psi, t;
-  phenomd_eval<double>(c, Mf, amp, psi, t);
-  double s, co;
-  dsincos(psi, &s, &co);
-  hp[i] = make_double2(c.pfac * amp * co, -(c.pfac * amp * s));
-  hc[i] = make_double2(-(c.cfac * amp * s), -(c.cfac * amp * co));
-  tf[i] = t;
+// host: products and quotients of pairs hi + lo (the leading phase terms reach
+// 1e5 rad: their coefficients are rounded once)
+struct DD {
+  double h, l;
+};
+static DD dd_two(double a, double b) {
+  const double s = a + b, t = s - a;
+  return {s, (a - (s - t)) + (b - t)};
+}
+static DD dd_mul(const DD& a, const DD& b) {
+  const double p = a.h * b.h;
+  return dd_two(p, std::fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h));
+}
+static DD dd_div(const DD& a, const DD& b) {
+  const double q = a.h / b.h;
+  const double p = q * b.h, e = std::fma(q, b.h, -p);
+  return dd_two(q, (((a.h - p) - e) + a.l - q * b.l) / b.h);
+}
+static DD dd_cbrt(const DD& a) {
+  const double c = std::cbrt(a.h);
+  const DD c3 = dd_mul(dd_mul({c, 0.0}, {c, 0.0}), {c, 0.0});
+  return dd_two(c, ((a.h - c3.h) + (a.l - c3.l)) / (3.0 * c * c));
 }
 
-// IMRPhenomHM modes on a frequency array: block (x, mode); h_lm = A e^{-i Psi},
-// hp = P_lm h_lm, hc = i C_lm h_lm, t(f) = dPsi_lm/df / (2 pi); zero above the
-// cut and above the mode's mapped Mf = 0.2.  Outputs mode-major (6, n).
-__global__ void k_phenomhm(ThetaArg th, double f_ref, double f_cut, const double* __restrict__ freqs, int64_t n,
-                           double2* __restrict__ hp, double2* __restrict__ hc, double* __restrict__ tf) {
-  __shared__ PhenomDCoef<double> c;
-  __shared__ PhenomHMCoef<double> h;
-  __shared__ double rows[kFCount][3];
-  if (threadIdx.x < 32) {
-    PhenomDCoef<double> own;
-    phenomd_setup<double>(th.v, f_ref, rows, threadIdx.x, 32, 0xffffffffu, own);
-    if (threadIdx.x == 0) {
-      c = own;
-      phenomhm_common<double>(th.v, own, h);
+static void wave_mode(const PhenomDCoef<double>& c, const HMMode<double>& md, const PhenomHMCoef<double>* h, int k,
+                      WaveMode& o) {
+  const double M = c.Msec, iM = 1.0 / M;
+  const double m = (double)kHMlmHost[k][1], hm = 0.5 * m, qt = md.qt;
+  // inspiral at 2 f / m: powers of tm M
+  const DD tm = dd_div({2.0, 0.0}, {m, 0.0}), Mt = dd_mul(tm, {M, 0.0}), cu = dd_cbrt(Mt), one = {1.0, 0.0};
+  const DD icu = dd_div(one, cu), icu2 = dd_mul(icu, icu);
+  DD pw = dd_mul(dd_mul(icu2, icu2), icu);
+  for (int j = 0; j < 12; ++j) {
+    o.pin[j] = dd_mul(pw, {hm * c.pin[j], 0.0}).h;
+    pw = dd_mul(pw, cu);
+  }
+  const double lcu = std::log(cu.h);
+  o.lg0 = hm * c.lg0;
+  o.lg1 = hm * c.lg1 * cu.h;
+  o.pin[5] += o.lg0 * lcu + qt;
+  o.pin[6] += o.lg1 * lcu;
+  for (int j = 0; j < 12; ++j) o.rin[j] = o.pin[j] * ((j - 5) / (6.0 * kPi));
+  // intermediate: 22 phase at x = ap f + bp
+  const double ia = 1.0 / md.aP;
+  o.ap = md.aP;
+  o.bp = md.bP * iM;
+  o.it0 = (c.pint[0] + c.pint[3] * std::log(M) + c.pint[1] * md.bP) * ia + md.cI0 + qt;
+  o.it1 = (c.pint[1] + md.cI1) * M;
+  o.it2 = c.pint[2] * (iM * iM * iM) * ia;
+  o.it3 = c.pint[3] * ia;
+  // merger-ringdown: at Rholm f
+  const double R = md.Rholm, iR = 1.0 / R, RM = R * M, q = std::sqrt(std::sqrt(RM));
+  o.mr0 = c.pm[0] * iR + md.cR0 + qt;
+  o.mr1 = (c.pm[1] + md.cR1) * M;
+  o.mr2 = c.pm[2] * iR / RM;
+  o.mr3 = c.pm[3] * (q * q * q) * iR;
+  o.mr4 = c.pm[4] * iR;
+  o.f5 = c.pm[5] / RM;
+  o.fd = md.fDMeff / RM;
+  o.ifd = RM / md.fDMeff;
+  o.fj1 = md.fiP * iM;
+  o.fj2 = md.frP * iM;
+  // amplitude
+  auto p76 = [](double x) { return 1.0 / (x * std::sqrt(std::cbrt(x))); };
+  o.a0 = c.amp_scale * p76(Mt.h);
+  o.a1 = c.amp_scale * p76(M);
+  o.a2 = c.amp_scale * p76(RM);
+  double s = cu.h * cu.h;
+  for (int j = 0; j < 8; ++j) {
+    o.ai[j] = c.ai[j] * s;
+    s *= cu.h;
+  }
+  s = 1.0;
+  for (int j = 0; j < 5; ++j) {
+    o.dl[j] = md.dl[j] * s;
+    s *= M;
+  }
+  o.fa = md.fiA * iM;
+  o.fb = md.frA * iM;
+  o.ifa = M / md.fiA;
+  o.R = R;
+  {
+    const double t = 2.0 / m, H = o.fb - o.fa, A = t * o.fa, B = R * o.fb;
+    // the cubic Hermite blend in powers of f - fa
+    o.y1 = t;
+    o.y2 = k == 0 ? 0.0 : (3.0 * (B - A) - H * (2.0 * t + R)) / (H * H);
+    o.y3 = k == 0 ? 0.0 : (2.0 * (A - B) + H * (t + R)) / (H * H * H);
+  }
+  o.fpk = md.fpeak * iM;
+  const double w = md.g3fDMeff * iM;
+  o.gm = c.g1 * w * iM;
+  o.w2 = w * w;
+  o.fr = c.fRD * iM;
+  o.gx = c.g2 / w;
+  o.ymax = kMfCut * iM;
+  o.b1 = o.b2 = o.b3 = o.h2 = o.cv = o.va = 0.0;
+  if (k > 0) {
+    const double r2 = std::sqrt(2.0), r23 = std::sqrt(2.0 / 3.0), r57 = 0.84515425472851657;
+    const double a2 = 0.75 * 1.0350983390135313 * h->dlt * r23;
+    if (k == 1) {
+      o.b1 = r2 / 3.0 * h->dlt;
+      o.b2 = -r2 / 2.0 * (h->chia + h->dlt * h->chis);
+      o.b3 = o.b1 * (-17.0 / 28.0 + (5.0 / 7.0) * h->eta);
+    } else if (k == 2) {
+      o.b1 = a2;
+      o.b3 = a2 * (-4.0 + 2.0 * h->eta);
+    } else if (k == 3) {
+      o.b2 = r57 / 3.0 * (1.0 - 3.0 * h->eta);
+    } else if (k == 4) {
+      o.b2 = 8.0 / 9.0 * r57 / r2 * (1.0 - 3.0 * h->eta);
+    } else {
+      o.b3 = 9.0 / (4.0 * 8.3666002653407556) * r23 * h->dlt * (1.0 - 2.0 * h->eta);
     }
-    if (threadIdx.x < kHMModes) phenomhm_mode<double>(th.v, own, threadIdx.x, h.md[threadIdx.x]);
+    o.h2 = -107.0 / 42.0 + (55.0 / 42.0) * h->eta;
+    o.cv = std::cbrt(md.tpm * M);
+    o.va = std::cbrt(md.tpm * md.fiA);
   }
+  o.P = md.P;
+  o.C = md.C;
+}
+
+// y^{-7/6} and y^{1/3}
+__device__ __forceinline__ double pow76(double y, double* u) {
+  *u = cbrt(y);
+  return rcp64(y) * rsqrt(*u);
+}
+__device__ __forceinline__ double wave_mrd(const WaveMode& c, double y) {
+  const double x = y - c.fr;
+  return c.gm * rcp64(fma(x, x, c.w2)) * exp(-(c.gx * x));
+}
+
+template <int kModes>
+__global__ void __launch_bounds__(kWaveThreads) k_wave(const __grid_constant__ WaveArg<kModes> arg, double f_cut,
+                                              const double* __restrict__ freqs, int64_t n, double2* __restrict__ hp,
+                                              double2* __restrict__ hc, double* __restrict__ tf) {
+  __shared__ double2 tab[kTrig];
+  fill_trig(tab);
   __syncthreads();
-  const int k = blockIdx.y;
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int64_t o = (int64_t)k * n + i;
-  const double f = freqs[i];
-  double amp = 0.0, psi = 0.0, t = 0.0, f22 = 0.0;
-  if (f <= f_cut) phenomhm_eval<double>(c, h, k, c.Msec * f, amp, psi, t, &f22);
-  if (f > f_cut || f22 > kMfCut) {
-    hp[o] = make_double2(0.0, 0.0);
-    hc[o] = make_double2(0.0, 0.0);
-    tf[o] = 0.0;
-    return;
+  const int64_t i = blockIdx.x * (int64_t)kWaveThreads + threadIdx.x;
+  if (i < n) {
+    const double f = freqs[i];
+    const bool in = !(f > f_cut);
+    double u = 0.0, jf = 0.0, lf3 = 0.0, iu5 = 0.0, p76 = 0.0;
+    if (in) {
+      u = cbrt(f);
+      jf = rcp64(f);
+      lf3 = log(f) * (1.0 / 3.0);
+      iu5 = (jf * jf) * u;  // u^{-5} = u / f^2
+      p76 = jf * rsqrt(u);
+    }
+#pragma unroll 1
+    for (int k = blockIdx.y; k < kModes; k += gridDim.y) {
+      const WaveMode& c = arg.md[k];
+      const int64_t o = (int64_t)k * n + i;
+      // ---- amplitude (NaN frequencies stay: they are not above the cut)
+      double A, y = 0.0, v = c.cv * u;
+      if (in) {
+        if (f < c.fa || (k > 0 && f == c.fa)) {
+          double p = c.ai[7];
+#pragma unroll
+          for (int j = 6; j >= 0; --j) p = fma(p, u, c.ai[j]);
+          A = c.a0 * p76 * fma(u * u, p, 1.0);
+        } else {
+          if (f < c.fb || k == 0) {
+            const double x = f - c.fa;
+            double uy = u, py = p76;
+            y = f;
+            if (k > 0) {
+              y = fma(x, fma(x, fma(x, c.y3, c.y2), c.y1), c.y1 * c.fa);
+              py = pow76(y, &uy);
+            }
+            const double ah = y >= c.fpk ? wave_mrd(c, y)
+                                         : fma(y, fma(y, fma(y, fma(y, c.dl[4], c.dl[3]), c.dl[2]), c.dl[1]), c.dl[0]);
+            A = c.a1 * py * ah;
+          } else {
+            y = c.R * f;
+            A = c.a2 * p76 * wave_mrd(c, y);
+          }
+          if (k > 0) v = c.va * cbrt(2.0 - exp(1.0 - f * c.ifa));
+        }
+        if (k > 0) {
+          const double v2 = v * v;
+          A *= v * fma(v, fma(v, c.b3, c.b2), c.b1) * rcp64(fma(v2, fma(2.0 * kPi, v, c.h2), 1.0));
+        }
+      }
+      if (!in || y > c.ymax) {
+        hp[o] = make_double2(0.0, 0.0);
+        hc[o] = make_double2(0.0, 0.0);
+        tf[o] = 0.0;
+        continue;
+      }
+      // ---- phase and t(f)
+      double psi, t;
+      if (f < c.fj1) {
+        double p = c.pin[11], r = c.rin[11];
+#pragma unroll
+        for (int j = 10; j >= 0; --j) {
+          p = fma(p, u, c.pin[j]);
+          if (j != 5) r = fma(r, u, c.rin[j]); else r *= u;
+        }
+        const double l1 = c.lg1 * u;
+        psi = fma(p, iu5, (c.lg0 + l1) * lf3);
+        t = jf * fma(r, iu5, fma(l1, lf3 + 1.0, c.lg0) * (1.0 / (6.0 * kPi)));
+      } else if (f < c.fj2) {
+        double jx = jf, l = 3.0 * lf3;
+        if (k > 0) {
+          const double x = fma(c.ap, f, c.bp);
+          jx = rcp64(x);
+          l = log(x);
+        }
+        const double j3 = jx * jx * jx;
+        psi = fma(c.it1, f, fma(c.it2, j3, fma(c.it3, l, c.it0)));
+        t = fma(c.ap * jx, fma(-3.0 * c.it2, j3, c.it3), c.it1) * (1.0 / (2.0 * kPi));
+      } else {
+        const double q = rsqrt(sqrt(f)), x = f - c.f5, rd = rcp64(fma(x, x, c.fd * c.fd));
+        psi = fma(c.mr1, f, fma(c.mr2, jf, fma(c.mr3, f * q, fma(c.mr4, atan64(tab, x * c.ifd), c.mr0))));
+        t = fma(-c.mr2 * jf, jf, fma(0.75 * c.mr3, q, fma(c.mr4 * c.fd, rd, c.mr1))) * (1.0 / (2.0 * kPi));
+      }
+      double sn, cs;
+      sincos64(tab, psi, &sn, &cs);
+      // h = A e^{-i Psi}; hp = P h, hc = i C h
+      const double ap = c.P * A, ac = c.C * A;
+      hp[o] = make_double2(ap * cs, -(ap * sn));
+      hc[o] = make_double2(ac * sn, ac * cs);
+      tf[o] = t;
+    }
   }
-  double s, co;
-  dsincos(psi, &s, &co);
-  const double ap = h.md[k].P * amp, ac = h.md[k].C * amp;
-  hp[o] = make_double2(ap * co, -(ap * s));
-  hc[o] = make_double2(ac * s, ac * co);
-  tf[o] = t;
+}
+
+// The sample's coefficients on the host and the launch.
+template <int kModes>
+static int launch_wave(const double* theta, const double* freqs, int64_t n, double f_ref, double f_cut, double* hp,
+                       double* hc, double* tf, cudaStream_t st) {
+  PhenomDCoef<double> c;
+  double rows[kFCount][3];
+  phenomd_setup<double, 3>(theta, f_ref, rows, 0, 1, 0u, c);
+  PhenomHMCoef<double> h;
+  phenomhm_common<double>(theta, c, h);
+  WaveArg<kModes> arg;
+  for (int k = 0; k < kModes; ++k) {
+    phenomhm_mode<double, 3>(theta, c, k, h.md[k]);
+    wave_mode(c, h.md[k], &h, k, arg.md[k]);
+  }
+  if (kModes == 1) {  // IMRPhenomD's own polarisation factors
+    arg.md[0].P = c.pfac;
+    arg.md[0].C = -c.cfac;
+  }
+  k_wave<kModes><<<dim3(ceil_div(n, kWaveThreads), kModes > 1 ? 2 : 1), kWaveThreads, 0, st>>>(
+      arg, f_cut, freqs, n, reinterpret_cast<double2*>(hp), reinterpret_cast<double2*>(hc), tf);
+  PES_CHECK_LAUNCH();
+  return PES_OK;
 }
 
 }  // namespace pes
@@ -784,11 +1129,11 @@ int pes_response_links(const PesOrbit* orbit, const double* freqs, int64_t n, in
   PES_REQUIRE(orbit->kind == 0 || orbit->kind == 1, "pes_response_links: unknown orbit kind %d", orbit->kind);
   if (n == 0) return PES_OK;
   PES_REQUIRE(freqs && hp && hc && tf && links, "pes_response_links: null pointer");
-  Polar<double> pol;
-  make_polar<double>(lam, ::sin(beta), ::cos(beta), psi, pol);
-  k_response_links<<<ceil_div(n, 128), 128, 0, as_stream(stream)>>>(
-      *orbit, pol, freqs, n, n_modes, reinterpret_cast<const double2*>(hp), reinterpret_cast<const double2*>(hc),
-      tf, tc, reinterpret_cast<double2*>(links));
+  LinkArg arg;
+  link_arg(*orbit, lam, beta, psi, tc, arg);
+  k_response_links<<<ceil_div(n, kLinkThreads), kLinkThreads, 0, as_stream(stream)>>>(
+      arg, freqs, n, n_modes, reinterpret_cast<const double2*>(hp), reinterpret_cast<const double2*>(hc), tf,
+      reinterpret_cast<double2*>(links));
   PES_CHECK_LAUNCH();
   return PES_OK;
 }
@@ -873,13 +1218,7 @@ int pes_phenomd(const double* theta, const double* freqs, int64_t n, double f_re
   PES_REQUIRE(n >= 0, "pes_phenomd: n < 0");
   if (n == 0) return PES_OK;
   PES_REQUIRE(freqs && hp && hc && tf, "pes_phenomd: null pointer");
-  ThetaArg th;
-  for (int j = 0; j < 11; ++j) th.v[j] = theta[j];
-  k_phenomd<<<ceil_div(n, 128), 128, 0, as_stream(stream)>>>(th, f_ref, f_cut_hz, freqs, n,
-                                                             reinterpret_cast<double2*>(hp),
-                                                             reinterpret_cast<double2*>(hc), tf);
-  PES_CHECK_LAUNCH();
-  return PES_OK;
+  return launch_wave<1>(theta, freqs, n, f_ref, f_cut_hz, hp, hc, tf, as_stream(stream));
 }
 
 int pes_phenomhm(const double* theta, const double* freqs, int64_t n, double f_ref, double f_cut_hz, double* hp,
@@ -888,12 +1227,7 @@ int pes_phenomhm(const double* theta, const double* freqs, int64_t n, double f_r
   PES_REQUIRE(n >= 0, "pes_phenomhm: n < 0");
   if (n == 0) return PES_OK;
   PES_REQUIRE(freqs && hp && hc && tf, "pes_phenomhm: null pointer");
-  ThetaArg th;
-  for (int j = 0; j < 11; ++j) th.v[j] = theta[j];
-  k_phenomhm<<<dim3(ceil_div(n, 128), kHMModes), 128, 0, as_stream(stream)>>>(
-      th, f_ref, f_cut_hz, freqs, n, reinterpret_cast<double2*>(hp), reinterpret_cast<double2*>(hc), tf);
-  PES_CHECK_LAUNCH();
-  return PES_OK;
+  return launch_wave<kHMModes>(theta, freqs, n, f_ref, f_cut_hz, hp, hc, tf, as_stream(stream));
 }
 
 int pes_pn_tf(const double* params, int64_t B, const double* freqs, int64_t n, double* tf, void* stream) {

@@ -44,6 +44,23 @@ def _modes(waveform):
     return list(waveform.values())
 
 
+def _stacked(rows, dtype):
+    """The modes' rows as one contiguous (modes, n) CUDA tensor: a view where they
+    are consecutive rows of one block (the waveform producers' containers), else a
+    copy."""
+    # (a lazy conjugate's memory holds the unconjugated numbers)
+    rows = [torch.as_tensor(r, dtype=dtype, device="cuda").resolve_conj().resolve_neg() for r in rows]
+    first = rows[0]
+    if len(rows) == 1:
+        return first[None].contiguous()
+    n = first.numel()
+    step = n * first.element_size()
+    if all(r.dim() == 1 and r.numel() == n and r.is_contiguous() and r.data_ptr() == first.data_ptr() + k * step
+           and r.untyped_storage().data_ptr() == first.untyped_storage().data_ptr() for k, r in enumerate(rows)):
+        return first.as_strided((len(rows), n), (n, 1))
+    return torch.stack(rows)
+
+
 class SingleLinkResponseModel(ABC):
     """antenna.py:326-344: the response plugin interface."""
 
@@ -75,12 +92,11 @@ class FDResponseModelMarset2018(SingleLinkResponseModel):
         freqs = det.tdi_data.frequency_samples
         n = freqs.numel()
         modes = _modes(waveform)
-        hp = torch.stack([torch.as_tensor(m["plus"], dtype=torch.complex128, device="cuda") for m in modes])
-        hc = torch.stack([torch.as_tensor(m["cross"], dtype=torch.complex128, device="cuda") for m in modes])
-        tf = torch.stack([torch.as_tensor(m["tf"], dtype=torch.float64, device="cuda") for m in modes])
+        hp = _stacked([m["plus"] for m in modes], torch.complex128)
+        hc = _stacked([m["cross"] for m in modes], torch.complex128)
+        tf = _stacked([m["tf"] for m in modes], torch.float64)
         if hp.shape[-1] != n:
             raise ValueError(f"waveform length {hp.shape[-1]} differs from the frequency grid ({n})")
-        hp, hc, tf = hp.contiguous(), hc.contiguous(), tf.contiguous()
         _lib.check(_lib.load().pes_response_links(
             det.orbit_model.to_c(), _lib.ptr(freqs), n, len(modes), _lib.ptr(hp), _lib.ptr(hc), _lib.ptr(tf),
             float(lam), float(beta), float(psi), float(tc), _lib.ptr(det.single_link_response),

@@ -22,6 +22,8 @@ from ..waveform.phenomd import IMRPhenomD, theta_from_parameters
 
 def _rows(data, labels, channels):
     idx = [labels.index(c) for c in channels]
+    if idx == list(range(data.shape[0])):  # every channel in order: no copy
+        return data.resolve_conj().resolve_neg().contiguous()
     return data[idx].contiguous()
 
 
