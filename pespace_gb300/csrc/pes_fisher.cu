@@ -8,6 +8,12 @@
 // A block of 64 threads evaluates 64 bins of one detector, stores
 // sqrt(w) dh in shared memory, and its threads then form the 66 pair sums of
 // those bins; per-block partials are summed in a fixed order.
+#include <algorithm>
+#include <cmath>
+#include <cstddef>
+
+#include "pes_ff.cuh"
+#include "pes_freq.cuh"
 #include "pes_plan.cuh"
 
 namespace pes {
@@ -149,60 +155,107 @@ __global__ void k_fisher_final(const SampleBlock<FisherScalar>* __restrict__ blo
   if (status && p == 0) status[s] = blocks[s].status;
 }
 
-// Fisher matrices of mixed plans in FP32, by the structure of the model:
-// h_c = A Y_c(T, lambda, sin beta, psi, cos iota) exp(-i phase), T = t(f) + t_c,
+// Fisher matrices of mixed IMRPhenomD plans in FP32, by the structure of the
+// model: h_c = A Y_c(T, lambda, sin beta, psi, cos iota) exp(-i phase), T = t(f) + t_c,
 // phase = Psi + 2 pi f (k.x0(T, lambda, sin beta) + t_c), with A, Psi, t(f)
 // depending on the mass and spin parameters only.  Its derivatives are
 //   dh/dtheta = (d(A Y)/dtheta - i A Y dphase/dtheta) exp(-i phase),
 // and the phase factor cancels in conj(dh_a) dh_b, so the Fisher needs no
-// phase values: PhenomD runs with FP32 duals over the four mass/spin
-// parameters (A, dPsi, dt), the response per unit amplitude with FP32 duals
-// over (T, lambda, sin beta, psi, cos iota); ln D_L and phi_c are analytic
-// (dh = -h and 2 i h).  A block of 128 threads evaluates 128 bins of one
-// detector, stores sqrt(w) times the 11 complex derivatives in shared memory,
-// and threads 0..65 each sum one pair over those bins (FP32 within the block,
-// FP64 across blocks, fixed order).  Amplitudes are scaled by
-// PC / (MRSUN MTSUN) and the weights by its inverse square to stay in FP32 range.
-constexpr int kFastThreads = 128;
-// ln Mc, q, chi_1, chi_2: float-float values and tangents (the phase tangents
-// are sums of large cancelling terms; FP32 tangents left 1e-4 errors in F_qq
-// at mass ratios near 7)
-using FM = Dual<4, FF, FF>;
-using FR = DualS<5>;  // T, lambda, sin beta, psi, cos iota
+// phase values.  The waveform's part per bin (A, t(f), and the tangents of Psi
+// and t(f) in float-float, of A in FP32, which enters beside Psi's with a factor
+// of 1e-2) is linear in the tangents of the model's coefficients: Horner
+// sums over tabulated powers of f, each sample's coefficients rescaled to them.
+// The response per unit amplitude takes FP32 duals over (T, lambda, sin beta,
+// psi, cos iota); ln D_L and phi_c are analytic (dh = -h and 2 i h).
+//
+// Four warps of a block evaluate 128 bins of one detector and store sqrt(w)
+// times the 11 complex derivatives in shared memory; the fifth sums the 66
+// pairs over the previous 128 (two buffers; FP32 within the 128 bins in their
+// order, FP64 across).  A lane takes up to three pairs of one row, so that it
+// loads 4 complex numbers for 6 products (a thread per pair loaded 12 values for
+// 6, three of four warps waiting).  Float-float dual numbers through the
+// waveform, and FP64 square roots and conversions of the weights per bin, took
+// most of the time before: 100 samples on 125 410 bins 5.21 -> 2.04 ms (1.97 ms of it
+// here, 5 200 FP32 operations per bin and detector, two thirds in the response).
+constexpr int kFastThreads = 128;              // bins per group
+constexpr int kFastBlock = kFastThreads + 32;  // and the summing warp
+constexpr int kFastBlocks = 152 * 2;           // small calls: blocks of the whole call
+using FR = DualS<5>;                           // T, lambda, sin beta, psi, cos iota
 
-struct FisherFastBlock {
-  PhenomDCoef<FM> wf;
+// Per bin, for the FP32 frequency that the response takes too: f, f^{1/3} | 1/f,
+// ln(f)/3 | f^{-5/3}, f^{-1/4} (hi, lo pairs) and f^{-7/6}.
+__global__ void k_fisher_grid(PlanDev P, float4* __restrict__ rows, float2* __restrict__ p76) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= P.nbins) return;
+  const double f = (double)(float)((double)(P.k0 + i) * P.f_step);
+  const double u = cbrt(f);
+  auto row = [](double a, double b) {
+    const FF x = ff_from(a), y = ff_from(b);
+    return make_float4(x.hi, x.lo, y.hi, y.lo);
+  };
+  rows[i] = row(f, u);
+  rows[P.nbins + i] = row(1.0 / f, log(f) / 3.0);
+  rows[2 * P.nbins + i] = row(1.0 / (f * u * u), 1.0 / sqrt(sqrt(f)));
+  const FF g = ff_from(1.0 / (f * sqrt(u)));
+  p76[i] = make_float2(g.hi, g.lo);
+}
+
+// A bin's TDI factors and the square roots of its weights over the amplitudes'
+// scale (zero off the channel mask) in FP32: [n_det][nbins] rows (D, P), (A, E, T, 0).
+__global__ void k_fisher_weights(PlanDev P, double inv_scale2, float4* __restrict__ wt) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int d = blockIdx.y;
+  if (i >= P.nbins) return;
+  const TdiFactor t = P.tdi[(size_t)d * P.nbins + i];
+  const double* w = P.w + (size_t)d * 3 * P.nbins + i;
+  float4* o = wt + (size_t)d * 2 * P.nbins + i;
+  o[0] = make_float4((float)t.dre, (float)t.dim, (float)t.pre, (float)t.pim);
+  o[P.nbins] = make_float4((float)sqrt(w[0] * inv_scale2), (float)sqrt(w[P.nbins] * inv_scale2),
+                           (float)sqrt(w[2 * P.nbins] * inv_scale2), 0.0f);
+}
+
+struct FisherSample {
+  // phase tangents, [term][ln Mc, q, chi_1, chi_2] as hi, lo pairs
+  float2 pin[12][4], lg0[4], lg1[4], pint[4][4], pm[5][4];
+  // t(f): inspiral (j - 5) pin_j / (6 pi), lg / (6 pi); intermediate; merger-ringdown
+  float2 rin[12], rl0, rl1, ri[3], rm[4];  // rm: pm1, pm2, 0.75 pm3, pm4 fd, over 2 pi
+  float2 drin[12][4], drl0[4], drl1[4], dri[3][4], drm[4][4];
+  float2 f5, ifd, fd2;
+  float fd, pm4, df5[4], dfd[4];
+  // amplitude: a0 scaled; Ahat and its tangents (intermediate in (f - fc) / hw)
+  float2 a0, ai[8], ei[5], fc, ihw, gm, w2, fr, gx;
+  float wf;
+  float dlna0[4], dai[8][4], dei[5][4], dlngm[4], dw[4], dfr[4], dgx[4];
+  float fj1, fj2, fa1, fa2;
   Polar<FR> pol;
   FR pfac, cfac;
   float tc;
-  int32_t status;
-  int64_t kcut;
+  int32_t status, kcut;
 };
 
-__global__ void __launch_bounds__(kFastThreads) k_fisher_fast(PlanDev P,
-                                                              const SampleBlock<FisherScalar>* __restrict__ blocks,
-                                                              double* __restrict__ partial) {
-  __shared__ FisherFastBlock sb;
-  __shared__ OrbitF orb[PES_MAX_DETECTORS];
-  __shared__ float dh[kFastThreads][3][22];  // sqrt(w) dRe h / dtheta_a, then sqrt(w) dIm h / dtheta_a
-  const int s = blockIdx.y, t = threadIdx.x;
-  {
-    // narrow the FP64 coefficient block (11 tangents in parameter order)
-    const SampleBlock<FisherScalar>& g = blocks[s];
-    constexpr int nwf = (int)(sizeof(PhenomDCoef<FisherScalar>) / sizeof(FisherScalar));
-    constexpr int npol = (int)(sizeof(Polar<FisherScalar>) / sizeof(FisherScalar));
-    static_assert(sizeof(PhenomDCoef<FM>) / sizeof(FM) == nwf, "coefficient block must be an array of scalars");
-    static_assert(sizeof(Polar<FR>) / sizeof(FR) == npol, "polarisation block must be an array of scalars");
-    const FisherScalar* ws = reinterpret_cast<const FisherScalar*>(&g.wf);
-    FM* wd = reinterpret_cast<FM*>(&sb.wf);
-    for (int k = t; k < nwf; k += blockDim.x) {
-      wd[k].v = ff_from(ws[k].v);
-#pragma unroll
-      for (int a = 0; a < 4; ++a) wd[k].d[a] = ff_from(ws[k].d[a]);
+// grid B: warp 0 the phase (a lane per tangent) and the polarisation, warp 1 the amplitude.
+__global__ void __launch_bounds__(64) k_fisher_prep(double scale, const SampleBlock<FisherScalar>* __restrict__ blocks,
+                                                    FisherSample* __restrict__ out) {
+  const int s = blockIdx.x, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  FisherSample& o = out[s];
+  const SampleBlock<FisherScalar>& b = blocks[s];
+  if (b.status != kSampleOk) {  // uniform
+    if (threadIdx.x == 0) {
+      o.status = b.status;
+      o.kcut = 0;
     }
-    const FisherScalar* ps = reinterpret_cast<const FisherScalar*>(&g.pol);
-    FR* pd = reinterpret_cast<FR*>(&sb.pol);
-    for (int k = t; k < npol; k += blockDim.x) {
+    return;
+  }
+  auto ff2 = [](double x) {
+    const FF q = ff_from(x);
+    return make_float2(q.hi, q.lo);
+  };
+  if (wid == 0 && lane >= 8) {
+    constexpr int npol = (int)(sizeof(Polar<FisherScalar>) / sizeof(FisherScalar));
+    static_assert(sizeof(Polar<FR>) / sizeof(FR) == npol, "polarisation block must be an array of scalars");
+    const FisherScalar* ps = reinterpret_cast<const FisherScalar*>(&b.pol);
+    FR* pd = reinterpret_cast<FR*>(&o.pol);
+    for (int k = lane - 8; k < npol; k += 24) {
       pd[k].v = (float)ps[k].v;
       pd[k].d[0] = 0.0f;
       pd[k].d[1] = (float)ps[k].d[6];  // lambda
@@ -210,107 +263,377 @@ __global__ void __launch_bounds__(kFastThreads) k_fisher_fast(PlanDev P,
       pd[k].d[3] = (float)ps[k].d[8];  // psi
       pd[k].d[4] = 0.0f;
     }
-    if (t == 0) {
-      sb.pfac.v = (float)g.wf.pfac.v;
-      sb.cfac.v = (float)g.wf.cfac.v;
+    if (lane == 31) {
+      o.pfac.v = (float)b.wf.pfac.v;
+      o.cfac.v = (float)b.wf.cfac.v;
 #pragma unroll
-      for (int a = 0; a < 4; ++a) sb.pfac.d[a] = sb.cfac.d[a] = 0.0f;
-      sb.pfac.d[4] = (float)g.wf.pfac.d[5];  // cos iota
-      sb.cfac.d[4] = (float)g.wf.cfac.d[5];
-      sb.tc = (float)g.tc.v;
-      sb.status = g.status;
-      sb.kcut = g.kcut;
+      for (int a = 0; a < 4; ++a) o.pfac.d[a] = o.cfac.d[a] = 0.0f;
+      o.pfac.d[4] = (float)b.wf.pfac.d[5];  // cos iota
+      o.cfac.d[4] = (float)b.wf.cfac.d[5];
+      o.tc = (float)b.tc.v;
     }
+    return;
+  }
+  if (lane >= 4) return;
+  // this lane's tangent of the coefficients, rescaled to f in Hz
+  using S = Dual<1>;
+  PhenomDCoef<S> c;
+  {
+    const FisherScalar* src = reinterpret_cast<const FisherScalar*>(&b.wf);
+    S* dst = reinterpret_cast<S*>(&c);
+#pragma unroll
+    for (int k = 0; k < (int)(sizeof(c) / sizeof(S)); ++k) {
+      dst[k].v = src[k].v;
+      dst[k].d[0] = src[k].d[lane];
+    }
+  }
+  FreqCoef<S> fc;
+  const double iM = 1.0 / c.Msec.v;
+  constexpr double i2p = 1.0 / (2.0 * kPi), i6p = 1.0 / (6.0 * kPi);
+  if (wid == 0) {
+    freq_coef<S, kPhasePart>(c, fc);
+#pragma unroll
+    for (int j = 0; j < 12; ++j) {
+      const double r = (j - 5) * i6p;
+      o.pin[j][lane] = ff2(fc.pin[j].d[0]);
+      o.drin[j][lane] = ff2(r * fc.pin[j].d[0]);
+      if (lane == 0) o.rin[j] = ff2(r * fc.pin[j].v);
+    }
+    o.lg0[lane] = ff2(fc.lg0.d[0]);
+    o.lg1[lane] = ff2(fc.lg1.d[0]);
+    o.drl0[lane] = ff2(i6p * fc.lg0.d[0]);
+    o.drl1[lane] = ff2(i6p * fc.lg1.d[0]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o.pint[j][lane] = ff2((j == 3 ? 3.0 : 1.0) * fc.pint[j].d[0]);
+    const S m4 = fc.pm[4] * fc.fd;
+    const double rm[4] = {1.0, -1.0, 0.75, 1.0};
+#pragma unroll
+    for (int j = 0; j < 5; ++j) o.pm[j][lane] = ff2(fc.pm[j].d[0]);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const double r = (j == 1 ? -3.0 : 1.0) * i2p;
+      o.dri[j][lane] = ff2(r * fc.pint[1 + j].d[0]);
+      if (lane == 0) o.ri[j] = ff2(r * fc.pint[1 + j].v);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const S x = j == 3 ? m4 : fc.pm[1 + j];
+      o.drm[j][lane] = ff2(rm[j] * i2p * x.d[0]);
+      if (lane == 0) o.rm[j] = ff2(rm[j] * i2p * x.v);
+    }
+    o.df5[lane] = (float)fc.f5.d[0];
+    o.dfd[lane] = (float)fc.fd.d[0];
+    if (lane == 0) {
+      o.rl0 = ff2(i6p * fc.lg0.v);
+      o.rl1 = ff2(i6p * fc.lg1.v);
+      o.f5 = ff2(fc.f5.v);
+      o.ifd = ff2(1.0 / fc.fd.v);
+      o.fd = (float)fc.fd.v;
+      o.fd2 = ff2(fc.fd.v * fc.fd.v);
+      o.pm4 = (float)fc.pm[4].v;
+      o.fj1 = (float)(kPhiJoinIns * iM);
+      o.fj2 = (float)(0.5 * (c.fRD.v * iM));
+      o.status = kSampleOk;
+      o.kcut = (int32_t)b.kcut;
+    }
+    return;
+  }
+  freq_coef<S, kAmpPart>(c, fc);
+  // the intermediate quartic about the middle of its range
+  const double f1 = kAmpJoinIns * iM, f2 = c.fpeak.v * iM, hw = 0.5 * (f2 - f1), mid = 0.5 * (f1 + f2);
+  {
+    S e[5];
+#pragma unroll
+    for (int j = 0; j < 5; ++j) e[j] = fc.dl[j];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int j = 3; j >= k; --j) e[j] = e[j] + e[j + 1] * mid;
+    double pw = 1.0;
+#pragma unroll
+    for (int j = 0; j < 5; ++j) {
+      o.dei[j][lane] = (float)(e[j].d[0] * pw);
+      if (lane == 0) o.ei[j] = ff2(e[j].v * pw);
+      pw *= hw;
+    }
+  }
+  o.dlna0[lane] = (float)(fc.a0.d[0] / fc.a0.v);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    o.dai[j][lane] = (float)fc.ai[j].d[0];
+    if (lane == 0) o.ai[j] = ff2(fc.ai[j].v);
+  }
+  o.dlngm[lane] = (float)(fc.gm.d[0] / fc.gm.v);
+  o.dw[lane] = (float)fc.w.d[0];
+  o.dfr[lane] = (float)fc.fr.d[0];
+  o.dgx[lane] = (float)fc.gx.d[0];
+  if (lane == 0) {
+    o.a0 = ff2(fc.a0.v * scale);
+    o.fc = ff2(mid);
+    o.ihw = ff2(1.0 / hw);
+    o.gm = ff2(fc.gm.v);
+    o.wf = (float)fc.w.v;
+    o.w2 = ff2(fc.w.v * fc.w.v);
+    o.fr = ff2(fc.fr.v);
+    o.gx = ff2(fc.gx.v);
+    o.fa1 = (float)f1;
+    o.fa2 = (float)f2;
+  }
+}
+
+// p x + c without renormalisation (the tail stays within a few ulps of the head)
+__device__ __forceinline__ FF ff_mad(const FF& p, const FF& x, const FF& c) {
+  const float t = p.hi * x.hi;
+  const float e = fmaf(p.hi, x.lo, fmaf(p.lo, x.hi, fmaf(p.hi, x.hi, -t)));
+  const FF s = ff_two_sum(t, c.hi);
+  return ff_make(s.hi, (s.lo + e) + c.lo);
+}
+__device__ __forceinline__ FF ff_load(const float2& a) { return ff_make(a.x, a.y); }
+
+// The waveform's part of a bin: amplitude, t(f), and the tangents over ln Mc, q, chi_1, chi_2.
+struct WaveTangents {
+  float A, tf;
+  float dA[4], ps[4], dt[4];
+};
+__device__ __forceinline__ void wave_tangents(const FisherSample& sb, const float4* __restrict__ rows,
+                                              const float2* __restrict__ p76, int64_t n, int64_t i, WaveTangents& o) {
+  float (&ps)[4] = o.ps, (&dt)[4] = o.dt;
+  const float4 r0 = rows[i], r1 = rows[n + i], r2 = rows[2 * n + i];
+  const FF ff = ff_make(r0.x, r0.y), uu = ff_make(r0.z, r0.w), jj = ff_make(r1.x, r1.y), ll = ff_make(r1.z, r1.w);
+  const float f = ff.hi, u = uu.hi, jf = jj.hi, lf3 = ll.hi;
+  // ---- phase tangents, t(f) and its tangents
+  FF tf;
+  if (f < sb.fj1) {
+    const FF iu5 = ff_make(r2.x, r2.y);
+    FF R = ff_load(sb.rin[11]);
+#pragma unroll
+    for (int j = 10; j >= 0; --j) R = ff_mad(R, uu, ff_load(sb.rin[j]));
+    const FF ul = uu * ff_addf(ll, 1.0f);
+    const FF l1 = ff_mad(ff_load(sb.rl1), ul, ff_load(sb.rl0));
+    tf = ff_mad(R, iu5, l1);
+    tf = jj * ff_fast_two_sum(tf.hi, tf.lo);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      FF p = ff_load(sb.pin[11][k]);
+      FF r = ff_load(sb.drin[11][k]);
+#pragma unroll
+      for (int j = 10; j >= 0; --j) {
+        p = ff_mad(p, uu, ff_load(sb.pin[j][k]));
+        r = ff_mad(r, uu, ff_load(sb.drin[j][k]));
+      }
+      const FF l = ff_mad(ff_load(sb.lg1[k]), uu, ff_load(sb.lg0[k])) * ll;
+      p = ff_mad(p, iu5, l);
+      ps[k] = p.hi + p.lo;
+      r = ff_mad(r, iu5, ff_mad(ff_load(sb.drl1[k]), ul, ff_load(sb.drl0[k])));
+      dt[k] = jf * (r.hi + r.lo);
+    }
+  } else if (f < sb.fj2) {
+    const FF j3 = (jj * jj) * jj;
+    const FF j4 = j3 * jj;
+    tf = ff_mad(ff_load(sb.ri[1]), j4, ff_load(sb.ri[0]));
+    tf = ff_mad(ff_load(sb.ri[2]), jj, tf);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      FF p = ff_mad(ff_load(sb.pint[1][k]), ff, ff_load(sb.pint[0][k]));
+      p = ff_mad(ff_load(sb.pint[2][k]), j3, p);
+      p = ff_mad(ff_load(sb.pint[3][k]), ll, p);
+      ps[k] = p.hi + p.lo;
+      const FF r = ff_mad(ff_load(sb.dri[2][k]), jj, ff_mad(ff_load(sb.dri[1][k]), j4, ff_load(sb.dri[0][k])));
+      dt[k] = r.hi + r.lo;
+    }
+  } else {
+    const FF q = ff_make(r2.z, r2.w), fq = ff * q;
+    const FF xx = ff - ff_load(sb.f5);
+    const FF rd = ff_make(1.0f, 0.0f) / (xx * xx + ff_load(sb.fd2));
+    const float x = xx.hi, rden = rd.hi;
+    const FF at = datan(xx * ff_load(sb.ifd));
+    tf = ff_mad(ff_load(sb.rm[1]), jj * jj, ff_load(sb.rm[0]));
+    tf = ff_mad(ff_load(sb.rm[2]), q, tf);
+    tf = ff_mad(ff_load(sb.rm[3]), rd, tf);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      FF p = ff_mad(ff_load(sb.pm[1][k]), ff, ff_load(sb.pm[0][k]));
+      p = ff_mad(ff_load(sb.pm[2][k]), jj, p);
+      p = ff_mad(ff_load(sb.pm[3][k]), fq, p);
+      p = ff_mad(ff_load(sb.pm[4][k]), at, p);
+      p = ff_addf(p, -(sb.pm4 * rden) * fmaf(sb.df5[k], sb.fd, x * sb.dfd[k]));
+      ps[k] = p.hi + p.lo;
+      const float drden = 2.0f * rden * fmaf(x, sb.df5[k], -(sb.fd * sb.dfd[k]));  // over rden
+      FF r = ff_mad(ff_load(sb.drm[1][k]), jj * jj, ff_load(sb.drm[0][k]));
+      r = ff_mad(ff_load(sb.drm[2][k]), q, r);
+      r = ff_mad(ff_load(sb.drm[3][k]), rd, r);
+      dt[k] = fmaf(rden * sb.rm[3].x, drden, r.hi + r.lo);
+    }
+  }
+  tf = ff_fast_two_sum(tf.hi, tf.lo);
+  o.tf = tf.hi;
+  // ---- amplitude, the tangents of its logarithm
+  FF ah;
+  float da[4];
+  if (f < sb.fa1) {
+    FF p = ff_load(sb.ai[7]);
+#pragma unroll
+    for (int j = 6; j >= 0; --j) p = ff_mad(p, uu, ff_load(sb.ai[j]));
+    ah = ff_addf(ff_fast_two_sum(p.hi, p.lo) * (uu * uu), 1.0f);
+    const float g = u * u / ah.hi;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float r = sb.dai[7][k];
+#pragma unroll
+      for (int j = 6; j >= 0; --j) r = fmaf(r, u, sb.dai[j][k]);
+      da[k] = fmaf(r, g, sb.dlna0[k]);
+    }
+  } else if (f < sb.fa2) {
+    const FF xx = (ff - ff_load(sb.fc)) * ff_load(sb.ihw);
+    const float x = xx.hi;
+    ah = ff_load(sb.ei[4]);
+#pragma unroll
+    for (int j = 3; j >= 0; --j) ah = ff_mad(ah, xx, ff_load(sb.ei[j]));
+    ah = ff_fast_two_sum(ah.hi, ah.lo);
+    const float g = 1.0f / ah.hi;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float r = fmaf(x, fmaf(x, fmaf(x, fmaf(x, sb.dei[4][k], sb.dei[3][k]), sb.dei[2][k]), sb.dei[1][k]), sb.dei[0][k]);
+      da[k] = fmaf(r, g, sb.dlna0[k]);
+    }
+  } else {
+    const FF xx = ff - ff_load(sb.fr);
+    const float x = xx.hi;
+    const FF den = xx * xx + ff_load(sb.w2);
+    const float rw = 1.0f / den.hi;
+    ah = ff_load(sb.gm) / den * dexp(-(ff_load(sb.gx) * xx));
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      da[k] = sb.dlna0[k] + sb.dlngm[k] + 2.0f * rw * fmaf(x, sb.dfr[k], -(sb.wf * sb.dw[k])) +
+              fmaf(sb.gx.x, sb.dfr[k], -(sb.dgx[k] * x));
+  }
+  o.A = (ff_load(sb.a0) * ff_load(p76[i]) * ah).hi;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) o.dA[k] = o.A * da[k];
+}
+
+// The summing warp's share: rows of the upper triangle in pieces of up to three pairs, one per lane.
+__device__ __forceinline__ void pairs_of(int lane, int& a, int& b, int& count) {
+  a = 0;
+  for (int piece = lane; a < 11; ++a) {
+    const int pieces = (11 - a + 2) / 3;
+    if (piece < pieces) {
+      b = a + 3 * piece;
+      count = min(3, 11 - b);
+      return;
+    }
+    piece -= pieces;
+  }
+  a = b = count = 0;
+}
+
+constexpr size_t fisher_smem() { return 2 * sizeof(float2) * kFastThreads * 3 * 11; }
+
+// grid (blocks, B), grid-stride over the groups of 128 live bins.
+__global__ void __launch_bounds__(kFastBlock, 2) k_fisher_fast(PlanDev P, const FisherSample* __restrict__ samples,
+                                                               const float4* __restrict__ rows,
+                                                               const float2* __restrict__ p76,
+                                                               const float4* __restrict__ wt,
+                                                               double* __restrict__ partial) {
+  extern __shared__ float2 dh_buf[];  // [2][bin][channel][11]: sqrt(w) dh / dtheta_a
+  __shared__ FisherSample sb;
+  __shared__ OrbitF orb[PES_MAX_DETECTORS];
+  const int s = blockIdx.y, t = threadIdx.x;
+  const int64_t n = P.nbins;
+  {
+    const int* src = reinterpret_cast<const int*>(&samples[s]);
+    int* dst = reinterpret_cast<int*>(&sb);
+    for (int k = t; k < (int)(sizeof(FisherSample) / 4); k += kFastBlock) dst[k] = src[k];
     if (t < P.n_det) orb[t] = orbit_f(P.orbit[t]);
   }
   __syncthreads();
-  const float scale = (float)(kPc / (kMRSun * kMTSun));
-  const double inv_scale2 = 1.0 / ((double)scale * (double)scale);
-  int pa = 0, pb = 0;
-  pair_of(t < kPairs ? t : 0, pa, pb);
-  double acc = 0.0;
-  if (sb.status == kSampleOk) {
-    for (int64_t base = (int64_t)blockIdx.x * kFastThreads; base < sb.kcut;
-         base += (int64_t)gridDim.x * kFastThreads) {
-      const int64_t i = base + t;
-      const bool live = i < sb.kcut;
-      const float f = (float)((double)(P.k0 + (live ? i : 0)) * P.f_step);
-      FM amp, psi, tf;
-      if (live) {
-        phenomd_eval<FM>(sb.wf, sb.wf.Msec * f, amp, psi, tf);
-        amp = amp * scale;
-      }
-      for (int d = 0; d < P.n_det; ++d) {
-        if (live) {
-          Cx<FR> Y[3];
-          FR kx0;
-          {
-            FR T = lift<FR>(0.0);
-            T.v = tf.v.hi + sb.tc;
-            T.d[0] = 1.0f;
-            const FR zero = lift<FR>(0.0);
-            Cx<FR> L[6];
-            single_links_impl<true, FR>(orb[d], f, cx(sb.pfac, zero), cx(zero, -sb.cfac), T, sb.pol, L, &kx0);
-            const TdiFactor tdb = P.tdi[(size_t)d * P.nbins + i];
-            tdi_channels_t<true, FR>(cx(lift<FR>((float)tdb.dre), lift<FR>((float)tdb.dim)),
-                                     cx(lift<FR>((float)tdb.pre), lift<FR>((float)tdb.pim)), 1, L, Y);
-          }
-          const float A = amp.v.hi, tp = 6.283185307179586f * f;
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            const float sw = (float)sqrt(P.w[((size_t)d * 3 + c) * P.nbins + i] * inv_scale2);  // 0 off the mask
-            const FR& Yr = Y[c].re;
-            const FR& Yi = Y[c].im;
-            const float ar = A * Yr.v, ai = A * Yi.v;  // A Y
-            float ur[11], ui[11];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {  // ln Mc, q, chi_1, chi_2
-              const float dA = amp.d[k].hi, dt = tf.d[k].hi;
-              const float ph = psi.d[k].hi + tp * kx0.d[0] * dt;
-              ur[k] = dA * Yr.v + A * Yr.d[0] * dt + ai * ph;
-              ui[k] = dA * Yi.v + A * Yi.d[0] * dt - ar * ph;
-            }
-            ur[4] = -ar;  // ln D_L: dh = -h
-            ui[4] = -ai;
-            ur[5] = A * Yr.d[4];  // cos iota
-            ui[5] = A * Yi.d[4];
-            ur[6] = A * Yr.d[1] + ai * tp * kx0.d[1];  // lambda
-            ui[6] = A * Yi.d[1] - ar * tp * kx0.d[1];
-            ur[7] = A * Yr.d[2] + ai * tp * kx0.d[2];  // sin beta
-            ui[7] = A * Yi.d[2] - ar * tp * kx0.d[2];
-            ur[8] = A * Yr.d[3];  // psi
-            ui[8] = A * Yi.d[3];
-            ur[9] = -2.0f * ai;  // phi_c: dh = 2 i h
-            ui[9] = 2.0f * ar;
-            const float pt = tp * (kx0.d[0] + 1.0f);  // t_c
-            ur[10] = A * Yr.d[0] + ai * pt;
-            ui[10] = A * Yi.d[0] - ar * pt;
-#pragma unroll
-            for (int a = 0; a < 11; ++a) {
-              dh[t][c][a] = sw * ur[a];
-              dh[t][c][11 + a] = sw * ui[a];
-            }
-          }
-        } else {
-#pragma unroll
-          for (int c = 0; c < 3; ++c)
-#pragma unroll
-            for (int a = 0; a < 22; ++a) dh[t][c][a] = 0.0f;
+  const int kcut = sb.status == kSampleOk ? sb.kcut : 0;
+  const bool summing = t >= kFastThreads;
+  int pa = 0, pb = 0, np = 0;
+  if (summing) pairs_of(t - kFastThreads, pa, pb, np);
+  double acc[3] = {0.0, 0.0, 0.0};
+  WaveTangents wv;
+  int step = 0;  // (group, detector) pairs evaluated so far
+  const int first = blockIdx.x * kFastThreads, stride = gridDim.x * kFastThreads;
+  const int steps = first < kcut ? (kcut - first + stride - 1) / stride * P.n_det : 0;
+  for (; step <= steps; ++step) {
+    float2* buf = dh_buf + (size_t)(step & 1) * (kFastThreads * 33);
+    if (!summing && step < steps) {
+      const int d = step % P.n_det;
+      const int i = first + step / P.n_det * stride + t;
+      float2* dst = buf + t * 33;
+      if (i < kcut) {
+        const float f = rows[i].x;
+        if (d == 0) wave_tangents(sb, rows, p76, n, i, wv);
+        const float4 td = wt[(size_t)d * 2 * n + i], sw3 = wt[((size_t)d * 2 + 1) * n + i];
+        Cx<FR> Y[3];
+        FR kx0;
+        {
+          FR T = lift<FR>(0.0);
+          T.v = wv.tf + sb.tc;
+          T.d[0] = 1.0f;
+          const FR zero = lift<FR>(0.0);
+          Cx<FR> L[6];
+          single_links_impl<true, FR>(orb[d], f, cx(sb.pfac, zero), cx(zero, -sb.cfac), T, sb.pol, L, &kx0);
+          tdi_channels_t<true, FR>(cx(lift<FR>(td.x), lift<FR>(td.y)), cx(lift<FR>(td.z), lift<FR>(td.w)), 1, L, Y);
         }
-        __syncthreads();
-        if (t < kPairs) {
-          float x = 0.0f;
-          for (int u = 0; u < kFastThreads; ++u)
+        const float A = wv.A, tp = 6.283185307179586f * f;
 #pragma unroll
-            for (int c = 0; c < 3; ++c)
-              x = fmaf(dh[u][c][pa], dh[u][c][pb], fmaf(dh[u][c][11 + pa], dh[u][c][11 + pb], x));
-          acc += (double)x;
+        for (int c = 0; c < 3; ++c) {
+          const float sw = c == 0 ? sw3.x : (c == 1 ? sw3.y : sw3.z);
+          const FR& Yr = Y[c].re;
+          const FR& Yi = Y[c].im;
+          const float ar = A * Yr.v, ai = A * Yi.v;  // A Y
+          float ur[11], ui[11];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {  // ln Mc, q, chi_1, chi_2
+            const float dA = wv.dA[k], dt = wv.dt[k];
+            const float ph = wv.ps[k] + tp * kx0.d[0] * dt;
+            ur[k] = dA * Yr.v + A * Yr.d[0] * dt + ai * ph;
+            ui[k] = dA * Yi.v + A * Yi.d[0] * dt - ar * ph;
+          }
+          ur[4] = -ar;  // ln D_L: dh = -h
+          ui[4] = -ai;
+          ur[5] = A * Yr.d[4];  // cos iota
+          ui[5] = A * Yi.d[4];
+          ur[6] = A * Yr.d[1] + ai * tp * kx0.d[1];  // lambda
+          ui[6] = A * Yi.d[1] - ar * tp * kx0.d[1];
+          ur[7] = A * Yr.d[2] + ai * tp * kx0.d[2];  // sin beta
+          ui[7] = A * Yi.d[2] - ar * tp * kx0.d[2];
+          ur[8] = A * Yr.d[3];  // psi
+          ui[8] = A * Yi.d[3];
+          ur[9] = -2.0f * ai;  // phi_c: dh = 2 i h
+          ui[9] = 2.0f * ar;
+          const float pt = tp * (kx0.d[0] + 1.0f);  // t_c
+          ur[10] = A * Yr.d[0] + ai * pt;
+          ui[10] = A * Yi.d[0] - ar * pt;
+#pragma unroll
+          for (int a = 0; a < 11; ++a) dst[c * 11 + a] = make_float2(sw * ur[a], sw * ui[a]);
         }
-        __syncthreads();
+      } else {
+        for (int a = 0; a < 33; ++a) dst[a] = make_float2(0.0f, 0.0f);
       }
     }
+    if (summing && step > 0) {
+      const float2* src = dh_buf + (size_t)((step & 1) ^ 1) * (kFastThreads * 33);
+      float x[3] = {0.0f, 0.0f, 0.0f};
+      const int b1 = min(pb + 1, 10), b2 = min(pb + 2, 10);
+#pragma unroll 4
+      for (int u = 0; u < kFastThreads * 3; ++u) {
+        const float2* q = src + u * 11;
+        const float2 va = q[pa], v0 = q[pb], v1 = q[b1], v2 = q[b2];
+        x[0] = fmaf(va.x, v0.x, fmaf(va.y, v0.y, x[0]));
+        x[1] = fmaf(va.x, v1.x, fmaf(va.y, v1.y, x[1]));
+        x[2] = fmaf(va.x, v2.x, fmaf(va.y, v2.y, x[2]));
+      }
+#pragma unroll
+      for (int k = 0; k < 3; ++k) acc[k] += (double)x[k];
+    }
+    __syncthreads();
   }
-  if (t < kPairs) partial[((size_t)s * gridDim.x + blockIdx.x) * kPairs + t] = acc;
+  if (summing)
+    for (int k = 0; k < np; ++k)
+      partial[((size_t)s * gridDim.x + blockIdx.x) * kPairs + (pa * 11 - pa * (pa - 1) / 2 + (pb + k - pa))] = acc[k];
 }
 
 }  // namespace pes
@@ -327,22 +650,45 @@ extern "C" int pes_fisher_batch(PesPlan* p, const double* theta, int64_t B, doub
   PES_REQUIRE((p->data_set_mask & need) == need, "pes_fisher_batch: PSD not set for every detector (pes_plan_set_data)");
   if (B == 0) return PES_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const bool hm = p->desc.approximant == PES_APPROX_PHENOMHM, fast = p->mixed && !hm;
+  const int64_t M = p->desc.max_batch, n = p->desc.nbins, nd = p->desc.n_det;
+  // blocks per sample: kFisherBlocks, more in calls that would leave SMs idle
+  const int64_t nblk = !fast ? (int64_t)kFisherBlocks
+                             : std::min<int64_t>(ceil_div(n, kFastThreads),
+                                                 std::max<int64_t>(kFisherBlocks, ceil_div(kFastBlocks, B)));
   if (!p->fisher_blocks) {
-    const int64_t M = p->desc.max_batch;
+    const int64_t rows = std::max<int64_t>(M * kFisherBlocks, kFastBlocks + M);
+    PES_CHECK_CUDA(cudaMalloc(&p->fisher_partial, sizeof(double) * rows * kPairs));
+    if (fast) {
+      PES_CHECK_CUDA(cudaMalloc(&p->fisher_samples, sizeof(FisherSample) * M));
+      PES_CHECK_CUDA(cudaMalloc(&p->fisher_rows, sizeof(float4) * n * (3 + 2 * nd)));
+      PES_CHECK_CUDA(cudaMalloc(&p->fisher_p76, sizeof(float2) * n));
+      PES_CHECK_CUDA(cudaFuncSetAttribute(k_fisher_fast, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fisher_smem()));
+      k_fisher_grid<<<ceil_div(n, 128), 128, 0, st>>>(p->dev, p->fisher_rows, p->fisher_p76);
+      PES_CHECK_LAUNCH();
+    }
     PES_CHECK_CUDA(cudaMalloc(&p->fisher_blocks, sizeof(SampleBlock<FisherScalar>) * M));
-    PES_CHECK_CUDA(cudaMalloc(&p->fisher_partial, sizeof(double) * M * kFisherBlocks * kPairs));
   }
   auto* blocks = reinterpret_cast<SampleBlock<FisherScalar>*>(p->fisher_blocks);
   k_setup<FisherScalar><<<setup_blocks(B), 64, 0, st>>>(p->dev, theta, B, 0, blocks, hm_blocks<FisherScalar>(p));
   PES_CHECK_LAUNCH();
-  const bool hm = p->desc.approximant == PES_APPROX_PHENOMHM;
-  if (p->mixed && !hm)  // mixed IMRPhenomD plans: FP32 structured derivatives
-    k_fisher_fast<<<dim3(kFisherBlocks, (unsigned)B), kFastThreads, 0, st>>>(p->dev, blocks, p->fisher_partial);
-  else  // FP64 plans and IMRPhenomHM: FP64 dual numbers through the whole model
+  if (fast) {  // mixed IMRPhenomD plans: FP32 structured derivatives
+    auto* samples = reinterpret_cast<FisherSample*>(p->fisher_samples);
+    float4* wt = p->fisher_rows + 3 * n;
+    const float scale = (float)(kPc / (kMRSun * kMTSun));
+    const double inv_scale2 = 1.0 / ((double)scale * (double)scale);
+    k_fisher_weights<<<dim3(ceil_div(n, 128), (unsigned)nd), 128, 0, st>>>(p->dev, inv_scale2, wt);
+    PES_CHECK_LAUNCH();
+    k_fisher_prep<<<(unsigned)B, 64, 0, st>>>(scale, blocks, samples);
+    PES_CHECK_LAUNCH();
+    k_fisher_fast<<<dim3((unsigned)nblk, (unsigned)B), kFastBlock, fisher_smem(), st>>>(
+        p->dev, samples, p->fisher_rows, p->fisher_p76, wt, p->fisher_partial);
+  } else {  // FP64 plans and IMRPhenomHM: FP64 dual numbers through the whole model
     k_fisher_bins<<<dim3(kFisherBlocks, (unsigned)B), kFisherThreads, 0, st>>>(
         p->dev, blocks, hm ? hm_blocks<FisherScalar>(p) : nullptr, p->fisher_partial);
+  }
   PES_CHECK_LAUNCH();
-  k_fisher_final<<<(unsigned)ceil_div(B * kPairs, 128), 128, 0, st>>>(blocks, B, kFisherBlocks, 4.0 * p->dev.df,
+  k_fisher_final<<<(unsigned)ceil_div(B * kPairs, 128), 128, 0, st>>>(blocks, B, (int)nblk, 4.0 * p->dev.df,
                                                                        p->fisher_partial, fisher, status);
   PES_CHECK_LAUNCH();
   return PES_OK;

@@ -360,6 +360,9 @@ int pes_plan_destroy(PesPlan* p) {
   if (p->fp64) fp64_destroy(p);
   cudaFree(p->fisher_blocks);
   cudaFree(p->fisher_partial);
+  cudaFree(p->fisher_samples);
+  cudaFree(p->fisher_rows);
+  cudaFree(p->fisher_p76);
   cudaFree(p->data);
   cudaFree(p->w);
   cudaFree(p->tdi);

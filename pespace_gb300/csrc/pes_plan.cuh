@@ -111,6 +111,11 @@ struct PesPlan {
   int sample_threads = pes::kPerSampleThreads;  // block size of the per-sample lnL kernels (PES_OPT_SAMPLE_THREADS)
   void* fisher_blocks = nullptr;     // [max_batch] SampleBlock<Dual<11>> (first Fisher call)
   double* fisher_partial = nullptr;  // [max_batch][blocks][66]
+  // mixed IMRPhenomD plans: coefficient blocks, powers of f, TDI factors and
+  // channel weights per bin (pes_fisher.cu)
+  void* fisher_samples = nullptr;
+  float4* fisher_rows = nullptr;
+  float2* fisher_p76 = nullptr;
   pes::Profiler prof;
 };
 
