@@ -1425,7 +1425,7 @@ __device__ __forceinline__ const R* spline_factor(const MixedDev& M, int which) 
   }
 }
 
-// Register-segment fit, staged through shared memory.  Each warp solves one
+// Segmented fit, staged through shared memory.  Each warp solves one
 // (sample, detector, quantity) system; lane l owns rows [l seg, (l+1) seg).
 // Those lane-strided accesses go to shared memory only: the block first
 // copies the shared grid's factor tables and each warp its system's node
@@ -1443,21 +1443,26 @@ __host__ __device__ __forceinline__ int fit_rows(int J) { return fit_pad(J) + 1;
 
 // dynamic shared memory of one staged-fit block: five R tables (h, 1/h, lo,
 // 1/den, cp), the FF 1/h table for the slopes (the R table itself for R = FF),
-// then per warp the node values and the four end-row values.
+// then per warp the node values, the four end-row values and the unknowns
+// (row k of lane l at k 32 + l).  The segment loops are rolled: unrolled around
+// unknowns in registers, each warp ran 200 KB of straight-line code once, and its
+// instruction fetch took half of the fit of a small call (phase fit of 16 systems of 1024
+// intervals 98 -> 57 us, of 72 systems of 2048 intervals 170 -> 87 us).
 // Grids of more than 32 x 32 intervals leave the tables in global memory
 // (staging them would leave room for one block per SM).
-template <class R, bool kStageTables>
+template <class R, bool kStageTables, int kSeg>
 __host__ __device__ __forceinline__ size_t fit_smem_bytes(int J) {
   const size_t rows = (size_t)fit_rows(J);
   const size_t tables =
       kStageTables ? 5 * rows * sizeof(R) + (std::is_same<R, FF>::value ? 0 : rows * sizeof(FF)) : 0;
-  return ((tables + 15) & ~(size_t)15) + (size_t)kFitWarps * (rows * sizeof(FF) + 4 * sizeof(FF));
+  return ((tables + 15) & ~(size_t)15) +
+         (size_t)kFitWarps * (rows * sizeof(FF) + 4 * sizeof(FF) + kSeg * 32 * sizeof(R));
 }
 
 template <int kSeg, class R, bool kStageTables>
 __device__ __forceinline__ void spline_fit_staged(const MixedDev& M, int64_t sd, int q, int n, const R* t_h,
                                                   const R* t_ih, const R* t_lo, const R* t_id, const R* t_cp,
-                                                  const FF* t_gih, const FF* y, R* smem4) {
+                                                  const FF* t_gih, const FF* y, R* smem4, R* xs) {
   const int lane = threadIdx.x & 31;
   auto tp = [](int i) { return kStageTables ? fit_pad(i) : i; };
   // staged: segments of 32 rows whatever n (lanes past n idle), which keeps
@@ -1469,115 +1474,107 @@ __device__ __forceinline__ void spline_fit_staged(const MixedDev& M, int64_t sd,
   const R lo_l = lift<R>(lo_d), iden_l = lift<R>(1.0 / (di_d - lo_d * M.gcp[n - 2]));
   const R zero = lift<R>(0.0);
   // right-hand sides 6 (slope_i - slope_{i-1}) of rows i0 + k
-  R x[kSeg];
+  xs += lane;  // x_k at xs[32 k]
+  if (cnt == 0) xs[0] = zero;
   {
     FF yc = y[fit_pad(i0)];
     FF sp = (i0 >= 1) ? (yc - y[fit_pad(i0 - 1)]) * t_gih[tp(i0 - 1)] : ff_make(0.0f, 0.0f);
-#pragma unroll
-    for (int k = 0; k < kSeg; ++k) {
-      x[k] = zero;
-      if (k < cnt) {
-        const int i = i0 + k;
-        const FF yn = y[fit_pad(i + 1)];
-        const FF sl = (yn - yc) * t_gih[tp(i)];
-        if (i >= 1) x[k] = ff_to_r<R>(ff_mulf(sl - sp, 6.0f));
-        sp = sl;
-        yc = yn;
-      }
+#pragma unroll 4
+    for (int k = 0; k < cnt; ++k) {
+      const int i = i0 + k;
+      const FF yn = y[fit_pad(i + 1)];
+      const FF sl = (yn - yc) * t_gih[tp(i)];
+      xs[32 * k] = i >= 1 ? ff_to_r<R>(ff_mulf(sl - sp, 6.0f)) : zero;
+      sp = sl;
+      yc = yn;
     }
   }
   // forward elimination (rows 1..n-1)
   R A = lift<R>(1.0), v = zero;
-#pragma unroll
-  for (int k = 0; k < kSeg; ++k) {
+#pragma unroll 4
+  for (int k = 0; k < cnt; ++k) {
     const int i = i0 + k;
-    if (k < cnt && i >= 1) {
+    if (i >= 1) {
       const bool last = i == n - 1;
       const R l = last ? lo_l : t_lo[tp(i)], id = last ? iden_l : t_id[tp(i)];
-      v = (x[k] - l * v) * id;
+      v = (xs[32 * k] - l * v) * id;
       A = -(l * id) * A;
     }
   }
   v = segment_carry_in<R>(A, v, false);
-#pragma unroll
-  for (int k = 0; k < kSeg; ++k) {
+#pragma unroll 4
+  for (int k = 0; k < cnt; ++k) {
     const int i = i0 + k;
-    if (k < cnt && i >= 1) {
+    if (i >= 1) {
       const bool last = i == n - 1;
       const R l = last ? lo_l : t_lo[tp(i)], id = last ? iden_l : t_id[tp(i)];
-      v = (x[k] - l * v) * id;
-      x[k] = v;
+      v = (xs[32 * k] - l * v) * id;
+      xs[32 * k] = v;
     }
   }
   // back substitution m_i = d'_i - cp_i m_{i+1}
   A = lift<R>(1.0);
   v = zero;
-#pragma unroll
-  for (int k = kSeg - 1; k >= 0; --k) {
+#pragma unroll 4
+  for (int k = cnt - 1; k >= 0; --k) {
     const int i = i0 + k;
-    if (k < cnt && i >= 1) {
+    if (i >= 1) {
       const R c = (i == n - 1) ? zero : t_cp[tp(i)];
-      v = x[k] - c * v;
+      v = xs[32 * k] - c * v;
       A = -c * A;
     }
   }
   v = segment_carry_in<R>(A, v, true);
-#pragma unroll
-  for (int k = kSeg - 1; k >= 0; --k) {
+#pragma unroll 4
+  for (int k = cnt - 1; k >= 0; --k) {
     const int i = i0 + k;
-    if (k < cnt && i >= 1) {
+    if (i >= 1) {
       const R c = (i == n - 1) ? zero : t_cp[tp(i)];
-      v = x[k] - c * v;
-      x[k] = v;
+      v = xs[32 * k] - c * v;
+      xs[32 * k] = v;
     }
   }
-  // m_1, m_2, m_{n-2}, m_{n-1} for the eliminated end values
+  // m_1, m_2, m_{n-2}, m_{n-1} for the eliminated end values, from the lanes that own them
+  {
+    const int row[4] = {1, 2, n - 2, n - 1};
 #pragma unroll
-  for (int k = 0; k < kSeg; ++k) {
-    const int i = i0 + k;
-    if (k < cnt) {
-      if (i == 1) smem4[0] = x[k];
-      if (i == 2) smem4[1] = x[k];
-      if (i == n - 2) smem4[2] = x[k];
-      if (i == n - 1) smem4[3] = x[k];
-    }
+    for (int e = 0; e < 4; ++e)
+      if (row[e] >= i0 && row[e] < i0 + cnt) smem4[e] = xs[32 * (row[e] - i0)];
   }
   __syncwarp();
   const R h0 = t_h[tp(0)], h1 = t_h[tp(1)], ha = t_h[tp(n - 2)], hb = t_h[tp(n - 1)];
   const R m0 = ((h0 + h1) * smem4[0] - h0 * smem4[1]) / h1;
   const R mn = ((ha + hb) * smem4[3] - hb * smem4[2]) / ha;
-  const R next_first = warp_shfl_down(x[0], 1);  // m at row i0 + cnt (when it is a row)
+  const R next_first = warp_shfl_down(xs[0], 1);  // m at row i0 + cnt (when it is a row)
   const R sixth = lift<R>(1.0 / 6.0), half = lift<R>(0.5), two = lift<R>(2.0);
   FF yc = y[fit_pad(i0)];
-#pragma unroll
-  for (int k = 0; k < kSeg; ++k) {
+#pragma unroll 4
+  for (int k = 0; k < cnt; ++k) {
     const int i = i0 + k;
-    if (k < cnt) {
-      const R mi = (i == 0) ? m0 : x[k];
-      R mj;
-      if (i + 1 == n) mj = mn;
-      else if (k + 1 < cnt) mj = x[(k + 1) < kSeg ? k + 1 : k];
-      else mj = next_first;
-      const FF yn = y[fit_pad(i + 1)];
-      const FF slf = (yn - yc) * t_gih[tp(i)];
-      const R corr = t_h[tp(i)] * (two * mi + mj) * sixth;
-      const R cc = half * mi;
-      const R dc = (mj - mi) * t_ih[tp(i)] * sixth;
-      if constexpr (std::is_same<R, FF>::value) {
-        FF* o = M.cphi + ((size_t)sd * M.J + i) * 4;
-        o[0] = yc;
-        o[1] = slf - corr;
-        o[2] = cc;
-        o[3] = dc;
-      } else {
-        // b = slope - h (2 m_i + m_j) / 6 from the float-float slope: FP32 head and tail
-        const FF bf = ff_addf(slf, -corr);
-        M.cg[((size_t)sd * M.J + i) * 8 + (q - 1)] = make_float4(yc.hi, bf.hi, cc, dc);
-        reinterpret_cast<float*>(M.cg + ((size_t)sd * M.J + i) * 8 + 6)[q - 1] = yc.lo;
-        M.cgb[((size_t)sd * M.J + i) * 6 + (q - 1)] = bf.lo;
-      }
-      yc = yn;
+    const R mi = (i == 0) ? m0 : xs[32 * k];
+    R mj;
+    if (i + 1 == n) mj = mn;
+    else if (k + 1 < cnt) mj = xs[32 * (k + 1)];
+    else mj = next_first;
+    const FF yn = y[fit_pad(i + 1)];
+    const FF slf = (yn - yc) * t_gih[tp(i)];
+    const R corr = t_h[tp(i)] * (two * mi + mj) * sixth;
+    const R cc = half * mi;
+    const R dc = (mj - mi) * t_ih[tp(i)] * sixth;
+    if constexpr (std::is_same<R, FF>::value) {
+      FF* o = M.cphi + ((size_t)sd * M.J + i) * 4;
+      o[0] = yc;
+      o[1] = slf - corr;
+      o[2] = cc;
+      o[3] = dc;
+    } else {
+      // b = slope - h (2 m_i + m_j) / 6 from the float-float slope: FP32 head and tail
+      const FF bf = ff_addf(slf, -corr);
+      M.cg[((size_t)sd * M.J + i) * 8 + (q - 1)] = make_float4(yc.hi, bf.hi, cc, dc);
+      reinterpret_cast<float*>(M.cg + ((size_t)sd * M.J + i) * 8 + 6)[q - 1] = yc.lo;
+      M.cgb[((size_t)sd * M.J + i) * 6 + (q - 1)] = bf.lo;
     }
+    yc = yn;
   }
 }
 
@@ -1599,8 +1596,9 @@ __global__ void __launch_bounds__(kFitWarps * 32, 3) k_spline_fit(MixedDev M, in
   const size_t tables = kStage ? 5 * (size_t)rows * sizeof(R) + (kPhase ? 0 : (size_t)rows * sizeof(FF)) : 0;
   unsigned char* wbase = fit_smem + ((tables + 15) & ~(size_t)15);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  FF* ys = reinterpret_cast<FF*>(wbase + (size_t)warp * (rows * sizeof(FF) + 4 * sizeof(FF)));
+  FF* ys = reinterpret_cast<FF*>(wbase + (size_t)warp * (rows * sizeof(FF) + 4 * sizeof(FF) + kSeg * 32 * sizeof(R)));
   R* sm4 = reinterpret_cast<R*>(ys + rows);
+  R* xs = reinterpret_cast<R*>(ys + rows + 4);
   if (!kStage) {
     t_h = const_cast<R*>(src + (size_t)kGfH * M.J);
     t_ih = const_cast<R*>(src + (size_t)kGfInvH * M.J);
@@ -1633,17 +1631,17 @@ __global__ void __launch_bounds__(kFitWarps * 32, 3) k_spline_fit(MixedDev M, in
   const FF* yq = M.yv + ((size_t)sd * kNodeQ + q) * M.J;
   for (int i = lane; i <= n; i += 32) ys[fit_pad(i)] = yq[i];
   __syncwarp();
-  spline_fit_staged<kSeg, R, kStage>(M, sd, q, n, t_h, t_ih, t_lo, t_id, t_cp, t_gih, ys, sm4);
+  spline_fit_staged<kSeg, R, kStage>(M, sd, q, n, t_h, t_ih, t_lo, t_id, t_cp, t_gih, ys, sm4, xs);
 }
 
 // Transpose of the fit with the same lane segments.  mom(i, p) gives the
 // interval moments, the tables are indexed through tp (padded rows when they
 // were staged in shared memory).
-template <int kSeg, class R, class MomAt, class TabIdx>
+template <class R, class MomAt, class TabIdx>
 __device__ __forceinline__ void spline_adjoint_seg(const MixedDev& M, int64_t sd, int q, int n, int seg, double wscale,
                                                    const R* __restrict__ fh, const R* __restrict__ fih,
                                                    const R* __restrict__ flo, const R* __restrict__ fup,
-                                                   const R* __restrict__ fid, MomAt mom, TabIdx tp) {
+                                                   const R* __restrict__ fid, MomAt mom, TabIdx tp, R* xs) {
   const int lane = threadIdx.x & 31;
   float* __restrict__ yb = M.ybar + (size_t)sd * M.J * kNodeQ + q;
   const int i0 = min(n, lane * seg), cnt = min(n, i0 + seg) - i0;
@@ -1659,98 +1657,95 @@ __device__ __forceinline__ void spline_adjoint_seg(const MixedDev& M, int64_t sd
   nak_row(M.node_f, n, n - 1, lo_d, di_d, up_d);
   const R lo_l = (R)lo_d, iden_l = (R)(1.0 / (di_d - lo_d * M.gcp[n - 2]));
   // right-hand sides (coefficient adjoints -> mbar, end eliminations), in FP64
-  R x[kSeg];
+  xs += lane;  // x_k at xs[32 k]
+  if (cnt == 0) xs[0] = R(0);
   {
     R right_prev = (i0 >= 1) ? mbar_right(i0 - 1) : R(0);
-#pragma unroll
-    for (int k = 0; k < kSeg; ++k) {
-      x[k] = R(0);
+#pragma unroll 4
+    for (int k = 0; k < cnt; ++k) {
       const int i = i0 + k;
-      if (k < cnt) {
-        const R left = mbar_left(i);
-        if (i >= 1) {
-          R w = right_prev + left;
-          if (i == 1) w += mb0 * (h0 + h1) / h1;
-          if (i == 2) w -= mb0 * h0 / h1;
-          if (i == n - 1) w += mbn * (ha + hb) / ha;
-          if (i == n - 2) w -= mbn * hb / ha;
-          x[k] = w;
-        }
-        right_prev = mbar_right(i);
+      const R left = mbar_left(i);
+      R w = R(0);
+      if (i >= 1) {
+        w = right_prev + left;
+        if (i == 1) w += mb0 * (h0 + h1) / h1;
+        if (i == 2) w -= mb0 * h0 / h1;
+        if (i == n - 1) w += mbn * (ha + hb) / ha;
+        if (i == n - 2) w -= mbn * hb / ha;
       }
+      xs[32 * k] = w;
+      right_prev = mbar_right(i);
     }
   }
   // U^T z = mbar
   R A = R(1), v = R(0);
-#pragma unroll
-  for (int k = 0; k < kSeg; ++k) {
+#pragma unroll 4
+  for (int k = 0; k < cnt; ++k) {
     const int i = i0 + k;
-    if (k < cnt && i >= 1) {
+    if (i >= 1) {
       const R sub = (i > 1) ? fup[tp(i - 1)] : R(0), id = (i == n - 1) ? iden_l : fid[tp(i)];
-      v = (x[k] - sub * v) * id;
+      v = (xs[32 * k] - sub * v) * id;
       A = -sub * id * A;
     }
   }
   v = segment_carry_in<R>(A, v, false);
-#pragma unroll
-  for (int k = 0; k < kSeg; ++k) {
+#pragma unroll 4
+  for (int k = 0; k < cnt; ++k) {
     const int i = i0 + k;
-    if (k < cnt && i >= 1) {
+    if (i >= 1) {
       const R sub = (i > 1) ? fup[tp(i - 1)] : R(0), id = (i == n - 1) ? iden_l : fid[tp(i)];
-      v = (x[k] - sub * v) * id;
-      x[k] = v;
+      v = (xs[32 * k] - sub * v) * id;
+      xs[32 * k] = v;
     }
   }
   // L^T rbar = z
   A = R(1);
   v = R(0);
-#pragma unroll
-  for (int k = kSeg - 1; k >= 0; --k) {
+#pragma unroll 4
+  for (int k = cnt - 1; k >= 0; --k) {
     const int i = i0 + k;
-    if (k < cnt && i >= 1) {
+    if (i >= 1) {
       const R c = (i == n - 1) ? R(0) : ((i + 1 == n - 1) ? lo_l : flo[tp(i + 1)]) * fid[tp(i)];
-      v = x[k] - c * v;
+      v = xs[32 * k] - c * v;
       A = -c * A;
     }
   }
   v = segment_carry_in<R>(A, v, true);
   R last = R(0);  // rbar of the segment's last row
-#pragma unroll
-  for (int k = kSeg - 1; k >= 0; --k) {
+#pragma unroll 4
+  for (int k = cnt - 1; k >= 0; --k) {
     const int i = i0 + k;
-    if (k < cnt && i >= 1) {
+    if (i >= 1) {
       const R c = (i == n - 1) ? R(0) : ((i + 1 == n - 1) ? lo_l : flo[tp(i + 1)]) * fid[tp(i)];
-      v = x[k] - c * v;
-      x[k] = v;
+      v = xs[32 * k] - c * v;
+      xs[32 * k] = v;
       if (k == cnt - 1) last = v;
     }
   }
   // node adjoints ybar_i = Dbar_{i-1}/h_{i-1} + wscale mm0_i - Dbar_i/h_i,
   // Dbar_i = wscale mm1_i + 6 (rbar_i - rbar_{i+1}); rbar_0 = rbar_n = 0
   const R prev_last = __shfl_up_sync(0xffffffffu, last, 1);
-  const R next_first = __shfl_down_sync(0xffffffffu, x[0], 1);
+  const R next_first = __shfl_down_sync(0xffffffffu, xs[0], 1);
   double gd = 0.0;
   if (cnt > 0) {
     R dprev = R(0);
     if (i0 > 0) {
       const R r_prev = (i0 - 1 >= 1) ? prev_last : R(0);
-      dprev = (mm(i0 - 1, 1) + R(6) * (r_prev - x[0])) * fih[tp(i0 - 1)];
+      dprev = (mm(i0 - 1, 1) + R(6) * (r_prev - xs[0])) * fih[tp(i0 - 1)];
     }
-#pragma unroll
-    for (int k = 0; k < kSeg; ++k) {
+#pragma unroll 4
+    for (int k = 0; k < cnt; ++k) {
       const int i = i0 + k;
-      if (k < cnt) {
-        const R rc = (i >= 1) ? x[k] : R(0);
-        R rn;
-        if (i + 1 >= n) rn = R(0);
-        else if (k + 1 < cnt) rn = x[(k + 1) < kSeg ? k + 1 : k];
-        else rn = next_first;
-        const R Db = mm(i, 1) + R(6) * (rc - rn);
-        yb[i * kNodeQ] = (float)(dprev + mm(i, 0) - Db * fih[tp(i)]);
-        dprev = Db * fih[tp(i)];
-        if (q == 0) gd += 2.0 * kPi * (M.node_f[i] * (double)mom(i, 0) +
-                                       (double)mom(i, 1));
-      }
+      const R rc = (i >= 1) ? xs[32 * k] : R(0);
+      R rn;
+      if (i + 1 >= n) rn = R(0);
+      else if (k + 1 < cnt) rn = xs[32 * (k + 1)];
+      else rn = next_first;
+      const R Db = mm(i, 1) + R(6) * (rc - rn);
+      yb[i * kNodeQ] = (float)(dprev + mm(i, 0) - Db * fih[tp(i)]);
+      dprev = Db * fih[tp(i)];
+      if (q == 0) gd += 2.0 * kPi * (M.node_f[i] * (double)mom(i, 0) +
+                                     (double)mom(i, 1));
     }
     if (i0 + cnt == n) yb[n * kNodeQ] = (float)dprev;
   }
@@ -1762,7 +1757,7 @@ __device__ __forceinline__ void spline_adjoint_seg(const MixedDev& M, int64_t sd
   }
 }
 
-// Register-segment adjoint, one system per warp, moments and tables read
+// Adjoint, one system per warp, moments and tables read
 // lane-strided from global memory (grids of more than 32 x 32 intervals).
 template <int kSeg>
 __global__ void __launch_bounds__(32) k_spline_adjoint(MixedDev M, double wscale) {
@@ -1778,14 +1773,16 @@ __global__ void __launch_bounds__(32) k_spline_adjoint(MixedDev M, double wscale
   const float* mom = M.mom + (size_t)sd * M.J * kNodeQ * kMoments + (size_t)q * kMoments;
   auto mat = [mom](int i, int p) { return mom[(size_t)i * kNodeQ * kMoments + p]; };
   auto tp = [](int i) { return i; };
+  __shared__ double xs[kSeg * 32];
   if (q == 0)
-    spline_adjoint_seg<kSeg, double>(M, sd, q, n, (n + 31) >> 5, wscale, spline_factor<double>(M, kGfH),
+    spline_adjoint_seg<double>(M, sd, q, n, (n + 31) >> 5, wscale, spline_factor<double>(M, kGfH),
                                      spline_factor<double>(M, kGfInvH), spline_factor<double>(M, kGfLo),
-                                     spline_factor<double>(M, kGfUp), spline_factor<double>(M, kGfInvDen), mat, tp);
+                                     spline_factor<double>(M, kGfUp), spline_factor<double>(M, kGfInvDen), mat, tp, xs);
   else
-    spline_adjoint_seg<kSeg, float>(M, sd, q, n, (n + 31) >> 5, wscale, spline_factor<float>(M, kGfH),
+    spline_adjoint_seg<float>(M, sd, q, n, (n + 31) >> 5, wscale, spline_factor<float>(M, kGfH),
                                     spline_factor<float>(M, kGfInvH), spline_factor<float>(M, kGfLo),
-                                    spline_factor<float>(M, kGfUp), spline_factor<float>(M, kGfInvDen), mat, tp);
+                                    spline_factor<float>(M, kGfUp), spline_factor<float>(M, kGfInvDen), mat, tp,
+                              reinterpret_cast<float*>(xs));
 }
 
 // Staged adjoint (32-row segments): kFitWarps systems per block; the block
@@ -1795,7 +1792,7 @@ __global__ void __launch_bounds__(32) k_spline_adjoint(MixedDev M, double wscale
 template <class R>
 __host__ __device__ __forceinline__ size_t adj_smem_bytes(int J) {
   const size_t rows = (size_t)fit_rows(J);
-  return ((5 * rows * sizeof(R) + 15) & ~(size_t)15) + (size_t)kFitWarps * rows * sizeof(float4);
+  return ((5 * rows * sizeof(R) + 15) & ~(size_t)15) + (size_t)kFitWarps * (rows * sizeof(float4) + 32 * 32 * sizeof(R));
 }
 
 template <class R>
@@ -1825,6 +1822,9 @@ __global__ void __launch_bounds__(kFitWarps * 32) k_spline_adjoint_staged(MixedD
   }
   float4* ms = reinterpret_cast<float4*>(adj_smem + ((5 * (size_t)rows * sizeof(R) + 15) & ~(size_t)15)) +
                (size_t)warp * rows;
+  R* xs = reinterpret_cast<R*>(adj_smem + ((5 * (size_t)rows * sizeof(R) + 15) & ~(size_t)15) +
+                               (size_t)kFitWarps * rows * sizeof(float4)) +
+          (size_t)warp * (32 * 32);
   const float* mom = M.mom + (size_t)sd * M.J * kNodeQ * kMoments + (size_t)q * kMoments;
   for (int i = lane; i < n; i += 32)
     ms[fit_pad(i)] = *reinterpret_cast<const float4*>(mom + (size_t)i * kNodeQ * kMoments);
@@ -1833,8 +1833,8 @@ __global__ void __launch_bounds__(kFitWarps * 32) k_spline_adjoint_staged(MixedD
     const float4 v = ms[fit_pad(i)];
     return p == 0 ? v.x : (p == 1 ? v.y : (p == 2 ? v.z : v.w));
   };
-  spline_adjoint_seg<32, R>(M, sd, q, n, 32, wscale, tab, tab + rows, tab + 2 * rows, tab + 3 * rows, tab + 4 * rows,
-                            mat, [](int i) { return fit_pad(i); });
+  spline_adjoint_seg<R>(M, sd, q, n, 32, wscale, tab, tab + rows, tab + 2 * rows, tab + 3 * rows, tab + 4 * rows,
+                         mat, [](int i) { return fit_pad(i); }, xs);
 }
 
 // ------------------------------------------------------------------ exact bins
@@ -3476,11 +3476,11 @@ static void launch_spline_fit(const MixedDev& M, int64_t B, cudaStream_t st_phas
   const unsigned bp = (unsigned)ceil_div(nsd, (int64_t)kFitWarps);
   const unsigned bt = (unsigned)ceil_div(nsd * 6, (int64_t)kFitWarps);
   if (seg == 32) {
-    k_spline_fit<32, FF><<<bp, kFitWarps * 32, fit_smem_bytes<FF, true>(M.J), st_phase>>>(M, nsd);
-    k_spline_fit<32, float><<<bt, kFitWarps * 32, fit_smem_bytes<float, true>(M.J), st_transfer>>>(M, nsd * 6);
+    k_spline_fit<32, FF><<<bp, kFitWarps * 32, fit_smem_bytes<FF, true, 32>(M.J), st_phase>>>(M, nsd);
+    k_spline_fit<32, float><<<bt, kFitWarps * 32, fit_smem_bytes<float, true, 32>(M.J), st_transfer>>>(M, nsd * 6);
   } else {
-    k_spline_fit<kSegMax, FF><<<bp, kFitWarps * 32, fit_smem_bytes<FF, false>(M.J), st_phase>>>(M, nsd);
-    k_spline_fit<kSegMax, float><<<bt, kFitWarps * 32, fit_smem_bytes<float, false>(M.J), st_transfer>>>(M,
+    k_spline_fit<kSegMax, FF><<<bp, kFitWarps * 32, fit_smem_bytes<FF, false, kSegMax>(M.J), st_phase>>>(M, nsd);
+    k_spline_fit<kSegMax, float><<<bt, kFitWarps * 32, fit_smem_bytes<float, false, kSegMax>(M.J), st_transfer>>>(M,
                                                                                                        nsd * 6);
   }
 }
@@ -3530,18 +3530,18 @@ int mixed_create(PesPlan* p) {
   const int64_t V = B * M.n_modes;  // virtual samples (sample, mode)
   if (spline_seg(J) == 32) {
     PES_CHECK_CUDA(cudaFuncSetAttribute(k_spline_fit<32, FF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)fit_smem_bytes<FF, true>(J)));
+                                        (int)fit_smem_bytes<FF, true, 32>(J)));
     PES_CHECK_CUDA(cudaFuncSetAttribute(k_spline_fit<32, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)fit_smem_bytes<float, true>(J)));
+                                        (int)fit_smem_bytes<float, true, 32>(J)));
     PES_CHECK_CUDA(cudaFuncSetAttribute(k_spline_adjoint_staged<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)adj_smem_bytes<double>(J)));
     PES_CHECK_CUDA(cudaFuncSetAttribute(k_spline_adjoint_staged<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)adj_smem_bytes<float>(J)));
   } else if (spline_seg(J) == kSegMax) {
     PES_CHECK_CUDA(cudaFuncSetAttribute(k_spline_fit<kSegMax, FF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)fit_smem_bytes<FF, false>(J)));
+                                        (int)fit_smem_bytes<FF, false, kSegMax>(J)));
     PES_CHECK_CUDA(cudaFuncSetAttribute(k_spline_fit<kSegMax, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)fit_smem_bytes<float, false>(J)));
+                                        (int)fit_smem_bytes<float, false, kSegMax>(J)));
   }
   M.scale = 3.085677581491367e16 / (1.476625038050124729627979840144936351e3 * 4.925490947641266978197229498498379006e-6);
   M.scale_ff = ff_from(M.scale);
