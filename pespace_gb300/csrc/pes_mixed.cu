@@ -416,8 +416,8 @@ __device__ __forceinline__ void load_block(const SampleBlock<T>* blocks, int s, 
 
 // Kink coefficients per (virtual sample, detector): the amplitude kink of
 // the sample's model (IMRPhenomD), or of mode k (IMRPhenomHM: hm_kink).
-__global__ void k_kink(PlanDev P, MixedDev M, GenArg G, const SampleBlock<double>* __restrict__ blocks, int64_t B) {
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+__device__ __forceinline__ void kink_sample(const PlanDev& P, const MixedDev& M, const GenArg& G,
+                                            const SampleBlock<double>* __restrict__ blocks, int64_t B, int64_t t) {
   if (t >= B * M.n_modes * (int64_t)M.n_det) return;
   const int64_t v = t / M.n_det;
   const int d = (int)(t % M.n_det);
@@ -842,7 +842,7 @@ __global__ void __launch_bounds__(kSparseThreads, 3) k_sparse_bwd_split(PlanDev 
 // live bin; xbin: bins below the first interval whose yearly orbital phase
 // advance omega |t(f_{j+1}) - t(f_j)| is at most kOrbitPhaseMax (that advance
 // falls monotonically with f over the inspiral, so a bisection finds it).
-// k_mixed_ranges writes nsp and nch (needed by the sparse stage),
+// range_sample writes nsp and nch (needed by the sparse stage),
 // k_exact_ranges xbin (needed from the exact bins and the run anchors on), so
 // the bisection can run on the side stream.
 __device__ __forceinline__ void range_counts(const MixedDev& M, int64_t kc, int& ns, int& nc) {
@@ -856,10 +856,10 @@ __device__ __forceinline__ void range_counts(const MixedDev& M, int64_t kc, int&
   ns = min(max(M.ch_iv[lo] + 1, 3), M.J - 1);
 }
 
-__global__ void k_mixed_ranges(PlanDev P, MixedDev M, const SampleBlock<double>* __restrict__ blocks, int64_t B) {
-  // kPart 0: one thread per virtual sample v
+__device__ __forceinline__ void range_sample(const PlanDev& P, const MixedDev& M,
+                                             const SampleBlock<double>* __restrict__ blocks, int64_t B, int64_t t) {
+  // one thread per virtual sample
   const int nm = M.n_modes;
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t < 2) M.rcount[t] = 0;  // this call's re-evaluation lists
   if (t >= B * nm) return;
   const int64_t s = t / nm;
@@ -920,6 +920,17 @@ __global__ void k_mixed_ranges(PlanDev P, MixedDev M, const SampleBlock<double>*
   if (kc > 0) range_counts(M, kc, ns, nc);
   M.nsp[t] = ns;
   M.nch[t] = nc;
+}
+
+// The ranges (the first range_blocks blocks) beside the kinks: two chains of FP64
+// operations that the node stage waits for (one after the other 7 + 47 us, with six
+// modes 43 + 54).
+__global__ void k_ranges_kink(PlanDev P, MixedDev M, GenArg G, const SampleBlock<double>* __restrict__ blocks,
+                              int64_t B, int range_blocks) {
+  if ((int)blockIdx.x < range_blocks)
+    range_sample(P, M, blocks, B, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
+  else
+    kink_sample(P, M, G, blocks, B, (blockIdx.x - range_blocks) * (int64_t)blockDim.x + threadIdx.x);
 }
 
 // xbin, xbind: a pair of threads per (sample, mode, detector), one for t(f) at
@@ -3921,6 +3932,13 @@ int mixed_ingest(PesPlan* p, int det, const double* data, const double* psd, cud
 }
 
 // The value set-up: IMRPhenomD plans in the plain order (phenomd_setup_serial).
+static void launch_ranges_kink(PesPlan* p, const SampleBlock<double>* blocks, int64_t B, cudaStream_t st) {
+  const MixedDev& M = p->mixed->dev;
+  const int64_t V = B * M.n_modes;
+  const unsigned ranges = ceil_div(V, p->sample_threads), kinks = ceil_div(V * M.n_det, p->sample_threads);
+  k_ranges_kink<<<ranges + kinks, p->sample_threads, 0, st>>>(p->dev, M, p->mixed->gen, blocks, B, (int)ranges);
+}
+
 // blocks of sample_threads threads, or of one sample's group where that is larger
 static void launch_exact_ranges(PesPlan* p, const SampleBlock<double>* blocks, int64_t B, cudaStream_t st) {
   const MixedDev& M = p->mixed->dev;
@@ -3945,10 +3963,9 @@ int mixed_model(PesPlan* p, const double* theta_dev, double* out, cudaStream_t s
   launch_setup(p, theta_dev, 1, blocks, st);
   PES_CHECK_LAUNCH();
   const unsigned nm = (unsigned)M.n_modes;
-  k_mixed_ranges<<<1, 64, 0, st>>>(p->dev, M, blocks, 1);
+  launch_ranges_kink(p, blocks, 1, st);
   launch_exact_ranges(p, blocks, 1, st);
   PES_CHECK_LAUNCH();
-  k_kink<<<1, 64, 0, st>>>(p->dev, M, G, blocks, 1);
   PES_CHECK_LAUNCH();
   k_sparse_fwd<false><<<dim3(M.nblk_sparse, M.n_det, nm), kSparseThreads, 0, st>>>(p->dev, M, G, blocks);
   PES_CHECK_LAUNCH();
@@ -4019,11 +4036,6 @@ int mixed_lnl(PesPlan* p, const double* theta, int64_t B, double* lnl, double* g
     launch_setup(p, theta, B, blocks, st);
   }
   PES_CHECK_LAUNCH();
-  {
-    ProfScope ps(p, kKOther, st);
-    k_mixed_ranges<<<ceil_div(V, 64), 64, 0, st>>>(p->dev, M, blocks, B);
-  }
-  PES_CHECK_LAUNCH();
   // side stream: the exact-bin range, the exact bins and the gradient set-up they need
   cudaStream_t side = p->mixed->side;
   PES_CHECK_CUDA(cudaEventRecord(p->mixed->fork, st));
@@ -4073,7 +4085,7 @@ int mixed_lnl(PesPlan* p, const double* theta, int64_t B, double* lnl, double* g
   // (the side stream's completion is recorded after the exact re-evaluation below)
   {
     ProfScope ps(p, kKSparse, st);
-    k_kink<<<ceil_div(V * M.n_det, p->sample_threads), p->sample_threads, 0, st>>>(p->dev, M, G, blocks, B);
+    launch_ranges_kink(p, blocks, B, st);
   }
   PES_CHECK_LAUNCH();
   cudaStream_t aux = p->mixed->aux;
