@@ -103,6 +103,26 @@ PES_HD FF ff_addf(const FF& x, float y) {
   s.lo += x.lo;
   return ff_fast_two_sum(s.hi, s.lo);
 }
+// Forms without renormalisation: the tail stays within a few ulps of the largest
+// term's head, and a result can go into another of them or be added up.
+PES_HD FF ff_mad(const FF& p, const FF& x, const FF& c) {  // p x + c
+  const float t = p.hi * x.hi;
+  const float e = fmaf(p.hi, x.lo, fmaf(p.lo, x.hi, fmaf(p.hi, x.hi, -t)));
+  const FF s = ff_two_sum(t, c.hi);
+  return ff_make(s.hi, (s.lo + e) + c.lo);
+}
+PES_HD FF ff_dot2(const FF& a, const FF& b, const FF& c, const FF& d) {  // a b + c d
+  const float p = a.hi * b.hi, q = c.hi * d.hi;
+  float e = fmaf(a.hi, b.hi, -p) + fmaf(c.hi, d.hi, -q);
+  e = fmaf(a.hi, b.lo, fmaf(a.lo, b.hi, e));
+  e = fmaf(c.hi, d.lo, fmaf(c.lo, d.hi, e));
+  const FF s = ff_two_sum(p, q);
+  return ff_make(s.hi, s.lo + e);
+}
+PES_HD FF ff_add_lazy(const FF& a, const FF& b) {
+  const FF s = ff_two_sum(a.hi, b.hi);
+  return ff_make(s.hi, s.lo + (a.lo + b.lo));
+}
 PES_HD FF operator/(const FF& x, const FF& y) {
   const float r = ff_rcp(y.hi);
   const float q1 = x.hi * r;

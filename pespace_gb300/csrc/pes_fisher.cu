@@ -381,13 +381,6 @@ __global__ void __launch_bounds__(64) k_fisher_prep(double scale, const SampleBl
   }
 }
 
-// p x + c without renormalisation (the tail stays within a few ulps of the head)
-__device__ __forceinline__ FF ff_mad(const FF& p, const FF& x, const FF& c) {
-  const float t = p.hi * x.hi;
-  const float e = fmaf(p.hi, x.lo, fmaf(p.lo, x.hi, fmaf(p.hi, x.hi, -t)));
-  const FF s = ff_two_sum(t, c.hi);
-  return ff_make(s.hi, (s.lo + e) + c.lo);
-}
 __device__ __forceinline__ FF ff_load(const float2& a) { return ff_make(a.x, a.y); }
 
 // The waveform's part of a bin: amplitude, t(f), and the tangents over ln Mc, q, chi_1, chi_2.

@@ -186,6 +186,7 @@ struct MixedDev {
   // float-float from the same splines (rounding: k_dense_ff), or exactly
   // (spline error: k_exact<3>).
   int32_t* rkind;           // [B] kRefineNone, kRefineFF or kRefineExact
+  const float4* trig_ff;    // [256] sine, cosine of 2 pi k / 256 (hi, lo pairs)
   int32_t nblk_ff;          // float-float partial sums per sample
   double* fpart;            // [B][nblk_ff] float-float dense-range partials
   // Float-float copies of the FP64 inputs of one bin for k_dense_ff, six rows
@@ -275,6 +276,7 @@ struct MixedBuffers {
   // the gradient pass of the dense stage stages its run inputs through shared
   // memory when they exceed half of L2 (they then stream from DRAM)
   bool stage_grad = false;
+  int sms = 1;
   int64_t exact_grid = 1, ff_grid = 1;  // blocks of the re-evaluations that the device holds
   cudaEvent_t ev_nodes = nullptr, ev_tfit = nullptr, ev_dense = nullptr, ev_tadj = nullptr, ev_hd = nullptr, ev_pfit = nullptr,
               ev_kink = nullptr, ev_xgrad = nullptr;
@@ -1448,7 +1450,11 @@ template <class R> __device__ __forceinline__ R ff_to_r(const FF& x);
 template <> __device__ __forceinline__ float ff_to_r<float>(const FF& x) { return x.hi; }
 template <> __device__ __forceinline__ FF ff_to_r<FF>(const FF& x) { return x; }
 
-constexpr int kFitWarps = 4;  // systems per block of the staged fit
+constexpr int kFitWarps = 4;  // systems per block of the staged fit and adjoint
+// systems per block of the fit: six where the tables are staged in FP32 (two blocks per SM
+// then hold 12 systems, four per block 8)
+template <class R, bool kStageTables>
+constexpr int kFitSystems = kStageTables && std::is_same<R, float>::value ? 6 : kFitWarps;
 __host__ __device__ __forceinline__ int fit_pad(int i) { return i + (i >> 5); }
 __host__ __device__ __forceinline__ int fit_rows(int J) { return fit_pad(J) + 1; }
 
@@ -1467,7 +1473,7 @@ __host__ __device__ __forceinline__ size_t fit_smem_bytes(int J) {
   const size_t tables =
       kStageTables ? 5 * rows * sizeof(R) + (std::is_same<R, FF>::value ? 0 : rows * sizeof(FF)) : 0;
   return ((tables + 15) & ~(size_t)15) +
-         (size_t)kFitWarps * (rows * sizeof(FF) + 4 * sizeof(FF) + kSeg * 32 * sizeof(R));
+         (size_t)kFitSystems<R, kStageTables> * (rows * sizeof(FF) + 4 * sizeof(FF) + kSeg * 32 * sizeof(R));
 }
 
 template <int kSeg, class R, bool kStageTables>
@@ -1592,7 +1598,7 @@ __device__ __forceinline__ void spline_fit_staged(const MixedDev& M, int64_t sd,
 // kFitWarps systems per block.  R = FF: the phase systems (one per sample and
 // detector, q = 0); R = float: the six transfer systems (q = 1..6).
 template <int kSeg, class R>
-__global__ void __launch_bounds__(kFitWarps * 32, 3) k_spline_fit(MixedDev M, int64_t n_sys) {
+__global__ void __launch_bounds__(kFitSystems<R, kSeg == 32> * 32, 2) k_spline_fit(MixedDev M, int64_t n_sys) {
   extern __shared__ __align__(16) unsigned char fit_smem[];
   constexpr bool kPhase = std::is_same<R, FF>::value;
   constexpr bool kStage = kSeg == 32;
@@ -1633,7 +1639,7 @@ __global__ void __launch_bounds__(kFitWarps * 32, 3) k_spline_fit(MixedDev M, in
     }
   }
   __syncthreads();
-  const int64_t sys = (int64_t)blockIdx.x * kFitWarps + warp;
+  const int64_t sys = (int64_t)blockIdx.x * kFitSystems<R, kStage> + warp;
   if (sys >= n_sys) return;
   const int64_t sd = kPhase ? sys : sys / 6;
   const int q = kPhase ? 0 : 1 + (int)(sys % 6);
@@ -1648,11 +1654,11 @@ __global__ void __launch_bounds__(kFitWarps * 32, 3) k_spline_fit(MixedDev M, in
 // Transpose of the fit with the same lane segments.  mom(i, p) gives the
 // interval moments, the tables are indexed through tp (padded rows when they
 // were staged in shared memory).
-template <class R, class MomAt, class TabIdx>
+template <class R, class MomAt, class TabIdx, class Unknown>
 __device__ __forceinline__ void spline_adjoint_seg(const MixedDev& M, int64_t sd, int q, int n, int seg, double wscale,
                                                    const R* __restrict__ fh, const R* __restrict__ fih,
                                                    const R* __restrict__ flo, const R* __restrict__ fup,
-                                                   const R* __restrict__ fid, MomAt mom, TabIdx tp, R* xs) {
+                                                   const R* __restrict__ fid, MomAt mom, TabIdx tp, Unknown xat) {
   const int lane = threadIdx.x & 31;
   float* __restrict__ yb = M.ybar + (size_t)sd * M.J * kNodeQ + q;
   const int i0 = min(n, lane * seg), cnt = min(n, i0 + seg) - i0;
@@ -1668,10 +1674,9 @@ __device__ __forceinline__ void spline_adjoint_seg(const MixedDev& M, int64_t sd
   nak_row(M.node_f, n, n - 1, lo_d, di_d, up_d);
   const R lo_l = (R)lo_d, iden_l = (R)(1.0 / (di_d - lo_d * M.gcp[n - 2]));
   // right-hand sides (coefficient adjoints -> mbar, end eliminations), in FP64
-  xs += lane;  // x_k at xs[32 k]
-  if (cnt == 0) xs[0] = R(0);
   {
     R right_prev = (i0 >= 1) ? mbar_right(i0 - 1) : R(0);
+    __syncwarp();  // the neighbour's row may hold its unknown from here on
 #pragma unroll 4
     for (int k = 0; k < cnt; ++k) {
       const int i = i0 + k;
@@ -1684,8 +1689,8 @@ __device__ __forceinline__ void spline_adjoint_seg(const MixedDev& M, int64_t sd
         if (i == n - 1) w += mbn * (ha + hb) / ha;
         if (i == n - 2) w -= mbn * hb / ha;
       }
-      xs[32 * k] = w;
       right_prev = mbar_right(i);
+      xat(i, k) = w;
     }
   }
   // U^T z = mbar
@@ -1695,7 +1700,7 @@ __device__ __forceinline__ void spline_adjoint_seg(const MixedDev& M, int64_t sd
     const int i = i0 + k;
     if (i >= 1) {
       const R sub = (i > 1) ? fup[tp(i - 1)] : R(0), id = (i == n - 1) ? iden_l : fid[tp(i)];
-      v = (xs[32 * k] - sub * v) * id;
+      v = (xat(i, k) - sub * v) * id;
       A = -sub * id * A;
     }
   }
@@ -1705,8 +1710,8 @@ __device__ __forceinline__ void spline_adjoint_seg(const MixedDev& M, int64_t sd
     const int i = i0 + k;
     if (i >= 1) {
       const R sub = (i > 1) ? fup[tp(i - 1)] : R(0), id = (i == n - 1) ? iden_l : fid[tp(i)];
-      v = (xs[32 * k] - sub * v) * id;
-      xs[32 * k] = v;
+      v = (xat(i, k) - sub * v) * id;
+      xat(i, k) = v;
     }
   }
   // L^T rbar = z
@@ -1717,7 +1722,7 @@ __device__ __forceinline__ void spline_adjoint_seg(const MixedDev& M, int64_t sd
     const int i = i0 + k;
     if (i >= 1) {
       const R c = (i == n - 1) ? R(0) : ((i + 1 == n - 1) ? lo_l : flo[tp(i + 1)]) * fid[tp(i)];
-      v = xs[32 * k] - c * v;
+      v = xat(i, k) - c * v;
       A = -c * A;
     }
   }
@@ -1728,29 +1733,30 @@ __device__ __forceinline__ void spline_adjoint_seg(const MixedDev& M, int64_t sd
     const int i = i0 + k;
     if (i >= 1) {
       const R c = (i == n - 1) ? R(0) : ((i + 1 == n - 1) ? lo_l : flo[tp(i + 1)]) * fid[tp(i)];
-      v = xs[32 * k] - c * v;
-      xs[32 * k] = v;
+      v = xat(i, k) - c * v;
+      xat(i, k) = v;
       if (k == cnt - 1) last = v;
     }
   }
   // node adjoints ybar_i = Dbar_{i-1}/h_{i-1} + wscale mm0_i - Dbar_i/h_i,
   // Dbar_i = wscale mm1_i + 6 (rbar_i - rbar_{i+1}); rbar_0 = rbar_n = 0
   const R prev_last = __shfl_up_sync(0xffffffffu, last, 1);
-  const R next_first = __shfl_down_sync(0xffffffffu, xs[0], 1);
+  const R x_first = cnt > 0 ? xat(i0, 0) : R(0);
+  const R next_first = __shfl_down_sync(0xffffffffu, x_first, 1);
   double gd = 0.0;
   if (cnt > 0) {
     R dprev = R(0);
     if (i0 > 0) {
       const R r_prev = (i0 - 1 >= 1) ? prev_last : R(0);
-      dprev = (mm(i0 - 1, 1) + R(6) * (r_prev - xs[0])) * fih[tp(i0 - 1)];
+      dprev = (mm(i0 - 1, 1) + R(6) * (r_prev - x_first)) * fih[tp(i0 - 1)];
     }
 #pragma unroll 4
     for (int k = 0; k < cnt; ++k) {
       const int i = i0 + k;
-      const R rc = (i >= 1) ? xs[32 * k] : R(0);
+      const R rc = (i >= 1) ? xat(i, k) : R(0);
       R rn;
       if (i + 1 >= n) rn = R(0);
-      else if (k + 1 < cnt) rn = xs[32 * (k + 1)];
+      else if (k + 1 < cnt) rn = xat(i + 1, k + 1);
       else rn = next_first;
       const R Db = mm(i, 1) + R(6) * (rc - rn);
       yb[i * kNodeQ] = (float)(dprev + mm(i, 0) - Db * fih[tp(i)]);
@@ -1784,16 +1790,18 @@ __global__ void __launch_bounds__(32) k_spline_adjoint(MixedDev M, double wscale
   const float* mom = M.mom + (size_t)sd * M.J * kNodeQ * kMoments + (size_t)q * kMoments;
   auto mat = [mom](int i, int p) { return mom[(size_t)i * kNodeQ * kMoments + p]; };
   auto tp = [](int i) { return i; };
-  __shared__ double xs[kSeg * 32];
+  __shared__ double xs[kSeg * 32];  // row k of lane l at 32 k + l
+  auto xd = [lane](int, int k) -> double& { return xs[32 * k + lane]; };
+  auto xf = [lane](int, int k) -> float& { return reinterpret_cast<float*>(xs)[32 * k + lane]; };
   if (q == 0)
     spline_adjoint_seg<double>(M, sd, q, n, (n + 31) >> 5, wscale, spline_factor<double>(M, kGfH),
                                      spline_factor<double>(M, kGfInvH), spline_factor<double>(M, kGfLo),
-                                     spline_factor<double>(M, kGfUp), spline_factor<double>(M, kGfInvDen), mat, tp, xs);
+                                     spline_factor<double>(M, kGfUp), spline_factor<double>(M, kGfInvDen), mat, tp, xd);
   else
     spline_adjoint_seg<float>(M, sd, q, n, (n + 31) >> 5, wscale, spline_factor<float>(M, kGfH),
                                     spline_factor<float>(M, kGfInvH), spline_factor<float>(M, kGfLo),
                                     spline_factor<float>(M, kGfUp), spline_factor<float>(M, kGfInvDen), mat, tp,
-                              reinterpret_cast<float*>(xs));
+                              xf);
 }
 
 // Staged adjoint (32-row segments): kFitWarps systems per block; the block
@@ -1803,7 +1811,7 @@ __global__ void __launch_bounds__(32) k_spline_adjoint(MixedDev M, double wscale
 template <class R>
 __host__ __device__ __forceinline__ size_t adj_smem_bytes(int J) {
   const size_t rows = (size_t)fit_rows(J);
-  return ((5 * rows * sizeof(R) + 15) & ~(size_t)15) + (size_t)kFitWarps * (rows * sizeof(float4) + 32 * 32 * sizeof(R));
+  return ((5 * rows * sizeof(R) + 15) & ~(size_t)15) + (size_t)kFitWarps * rows * sizeof(float4);
 }
 
 template <class R>
@@ -1833,9 +1841,6 @@ __global__ void __launch_bounds__(kFitWarps * 32) k_spline_adjoint_staged(MixedD
   }
   float4* ms = reinterpret_cast<float4*>(adj_smem + ((5 * (size_t)rows * sizeof(R) + 15) & ~(size_t)15)) +
                (size_t)warp * rows;
-  R* xs = reinterpret_cast<R*>(adj_smem + ((5 * (size_t)rows * sizeof(R) + 15) & ~(size_t)15) +
-                               (size_t)kFitWarps * rows * sizeof(float4)) +
-          (size_t)warp * (32 * 32);
   const float* mom = M.mom + (size_t)sd * M.J * kNodeQ * kMoments + (size_t)q * kMoments;
   for (int i = lane; i < n; i += 32)
     ms[fit_pad(i)] = *reinterpret_cast<const float4*>(mom + (size_t)i * kNodeQ * kMoments);
@@ -1845,7 +1850,9 @@ __global__ void __launch_bounds__(kFitWarps * 32) k_spline_adjoint_staged(MixedD
     return p == 0 ? v.x : (p == 1 ? v.y : (p == 2 ? v.z : v.w));
   };
   spline_adjoint_seg<R>(M, sd, q, n, 32, wscale, tab, tab + rows, tab + 2 * rows, tab + 3 * rows, tab + 4 * rows,
-                         mat, [](int i) { return fit_pad(i); }, xs);
+                         mat, [](int i) { return fit_pad(i); },
+                         // a row's unknown in the place of its moments 2 and 3, which only its right-hand side reads
+                         [ms](int i, int) -> R& { return *reinterpret_cast<R*>(&ms[fit_pad(i)].z); });
 }
 
 // ------------------------------------------------------------------ exact bins
@@ -2950,6 +2957,41 @@ __global__ void __launch_bounds__(kMixThreads, 5) k_dense_mixed(PlanDev P, Mixed
 // the groups' phase anchors (run, mode, detector), then its warps every fourth
 // run, a bin per lane (32 runs per warp left a call of 16 samples with less
 // than one warp per SM partition).  Partials: fpart [B][nblk_ff].
+constexpr int kFfTrig = 256;
+__global__ void k_trig_ff(float4* __restrict__ tab) {
+  double sn, cs;
+  sincospi(2.0 * (double)threadIdx.x / kFfTrig, &sn, &cs);
+  const FF a = ff_from(sn), b = ff_from(cs);
+  tab[threadIdx.x] = make_float4(a.hi, a.lo, b.hi, b.lo);
+}
+
+// sin and cos of |x| < 1e4: x = k 2 pi / 256 + r, |r| <= pi / 256, the table's
+// entry turned by r (sine and cosine - 1 of r by Taylor series: r and r^2 / 2 in
+// float-float, the rest in FP32, below 1e-13).  The step 2 pi / 256 in three parts;
+// k times the first, subtracted from x.hi, is exact (within a factor two of it for
+// k != 0).  About 75 operations against 250 of the general function.
+__device__ __forceinline__ void sincos_tab(const float4* __restrict__ tab, const FF& x, FF* sn, FF* cs) {
+  constexpr float c1 = 2.454369328916072845458984375e-02f;  // 2 pi / 256 rounded
+  constexpr float c2 = (float)(6.283185307179586476925 / 256.0 - (double)c1);
+  constexpr float c3 = (float)(6.283185307179586476925 / 256.0 - (double)c1 - (double)c2 + 2.4492935982947064e-16 / 256.0);
+  const float kf = rintf(x.hi * 40.74366543152521f);
+  const float p = kf * c1, pe = fmaf(kf, c1, -p);
+  const FF a = ff_two_sum(x.hi - p, x.lo);
+  const FF b = ff_two_prod(kf, c2);
+  const FF d = ff_two_sum(a.hi, -b.hi);
+  const FF r = ff_fast_two_sum(d.hi, d.lo + ((a.lo - pe) - fmaf(kf, c3, b.lo)));
+  const float z = r.hi * r.hi;
+  const FF sr = ff_make(r.hi, fmaf(r.hi * z, fmaf(z, 1.0f / 120.0f, -1.0f / 6.0f), r.lo));
+  // cos r - 1 = -r^2 / 2 + r^4 / 24 - r^6 / 720
+  const FF cr = ff_make(-0.5f * z, fmaf(-0.5f, fmaf(r.hi, r.hi, -z), -(r.hi * r.lo)) +
+                                       z * z * fmaf(z, -1.0f / 720.0f, 1.0f / 24.0f));
+  const float4 e = tab[(int)kf & (kFfTrig - 1)];
+  const FF S = ff_make(e.x, e.y), C = ff_make(e.z, e.w);
+  const FF u = ff_add_lazy(S, ff_dot2(S, cr, C, sr)), v = ff_add_lazy(C, ff_dot2(C, cr, -S, sr));
+  *sn = ff_fast_two_sum(u.hi, u.lo);
+  *cs = ff_fast_two_sum(v.hi, v.lo);
+}
+
 template <int kNM>
 __global__ void __launch_bounds__(kMixThreads) k_dense_ff(PlanDev P, MixedDev M,
                                                           const SampleBlock<double>* __restrict__ blocks) {
@@ -2958,7 +3000,10 @@ __global__ void __launch_bounds__(kMixThreads) k_dense_ff(PlanDev P, MixedDev M,
   __shared__ float4 anc[PES_MAX_DETECTORS][kNM][kChunkMax][2];
   __shared__ int ancq[PES_MAX_DETECTORS][kNM][kChunkMax];
   __shared__ double red[kMixThreads / 32];
+  __shared__ float4 tab[kFfTrig];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if ((int)blockIdx.x >= M.rcount[0] * M.nblk_ff) return;
+  for (int k = threadIdx.x; k < kFfTrig; k += kMixThreads) tab[k] = M.trig_ff[k];  // (the anchors' barrier follows)
   for (int item = blockIdx.x; item < M.rcount[0] * M.nblk_ff; item += gridDim.x) {
     const int s = M.rlist[item / M.nblk_ff], blk = item % M.nblk_ff;
     const int first = blk * kChunkMax;
@@ -3002,6 +3047,9 @@ __global__ void __launch_bounds__(kMixThreads) k_dense_ff(PlanDev P, MixedDev M,
         const float2 nfj = M.node_ff[j];
         const FF t = f - ff_make(nfj.x, nfj.y);
         const float tf = t.hi, u = (float)lane;
+        const float4* X = M.xff + (size_t)d * 6 * P.nbins + i;
+        const float4 x3 = X[3 * (size_t)P.nbins], x4 = X[4 * (size_t)P.nbins], x5 = X[5 * (size_t)P.nbins];
+        const FF pr = ff_make(x4.z, x4.w), pim = ff_make(x5.x, x5.y);
         FF hr[3], hi[3];
 #pragma unroll
         for (int ch = 0; ch < 3; ++ch) hr[ch] = hi[ch] = ff_make(0.0f, 0.0f);
@@ -3011,9 +3059,10 @@ __global__ void __launch_bounds__(kMixThreads) k_dense_ff(PlanDev P, MixedDev M,
           if (kNM > 1 && (c >= M.nch[v] || i >= M.vcut[v])) continue;  // past the mode's range
           const size_t sdk = sd + (size_t)k * M.n_det;
           const float4 a0 = anc[d][k][c - first][0], a1 = anc[d][k][c - first][1];
-          FF ph = ff_make(a0.x, a0.y) + ff_mulf(ff_make(a0.z, a0.w), u);
-          ph = ph + ff_mulf(ff_make(a1.x, a1.y), u * u);  // u^2, u^3 < 2^15: exact
-          ph = ph + ff_mulf(ff_make(a1.z, a1.w), u * u * u);
+          // u, u^2, u^3 < 2^15: exact
+          FF ph = ff_mad(ff_make(a0.z, a0.w), ff_make(u, 0.0f), ff_make(a0.x, a0.y));
+          ph = ff_mad(ff_make(a1.x, a1.y), ff_make(u * u, 0.0f), ph);
+          ph = ff_mad(ff_make(a1.z, a1.w), ff_make(u * u * u, 0.0f), ph);
           const float4 sa = M.sff[2 * v];
           const FF msf = ff_make(sa.z, sa.w);
           if (kNM > 1) {
@@ -3021,11 +3070,18 @@ __global__ void __launch_bounds__(kMixThreads) k_dense_ff(PlanDev P, MixedDev M,
             if (qk >= 0) {
               const float4 k4 = M.pkink[2 * v + qk];
               const FF xq = msf * f - ff_make(k4.x, k4.y);
-              if (xq.hi > 0.0f) ph = ph + ff_make(k4.z, k4.w) * (xq * xq);
+              if (xq.hi > 0.0f) ph = ff_mad(xq * xq, ff_make(k4.z, k4.w), ph);
             }
           }
+          ph = ff_fast_two_sum(ph.hi, ph.lo);
           FF sn, cs;
-          dsincos(ff_wrap_2pi(ph), &sn, &cs);
+          sincos_tab(tab, ph, &sn, &cs);
+          if (kNM == 1) {
+            // the TDI prefactor on the phasor: (cos - i sin)(Pr + i Pi)
+            const FF er_ = ff_dot2(cs, pr, sn, pim), ei_ = ff_dot2(sn, pr, -cs, pim);
+            cs = er_;
+            sn = ei_;
+          }
           // the mode's transfer quantities on interval j: the spline (value and
           // slope coefficients in float-float), its midpoint correction, the kink
           const float4* G = M.cg + (sdk * M.J + j) * 8;
@@ -3058,30 +3114,35 @@ __global__ void __launch_bounds__(kMixThreads) k_dense_ff(PlanDev P, MixedDev M,
             for (int pp = 0; pp < 2; ++pp) {
               const int q = 2 * ch + pp;
               const float4 c4 = G[q];
-              FF gq = ff_make(c4.x, alo[q]) + t * ff_addf(ff_make(c4.y, blo[q]), tf * fmaf(tf, c4.w, c4.z));
-              gq = ff_addf(gq, bump[q]);
-              if (kinked) gq = gq + ff_make(kfh[q], kfl[q]) * x2;
+              const FF in = ff_two_sum(c4.y, tf * fmaf(tf, c4.w, c4.z));
+              FF gq = ff_mad(t, ff_make(in.hi, in.lo + blo[q]), ff_make(c4.x, alo[q]));
+              gq.lo += bump[q];
+              if (kinked) gq = ff_mad(x2, ff_make(kfh[q], kfl[q]), gq);
               g[pp] = gq;
             }
             // G e^{-i phase} = (g0 + i g1)(cos - i sin)
-            hr[ch] = hr[ch] + (g[0] * cs + g[1] * sn);
-            hi[ch] = hi[ch] + (g[1] * cs - g[0] * sn);
+            const FF xr = ff_dot2(g[0], cs, g[1], sn), xi = ff_dot2(g[1], cs, -g[0], sn);
+            hr[ch] = kNM == 1 ? xr : ff_add_lazy(hr[ch], xr);
+            hi[ch] = kNM == 1 ? xi : ff_add_lazy(hi[ch], xi);
           }
         }
-        // TDI prefactor, residual against the data, weight
-        const float4* X = M.xff + (size_t)d * 6 * P.nbins + i;
-        const float4 x3 = X[3 * (size_t)P.nbins], x4 = X[4 * (size_t)P.nbins], x5 = X[5 * (size_t)P.nbins];
-        const FF pr = ff_make(x4.z, x4.w), pim = ff_make(x5.x, x5.y);
+        // (several modes: the TDI prefactor), residual against the data, weight
         const FF wch[3] = {ff_make(x3.x, x3.y), ff_make(x3.z, x3.w), ff_make(x4.x, x4.y)};
 #pragma unroll
         for (int ch = 0; ch < 3; ++ch) {
           const float4 dv = X[(size_t)ch * P.nbins];
-          const FF er = ff_make(dv.x, dv.y) - (hr[ch] * pr - hi[ch] * pim);
-          const FF ei = ff_make(dv.z, dv.w) - (hr[ch] * pim + hi[ch] * pr);
-          acc = acc + (er * er + ei * ei) * wch[ch];
+          FF mr = hr[ch], mi = hi[ch];
+          if (kNM > 1) {
+            mr = ff_dot2(hr[ch], pr, -hi[ch], pim);
+            mi = ff_dot2(hr[ch], pim, hi[ch], pr);
+          }
+          const FF er = ff_add_lazy(ff_make(dv.x, dv.y), -mr), ei = ff_add_lazy(ff_make(dv.z, dv.w), -mi);
+          const FF r2 = ff_dot2(er, er, ei, ei);
+          acc = ff_mad(r2, wch[ch], acc);
         }
       }
     }
+    acc = ff_fast_two_sum(acc.hi, acc.lo);
     // lanes and warps in float-float, the block partial in FP64
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -3109,7 +3170,8 @@ __global__ void __launch_bounds__(kMixThreads) k_dense_ff(PlanDev P, MixedDev M,
 // coefficients of |G_c|^2: no per-bin rounding of the model.  Float-float on
 // the FP32 pipes, in the interval's variable u = t / h (so that the moments
 // sum u^p W stay in range); in FP64 this kernel bound the FP64 pipe.
-constexpr int kHdThreads = 128;  // one block per (sample, detector), threads over its intervals
+// one block per (sample, detector), threads over its intervals: 128, or 512 in calls of
+// fewer blocks than the chip has SMs (16 samples on 1024 intervals 65 us at 128)
 __device__ __forceinline__ FF hd_piece(const FF (&A)[6], const FF (&Bc)[6], const FF (&Cc)[6], const FF (&Dc)[6],
                                        const FF* Sm) {
   FF acc = ff_make(0.0f, 0.0f);
@@ -3129,6 +3191,7 @@ __device__ __forceinline__ FF hd_piece(const FF (&A)[6], const FF (&Bc)[6], cons
   return acc;
 }
 
+template <int kHdThreads>
 __global__ void __launch_bounds__(kHdThreads) k_hd(PlanDev P, MixedDev M,
                                                   const SampleBlock<double>* __restrict__ blocks, int64_t B) {
   __shared__ double red[kHdThreads / 32][4];
@@ -3485,14 +3548,15 @@ static void launch_spline_fit(const MixedDev& M, int64_t B, cudaStream_t st_phas
     return;
   }
   const unsigned bp = (unsigned)ceil_div(nsd, (int64_t)kFitWarps);
-  const unsigned bt = (unsigned)ceil_div(nsd * 6, (int64_t)kFitWarps);
   if (seg == 32) {
     k_spline_fit<32, FF><<<bp, kFitWarps * 32, fit_smem_bytes<FF, true, 32>(M.J), st_phase>>>(M, nsd);
-    k_spline_fit<32, float><<<bt, kFitWarps * 32, fit_smem_bytes<float, true, 32>(M.J), st_transfer>>>(M, nsd * 6);
+    constexpr int systems = kFitSystems<float, true>;
+    k_spline_fit<32, float><<<(unsigned)ceil_div(nsd * 6, (int64_t)systems), systems * 32,
+                              fit_smem_bytes<float, true, 32>(M.J), st_transfer>>>(M, nsd * 6);
   } else {
     k_spline_fit<kSegMax, FF><<<bp, kFitWarps * 32, fit_smem_bytes<FF, false, kSegMax>(M.J), st_phase>>>(M, nsd);
-    k_spline_fit<kSegMax, float><<<bt, kFitWarps * 32, fit_smem_bytes<float, false, kSegMax>(M.J), st_transfer>>>(M,
-                                                                                                       nsd * 6);
+    k_spline_fit<kSegMax, float><<<(unsigned)ceil_div(nsd * 6, (int64_t)kFitWarps), kFitWarps * 32,
+                                   fit_smem_bytes<float, false, kSegMax>(M.J), st_transfer>>>(M, nsd * 6);
   }
 }
 
@@ -3519,6 +3583,7 @@ int mixed_create(PesPlan* p) {
     int sms = 0, per = 0;
     PES_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device));
     PES_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_exact<3, double>, kExactThreads, 0));
+    mb->sms = sms;
     mb->exact_grid = (int64_t)sms * std::max(per, 1);
     if (p->desc.approximant == PES_APPROX_PHENOMHM)
       PES_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_dense_ff<kHMModes>, kMixThreads, 0));
@@ -3624,6 +3689,7 @@ int mixed_create(PesPlan* p) {
   FF *wmom, *wtot;
   double *dsuf, *wrow, *hdv, *rpart, *fpart;
   int32_t *rkind, *rcount, *rlist;
+  float4* trig;
   float4* xff;
   float* cgb;
   float2* mid_ff;
@@ -3660,7 +3726,7 @@ int mixed_create(PesPlan* p) {
       (rc = alloc(mb, &mid_ff, J)) || (rc = alloc(mb, &tdm_ff, (size_t)nd * J)) || (rc = alloc(mb, &ymv, sd * 7 * J)) ||
       (rc = alloc(mb, &cbump, sd * J * 2)) || (rc = alloc(mb, &wspk, (size_t)nd * J)) ||
       (rc = alloc(mb, &rpart, (size_t)B * M.rblocks)) || (rc = alloc(mb, &rkind, (size_t)B)) ||
-      (rc = alloc(mb, &rcount, 2)) || (rc = alloc(mb, &rlist, (size_t)2 * B)) ||
+      (rc = alloc(mb, &rcount, 2)) || (rc = alloc(mb, &trig, kFfTrig)) || (rc = alloc(mb, &rlist, (size_t)2 * B)) ||
       (rc = alloc(mb, &fpart, (size_t)B * M.nblk_ff)) || (rc = alloc(mb, &xff, (size_t)nd * 6 * n)) ||
       (rc = alloc(mb, &gpart, gsd * M.nblk_sparse * 11)) || (rc = alloc(mb, &gdir, gsd)) ||
       (rc = alloc(mb, &gblk, (size_t)B)) || (rc = alloc(mb, &kR, sd * 6)) || (rc = alloc(mb, &kC, sd * 6)) ||
@@ -3806,6 +3872,10 @@ int mixed_create(PesPlan* p) {
   PES_CHECK_CUDA(cudaMemset(wspk, 0, sizeof(int32_t) * nd * J));
   M.rpart = rpart;
   M.rcount = rcount;
+  M.trig_ff = trig;
+  k_trig_ff<<<1, kFfTrig>>>(trig);
+  PES_CHECK_LAUNCH();
+  PES_CHECK_CUDA(cudaStreamSynchronize(nullptr));
   M.rlist = rlist;
   M.list_cap = (int32_t)B;
   M.refine_all = 0;
@@ -4126,7 +4196,10 @@ int mixed_lnl(PesPlan* p, const double* theta, int64_t B, double* lnl, double* g
     // <h|h> and <d|d> of the dense ranges (per mode), beside the anchors and the dense stage
     PES_CHECK_CUDA(cudaStreamWaitEvent(aux, p->mixed->xready, 0));
     ProfScope ps(p, kKOther, aux);
-    k_hd<<<(unsigned)(V * M.n_det), kHdThreads, 0, aux>>>(p->dev, M, blocks, B);
+    if (V * M.n_det <= p->mixed->sms)
+      k_hd<512><<<(unsigned)(V * M.n_det), 512, 0, aux>>>(p->dev, M, blocks, B);
+    else
+      k_hd<128><<<(unsigned)(V * M.n_det), 128, 0, aux>>>(p->dev, M, blocks, B);
   }
   PES_CHECK_LAUNCH();
   PES_CHECK_CUDA(cudaEventRecord(p->mixed->ev_hd, p->mixed->aux));
