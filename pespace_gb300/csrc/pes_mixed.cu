@@ -3178,17 +3178,21 @@ __device__ __forceinline__ FF hd_piece(const FF (&A)[6], const FF (&Bc)[6], cons
 #pragma unroll
   for (int ch = 0; ch < 3; ++ch) {
     const int r = 2 * ch, i = 2 * ch + 1;
-    const FF g0 = A[r] * A[r] + A[i] * A[i];
-    const FF g1 = ff_mulf(A[r] * Bc[r] + A[i] * Bc[i], 2.0f);
-    const FF g2 = (Bc[r] * Bc[r] + Bc[i] * Bc[i]) + ff_mulf(A[r] * Cc[r] + A[i] * Cc[i], 2.0f);
-    const FF g3 = ff_mulf((A[r] * Dc[r] + A[i] * Dc[i]) + (Bc[r] * Cc[r] + Bc[i] * Cc[i]), 2.0f);
-    const FF g4 = (Cc[r] * Cc[r] + Cc[i] * Cc[i]) + ff_mulf(Bc[r] * Dc[r] + Bc[i] * Dc[i], 2.0f);
-    const FF g5 = ff_mulf(Cc[r] * Dc[r] + Cc[i] * Dc[i], 2.0f);
-    const FF g6 = Dc[r] * Dc[r] + Dc[i] * Dc[i];
+    auto dot = [&](const FF (&x)[6], const FF (&y)[6]) { return ff_dot2(x[r], y[r], x[i], y[i]); };
+    auto twice = [](const FF& x) { return ff_make(2.0f * x.hi, 2.0f * x.lo); };
+    const FF g2 = ff_add_lazy(dot(Bc, Bc), twice(dot(A, Cc)));
+    const FF g3 = twice(ff_add_lazy(dot(A, Dc), dot(Bc, Cc)));
+    const FF g4 = ff_add_lazy(dot(Cc, Cc), twice(dot(Bc, Dc)));
     const FF* m = Sm + ch * 7;
-    acc = acc + ((g0 * m[0] + g1 * m[1]) + (g2 * m[2] + g3 * m[3]) + (g4 * m[4] + (g5 * m[5] + g6 * m[6])));
+    acc = ff_mad(dot(Dc, Dc), m[6], acc);
+    acc = ff_mad(twice(dot(Cc, Dc)), m[5], acc);
+    acc = ff_mad(g4, m[4], acc);
+    acc = ff_mad(g3, m[3], acc);
+    acc = ff_mad(g2, m[2], acc);
+    acc = ff_mad(twice(dot(A, Bc)), m[1], acc);
+    acc = ff_mad(dot(A, A), m[0], acc);
   }
-  return acc;
+  return ff_fast_two_sum(acc.hi, acc.lo);
 }
 
 template <int kHdThreads>
@@ -3251,6 +3255,9 @@ __global__ void __launch_bounds__(kHdThreads) k_hd(PlanDev P, MixedDev M,
     if (k1 >= k2) continue;
     const FF* tot = M.wtot + ((size_t)d * M.J + j) * kMomStride;
     auto F = [&](int64_t k, int idx) { return k >= e2 ? tot[idx] : wm[(size_t)k * kMomStride + idx]; };
+    // the moments start from 0 at the interval's first bin: all intervals but the range's first
+    const bool whole = k1 == e1;
+    auto from_start = [&](int64_t k, int idx) { return whole ? F(k, idx) : F(k, idx) - F(k1, idx); };
     // the spline coefficients in the interval's own variable u = t / h (the
     // moments are sums of u^p W): A, B h, C h^2, D h^3
     const FF h = M.gff[j], h2 = h * h, h3 = h2 * h;
@@ -3288,7 +3295,7 @@ __global__ void __launch_bounds__(kHdThreads) k_hd(PlanDev P, MixedDev M,
     const int64_t ks = folded ? k2 : min(max(kpk, k1), k2);
     if (ks > k1) {
 #pragma unroll
-      for (int x = 0; x < 21; ++x) Sm[x] = F(ks, x) - F(k1, x);
+      for (int x = 0; x < 21; ++x) Sm[x] = from_start(ks, x);
       sum = sum + hd_piece(A, Bc, Cc, Dc, Sm);
     }
     if (ks < k2) {
@@ -3302,7 +3309,7 @@ __global__ void __launch_bounds__(kHdThreads) k_hd(PlanDev P, MixedDev M,
         C2[q] = Cc[q] + KC[q] * K2;
       }
 #pragma unroll
-      for (int x = 0; x < 21; ++x) Sm[x] = F(k2, x) - F(ks, x);
+      for (int x = 0; x < 21; ++x) Sm[x] = ks == k1 ? from_start(k2, x) : F(k2, x) - F(ks, x);
       sum = sum + hd_piece(A2, B2, C2, Dc, Sm);
     }
     // first-order change of sum |h|^2 w over the interval if the splines' error
@@ -3311,8 +3318,8 @@ __global__ void __launch_bounds__(kHdThreads) k_hd(PlanDev P, MixedDev M,
       float e = 0.0f;
 #pragma unroll
       for (int ch = 0; ch < 3; ++ch) {
-        const float m2 = (F(k2, ch * 7 + 2) - F(k1, ch * 7 + 2)).hi, m3 = (F(k2, ch * 7 + 3) - F(k1, ch * 7 + 3)).hi,
-                    m4 = (F(k2, ch * 7 + 4) - F(k1, ch * 7 + 4)).hi;
+        const float m2 = from_start(k2, ch * 7 + 2).hi, m3 = from_start(k2, ch * 7 + 3).hi,
+                    m4 = from_start(k2, ch * 7 + 4).hi;
         const float bump = 16.0f * (m2 - 2.0f * m3 + m4);
         e += 2.0f * (gm[2 * ch] * delta[2 * ch] + gm[2 * ch + 1] * delta[2 * ch + 1]) * bump;
       }
