@@ -168,18 +168,21 @@ __global__ void k_fisher_final(const SampleBlock<FisherScalar>* __restrict__ blo
 // The response per unit amplitude takes FP32 duals over (T, lambda, sin beta,
 // psi, cos iota); ln D_L and phi_c are analytic (dh = -h and 2 i h).
 //
-// Four warps of a block evaluate 128 bins of one detector and store sqrt(w)
-// times the 11 complex derivatives in shared memory; the fifth sums the 66
-// pairs over the previous 128 (two buffers; FP32 within the 128 bins in their
+// Four warps evaluate 128 bins of one detector and store sqrt(w) times the 11
+// complex derivatives in shared memory; a fifth sums the 66 pairs over the
+// previous 128 (two buffers; FP32 within the 128 bins in their
 // order, FP64 across).  A lane takes up to three pairs of one row, so that it
 // loads 4 complex numbers for 6 products (a thread per pair loaded 12 values for
 // 6, three of four warps waiting).  Float-float dual numbers through the
 // waveform, and FP64 square roots and conversions of the weights per bin, took
-// most of the time before: 100 samples on 125 410 bins 5.21 -> 2.04 ms (1.97 ms of it
-// here, 5 200 FP32 operations per bin and detector, two thirds in the response).
-constexpr int kFastThreads = 128;              // bins per group
-constexpr int kFastBlock = kFastThreads + 32;  // and the summing warp
-constexpr int kFastBlocks = 152 * 2;           // small calls: blocks of the whole call
+// most of the time before: 100 samples on 125 410 bins 5.21 -> 2.04 ms, and 1.88 ms with
+// two groups of 128 bins per block, whose warps fetch the same code (5 200 FP32
+// operations per bin and detector, two thirds in the response).
+constexpr int kFastThreads = 128;  // bins per group
+constexpr int kFastGroups = 2;     // groups per block
+constexpr int kFastBins = kFastThreads * kFastGroups;
+constexpr int kFastBlock = kFastBins + 32 * kFastGroups;  // and a summing warp per group
+constexpr int kFastRows = 152 * kFastGroups;              // small calls: partial sums of the whole call
 using FR = DualS<5>;                           // T, lambda, sin beta, psi, cos iota
 
 // Per bin, for the FP32 frequency that the response takes too: f, f^{1/3} | 1/f,
@@ -520,10 +523,10 @@ __device__ __forceinline__ void pairs_of(int lane, int& a, int& b, int& count) {
   a = b = count = 0;
 }
 
-constexpr size_t fisher_smem() { return 2 * sizeof(float2) * kFastThreads * 3 * 11; }
+constexpr size_t fisher_smem() { return 2 * sizeof(float2) * kFastBins * 3 * 11; }
 
-// grid (blocks, B), grid-stride over the groups of 128 live bins.
-__global__ void __launch_bounds__(kFastBlock, 2) k_fisher_fast(PlanDev P, const FisherSample* __restrict__ samples,
+// grid (blocks, B), grid-stride over pairs of groups of 128 live bins.
+__global__ void __launch_bounds__(kFastBlock, 1) k_fisher_fast(PlanDev P, const FisherSample* __restrict__ samples,
                                                                const float4* __restrict__ rows,
                                                                const float2* __restrict__ p76,
                                                                const float4* __restrict__ wt,
@@ -541,16 +544,17 @@ __global__ void __launch_bounds__(kFastBlock, 2) k_fisher_fast(PlanDev P, const 
   }
   __syncthreads();
   const int kcut = sb.status == kSampleOk ? sb.kcut : 0;
-  const bool summing = t >= kFastThreads;
+  const bool summing = t >= kFastBins;
+  const int grp = summing ? (t - kFastBins) >> 5 : t / kFastThreads;
   int pa = 0, pb = 0, np = 0;
-  if (summing) pairs_of(t - kFastThreads, pa, pb, np);
+  if (summing) pairs_of(t & 31, pa, pb, np);
   double acc[3] = {0.0, 0.0, 0.0};
   WaveTangents wv;
   int step = 0;  // (group, detector) pairs evaluated so far
-  const int first = blockIdx.x * kFastThreads, stride = gridDim.x * kFastThreads;
+  const int first = blockIdx.x * kFastBins, stride = gridDim.x * kFastBins;
   const int steps = first < kcut ? (kcut - first + stride - 1) / stride * P.n_det : 0;
   for (; step <= steps; ++step) {
-    float2* buf = dh_buf + (size_t)(step & 1) * (kFastThreads * 33);
+    float2* buf = dh_buf + (size_t)(step & 1) * (kFastBins * 33);
     if (!summing && step < steps) {
       const int d = step % P.n_det;
       const int i = first + step / P.n_det * stride + t;
@@ -608,7 +612,7 @@ __global__ void __launch_bounds__(kFastBlock, 2) k_fisher_fast(PlanDev P, const 
       }
     }
     if (summing && step > 0) {
-      const float2* src = dh_buf + (size_t)((step & 1) ^ 1) * (kFastThreads * 33);
+      const float2* src = dh_buf + (size_t)((step & 1) ^ 1) * (kFastBins * 33) + grp * (kFastThreads * 33);
       float x[3] = {0.0f, 0.0f, 0.0f};
       const int b1 = min(pb + 1, 10), b2 = min(pb + 2, 10);
 #pragma unroll 4
@@ -626,7 +630,7 @@ __global__ void __launch_bounds__(kFastBlock, 2) k_fisher_fast(PlanDev P, const 
   }
   if (summing)
     for (int k = 0; k < np; ++k)
-      partial[((size_t)s * gridDim.x + blockIdx.x) * kPairs + (pa * 11 - pa * (pa - 1) / 2 + (pb + k - pa))] = acc[k];
+      partial[((size_t)s * gridDim.x * kFastGroups + blockIdx.x * kFastGroups + grp) * kPairs + (pa * 11 - pa * (pa - 1) / 2 + (pb + k - pa))] = acc[k];
 }
 
 }  // namespace pes
@@ -645,12 +649,13 @@ extern "C" int pes_fisher_batch(PesPlan* p, const double* theta, int64_t B, doub
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool hm = p->desc.approximant == PES_APPROX_PHENOMHM, fast = p->mixed && !hm;
   const int64_t M = p->desc.max_batch, n = p->desc.nbins, nd = p->desc.n_det;
-  // blocks per sample: kFisherBlocks, more in calls that would leave SMs idle
-  const int64_t nblk = !fast ? (int64_t)kFisherBlocks
+  // partial sums per sample: kFisherBlocks, more in calls that would leave SMs idle
+  const int64_t nrow = !fast ? (int64_t)kFisherBlocks
                              : std::min<int64_t>(ceil_div(n, kFastThreads),
-                                                 std::max<int64_t>(kFisherBlocks, ceil_div(kFastBlocks, B)));
+                                                 std::max<int64_t>(kFisherBlocks, ceil_div(kFastRows, B)));
+  const int64_t nblk = !fast ? nrow : ceil_div(nrow, kFastGroups) * (int64_t)kFastGroups;
   if (!p->fisher_blocks) {
-    const int64_t rows = std::max<int64_t>(M * kFisherBlocks, kFastBlocks + M);
+    const int64_t rows = std::max<int64_t>(M * kFisherBlocks, kFastRows + M * (int64_t)kFastGroups);
     PES_CHECK_CUDA(cudaMalloc(&p->fisher_partial, sizeof(double) * rows * kPairs));
     if (fast) {
       PES_CHECK_CUDA(cudaMalloc(&p->fisher_samples, sizeof(FisherSample) * M));
@@ -659,6 +664,7 @@ extern "C" int pes_fisher_batch(PesPlan* p, const double* theta, int64_t B, doub
       PES_CHECK_CUDA(cudaFuncSetAttribute(k_fisher_fast, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fisher_smem()));
       k_fisher_grid<<<ceil_div(n, 128), 128, 0, st>>>(p->dev, p->fisher_rows, p->fisher_p76);
       PES_CHECK_LAUNCH();
+      PES_CHECK_CUDA(cudaStreamSynchronize(st));  // later calls may come on another stream
     }
     PES_CHECK_CUDA(cudaMalloc(&p->fisher_blocks, sizeof(SampleBlock<FisherScalar>) * M));
   }
@@ -674,7 +680,7 @@ extern "C" int pes_fisher_batch(PesPlan* p, const double* theta, int64_t B, doub
     PES_CHECK_LAUNCH();
     k_fisher_prep<<<(unsigned)B, 64, 0, st>>>(scale, blocks, samples);
     PES_CHECK_LAUNCH();
-    k_fisher_fast<<<dim3((unsigned)nblk, (unsigned)B), kFastBlock, fisher_smem(), st>>>(
+    k_fisher_fast<<<dim3((unsigned)(nblk / kFastGroups), (unsigned)B), kFastBlock, fisher_smem(), st>>>(
         p->dev, samples, p->fisher_rows, p->fisher_p76, wt, p->fisher_partial);
   } else {  // FP64 plans and IMRPhenomHM: FP64 dual numbers through the whole model
     k_fisher_bins<<<dim3(kFisherBlocks, (unsigned)B), kFisherThreads, 0, st>>>(

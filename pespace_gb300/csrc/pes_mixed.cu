@@ -43,7 +43,14 @@ constexpr int kNodeQ = 7;         // Phi_s, Re/Im G_A, G_E, G_T
 constexpr int kChunkMax = 32;     // bins per phase-anchored run (one warp)
 constexpr int kMixThreads = 128;  // 4 warps; each warp owns 32 consecutive runs
 constexpr int kMoments = 4;       // t^0..t^3
-constexpr int kSparseThreads = 128;
+// Blocks of the node stage's forward and backward passes: all the warps that an SM
+// holds at their registers in one block.  A node evaluation is about 100 KB of
+// straight-line code, and instruction fetch is its top stall; the warps of one block
+// start together and share what they fetch (blocks of 128: lnL of 1024 prior draws
+// 2.75 ms, with the gradient 3.95 ms; so 2.65 and 3.83 ms.  Loops rolled around arrays in
+// local memory, or only the Horner sums, were slower: 2.83 and 2.93 ms).
+constexpr int kSparseThreads = 512;
+constexpr int kBwdThreads = 384;
 // FP32 copies of the shared grid's spline factors, [kGfCount][J]: h, 1/h, lo, up, 1/den, cp.
 enum { kGfH = 0, kGfInvH, kGfLo, kGfUp, kGfInvDen, kGfCp, kGfCount };
 // Gradient: one pass with FP64 values and FP32 tangents for the 9 parameters
@@ -54,6 +61,12 @@ constexpr double kOrbitPhaseMax = 0.3;  // rad of yearly orbital phase per node 
 constexpr int kExactBlocks = 4;         // blocks per sample of the exact-bin kernel (heliocentric plans)
 constexpr int kExactBlocksGeo = 64;     // with a geocentric detector most inspiral bins are exact
 constexpr int kExactThreads = 128;
+// Threads of the exact re-evaluation and of six-mode plans' exact bins: as many warps
+// per SM as with three blocks of 128, but one block's, which fetch the model's long
+// straight-line code together and narrow one copy of the modes' coefficients (lnL of 12
+// six-mode samples on the network 3.34 -> 3.16 ms; the few exact bins of one mode were
+// slower so: lnL and gradient of 24 samples 1.19 -> 1.22 ms).
+constexpr int kExactWide = 384;
 __device__ __constant__ static const int kSlotParam[kMixNT] = {0, 1, 2, 3, 5, 6, 7, 8, 10};
 using GradScalar = DualF<kMixNT>;    // exact bins: FP64 values (phases of 1e6 rad), FP32 tangents
 
@@ -76,7 +89,7 @@ struct MixedDev {
   int32_t nchunks;
   int32_t n_det;
   int32_t nblk_dense;
-  int32_t nblk_sparse;
+  int32_t nblk_sparse, nblk_bwd;
   int32_t pad;
   double scale;             // FP32 storage scale of data and model
   const double* node_f;     // [J]
@@ -133,7 +146,7 @@ struct MixedDev {
   double* part;             // [B][nblk_dense][kPartW] partials: sum |d - h|^2 w (direct form), sum -2 Re(d^* h) w,
                             //   sum 2 Re sum_{k<l} h_k conj(h_l) w (the modes' cross terms; 0 for one mode),
                             //   the rounding estimate (k_refine_select)
-  double* gpart;            // [B][n_det][nblk_sparse][11] gradient partials
+  double* gpart;            // [B][n_det][nblk_bwd][11] gradient partials
   void* gblocks;            // [B] SampleBlock<GradScalar>
   double* gdir;             // [B][n_det] direct t_c term of the gradient
   // Amplitude kink at f_peak: the transfer quantities carry C_q max(0, Mf - Mf_peak)^2
@@ -662,10 +675,10 @@ struct BwdBlock {
   int status;
 };
 
-__global__ void __launch_bounds__(kSparseThreads, 3) k_sparse_bwd_split(PlanDev P, MixedDev M, GenArg G,
+__global__ void __launch_bounds__(kBwdThreads, 1) k_sparse_bwd_split(PlanDev P, MixedDev M, GenArg G,
                                                                       double wscale) {
   __shared__ BwdBlock sb;
-  __shared__ float2 red[kSparseThreads / 32][11];  // per warp: float-float partial sums
+  __shared__ float2 red[kBwdThreads / 32][11];  // per warp: float-float partial sums
   __shared__ double kadd[6][5];                     // dense-side kink terms, added in order to warp 0's sums
   __shared__ int kink_on;
   __shared__ float kR[6];  // the kink coefficients R_q held fixed, narrowed once
@@ -829,13 +842,13 @@ __global__ void __launch_bounds__(kSparseThreads, 3) k_sparse_bwd_split(PlanDev 
     const int k = threadIdx.x;
     double x = 0.0;
 #pragma unroll
-    for (int w = 0; w < kSparseThreads / 32; ++w) {
+    for (int w = 0; w < kBwdThreads / 32; ++w) {
       double v = (double)red[w][k].x + (double)red[w][k].y;
       if (w == 0 && kink_on && k < 5)
         for (int q = 0; q < 6; ++q) v += kadd[q][k];
       x += v;
     }
-    M.gpart[(((size_t)s * M.n_det + d) * M.nblk_sparse + blockIdx.x) * 11 + k] = x;
+    M.gpart[(((size_t)s * M.n_det + d) * M.nblk_bwd + blockIdx.x) * 11 + k] = x;
   }
 }
 
@@ -1929,8 +1942,8 @@ __global__ void __launch_bounds__(kSampleWarps * 32) k_refine_select(PlanDev P, 
 // the parts of the listed samples; threads stride over the bins.  The
 // value passes are held to 168 registers (3 blocks per SM instead of 2: the
 // bench step 1.5% faster).
-template <int kMode, class T>
-__global__ void __launch_bounds__(kExactThreads, kMode == 1 ? 1 : 3) k_exact(PlanDev P, MixedDev M, GenArg G,
+template <int kMode, class T, int kT>
+__global__ void __launch_bounds__(kT, kMode == 1 || kT == kExactWide ? 1 : 3) k_exact(PlanDev P, MixedDev M, GenArg G,
                                                          const SampleBlock<T>* __restrict__ blocks,
                                                          double2* __restrict__ model) {
   constexpr bool kGradPass = kMode == 1;
@@ -1943,7 +1956,7 @@ __global__ void __launch_bounds__(kExactThreads, kMode == 1 ? 1 : 3) k_exact(Pla
   using SBF = std::conditional_t<kGradPass, ExactGradBlock, SampleBlock<FF>>;
   __shared__ SampleBlock<T> sb;
   __shared__ SBF sbf;
-  __shared__ double red[kExactThreads / 32][NV];
+  __shared__ double red[kT / 32][NV];
   __shared__ PhenomHMCoef<double> hmd;  // multi-mode plans (value passes)
   __shared__ PhenomHMCoef<FF> hmf;
   const int nm = M.n_modes;
@@ -1957,7 +1970,7 @@ __global__ void __launch_bounds__(kExactThreads, kMode == 1 ? 1 : 3) k_exact(Pla
     int most = 0;
     for (int d = 0; d < M.n_det; ++d)
       most = max(most, (int)blocks[s].kcut - M.xbind[(size_t)s * nm * M.n_det + d]);
-    if (part * kExactThreads >= most) {  // no bins in this part (uniform)
+    if (part * kT >= most) {  // no bins in this part (uniform)
       if (threadIdx.x == 0) M.rpart[(size_t)s * parts + part] = 0.0;
       continue;
     }
@@ -1982,7 +1995,7 @@ __global__ void __launch_bounds__(kExactThreads, kMode == 1 ? 1 : 3) k_exact(Pla
       const int xbd = M.xbind[(size_t)s * nm * M.n_det + d];
       const int i0 = kRefine ? xbd : 0, i1 = kRefine ? (int)sb.kcut : xbd;
       const int n_it = kZero ? M.nzb[d] : i1 - i0;
-      for (int it = part * kExactThreads + threadIdx.x; it < n_it; it += parts * kExactThreads) {
+      for (int it = part * kT + threadIdx.x; it < n_it; it += parts * kT) {
         int i = i0 + it;
         if constexpr (kZero) {
           i = M.zbin[(size_t)d * kZeroMax + it];
@@ -2113,7 +2126,7 @@ __global__ void __launch_bounds__(kExactThreads, kMode == 1 ? 1 : 3) k_exact(Pla
   if (threadIdx.x < NV) {
     double x = 0.0;
 #pragma unroll
-    for (int w = 0; w < kExactThreads / 32; ++w) x += red[w][threadIdx.x];
+    for (int w = 0; w < kT / 32; ++w) x += red[w][threadIdx.x];
     if (kMode == 0)
       M.xpart[(size_t)s * parts + part] = x;
     else if (kMode == 3)
@@ -3424,7 +3437,7 @@ __global__ void __launch_bounds__(kSampleWarps * 32) k_mixed_grad_finalize(Mixed
   const int p = (int)(t % 11);
   double acc = 0.0, x = 0.0;
   if (reinterpret_cast<const SampleBlock<GradScalar>*>(M.gblocks)[s].status == kSampleOk) {
-    const int nb = M.n_det * M.nblk_sparse;
+    const int nb = M.n_det * M.nblk_bwd;
     for (int b = lane; b < nb; b += 32) acc += M.gpart[((size_t)s * nb + b) * 11 + p];
     if (p == 10 && lane < M.n_det) acc += M.gdir[(size_t)s * M.n_det + lane];
     if (M.xbin[s] > 0)
@@ -3589,7 +3602,7 @@ int mixed_create(PesPlan* p) {
   {
     int sms = 0, per = 0;
     PES_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device));
-    PES_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_exact<3, double>, kExactThreads, 0));
+    PES_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_exact<3, double, kExactWide>, kExactWide, 0));
     mb->sms = sms;
     mb->exact_grid = (int64_t)sms * std::max(per, 1);
     if (p->desc.approximant == PES_APPROX_PHENOMHM)
@@ -3671,7 +3684,7 @@ int mixed_create(PesPlan* p) {
     M.omega[k] = std::fabs(d.det[k].orbit.omega_revolution);
     if (d.det[k].orbit.kind == 1) {
       M.omega[k] = std::max(M.omega[k], std::fabs(d.det[k].orbit.omega_rotation));
-      M.xblocks = kExactBlocksGeo;
+      M.xblocks = p->desc.approximant == PES_APPROX_PHENOMHM ? kExactBlocksGeo / 2 : kExactBlocksGeo;
     }
   }
   M.nchunks = (int32_t)cb.size();
@@ -3679,6 +3692,7 @@ int mixed_create(PesPlan* p) {
   M.nblk_ff = (int32_t)ceil_div(M.nchunks, (long long)kChunkMax);
   M.rblocks = (int32_t)std::min<int64_t>(kRefinePartsMax, std::max<int64_t>(kRefinePartsMin, n / kRefineBins));
   M.nblk_sparse = (int32_t)ceil_div(J, kSparseThreads);
+  M.nblk_bwd = (int32_t)ceil_div(J, kBwdThreads);
   int rc = PES_OK;
   double *node_f = nullptr, *scr, *part, *gpart, *gdir;
   float* ybar;
@@ -3735,7 +3749,7 @@ int mixed_create(PesPlan* p) {
       (rc = alloc(mb, &rpart, (size_t)B * M.rblocks)) || (rc = alloc(mb, &rkind, (size_t)B)) ||
       (rc = alloc(mb, &rcount, 2)) || (rc = alloc(mb, &trig, kFfTrig)) || (rc = alloc(mb, &rlist, (size_t)2 * B)) ||
       (rc = alloc(mb, &fpart, (size_t)B * M.nblk_ff)) || (rc = alloc(mb, &xff, (size_t)nd * 6 * n)) ||
-      (rc = alloc(mb, &gpart, gsd * M.nblk_sparse * 11)) || (rc = alloc(mb, &gdir, gsd)) ||
+      (rc = alloc(mb, &gpart, gsd * M.nblk_bwd * 11)) || (rc = alloc(mb, &gdir, gsd)) ||
       (rc = alloc(mb, &gblk, (size_t)B)) || (rc = alloc(mb, &kR, sd * 6)) || (rc = alloc(mb, &kC, sd * 6)) ||
       (rc = alloc(mb, &kF, sd * 16)) || (rc = alloc(mb, &kM, gsd * 12)) || (rc = alloc(mb, &xbin, V)) || (rc = alloc(mb, &xbind, sd)) ||
       (rc = alloc(mb, &ivfirst, J + 1)) || (rc = alloc(mb, &xpart, (size_t)B * M.xblocks)) ||
@@ -4061,7 +4075,7 @@ int mixed_model(PesPlan* p, const double* theta_dev, double* out, cudaStream_t s
     k_dense_mixed<2, false, 1><<<dim3(M.nblk_dense, 1), kMixThreads, 0, st>>>(p->dev, M, blocks,
                                                                      reinterpret_cast<double2*>(out));
   PES_CHECK_LAUNCH();
-  k_exact<2, double><<<dim3(M.xblocks, 1), kExactThreads, 0, st>>>(p->dev, M, G, blocks,
+  k_exact<2, double, kExactThreads><<<dim3(M.xblocks, 1), kExactThreads, 0, st>>>(p->dev, M, G, blocks,
                                                                       reinterpret_cast<double2*>(out));
   PES_CHECK_LAUNCH();
   return PES_OK;
@@ -4125,12 +4139,16 @@ int mixed_lnl(PesPlan* p, const double* theta, int64_t B, double* lnl, double* g
   PES_CHECK_CUDA(cudaEventRecord(p->mixed->xready, side));
   {
     ProfScope ps(p, kKDenseFp64, side);
-    k_exact<0, double><<<dim3(M.xblocks, (unsigned)B), kExactThreads, 0, side>>>(p->dev, M, G, blocks, nullptr);
+    if (multi)
+      k_exact<0, double, kExactWide><<<dim3(M.xblocks, (unsigned)B), kExactWide, 0, side>>>(p->dev, M, G, blocks, nullptr);
+    else
+      k_exact<0, double, kExactThreads><<<dim3(M.xblocks, (unsigned)B), kExactThreads, 0, side>>>(p->dev, M, G, blocks,
+                                                                                               nullptr);
   }
   PES_CHECK_LAUNCH();
   if (M.zblocks > 0) {
     ProfScope ps(p, kKDenseFp64, side);
-    k_exact<4, double><<<dim3(M.zblocks, (unsigned)B), kExactThreads, 0, side>>>(p->dev, M, G, blocks, nullptr);
+    k_exact<4, double, kExactThreads><<<dim3(M.zblocks, (unsigned)B), kExactThreads, 0, side>>>(p->dev, M, G, blocks, nullptr);
   }
   PES_CHECK_LAUNCH();
   if (grad) {
@@ -4145,7 +4163,7 @@ int mixed_lnl(PesPlan* p, const double* theta, int64_t B, double* lnl, double* g
     PES_CHECK_LAUNCH();
     {
       ProfScope ps(p, kKDenseFp64, side);
-      k_exact<1, GradScalar><<<dim3(M.xblocks, (unsigned)B), kExactThreads, 0, side>>>(
+      k_exact<1, GradScalar, kExactThreads><<<dim3(M.xblocks, (unsigned)B), kExactThreads, 0, side>>>(
           p->dev, M, G, reinterpret_cast<const SampleBlock<GradScalar>*>(M.gblocks), nullptr);
     }
     PES_CHECK_LAUNCH();
@@ -4223,7 +4241,7 @@ int mixed_lnl(PesPlan* p, const double* theta, int64_t B, double* lnl, double* g
     PES_CHECK_LAUNCH();
     {
       ProfScope ps(p, kKDenseFp64, side);
-      k_exact<3, double><<<(unsigned)std::min<int64_t>(p->mixed->exact_grid, B * M.rblocks), kExactThreads, 0, side>>>(
+      k_exact<3, double, kExactWide><<<(unsigned)std::min<int64_t>(p->mixed->exact_grid, B * M.rblocks), kExactWide, 0, side>>>(
           p->dev, M, G, blocks, nullptr);
     }
     PES_CHECK_LAUNCH();
@@ -4289,7 +4307,7 @@ int mixed_lnl(PesPlan* p, const double* theta, int64_t B, double* lnl, double* g
   // node adjoints: phase systems here, transfer systems on the second stream;
   // then the backward node stage
   const double ws = 4.0 * p->dev.df;
-  const dim3 sgrid(M.nblk_sparse, M.n_det, (unsigned)B);
+  const dim3 sgrid(M.nblk_bwd, M.n_det, (unsigned)B);
   if (spline_seg(M.J) == 32) {
     const int64_t nsd = B * M.n_det;
     {
@@ -4318,7 +4336,7 @@ int mixed_lnl(PesPlan* p, const double* theta, int64_t B, double* lnl, double* g
   PES_CHECK_CUDA(cudaStreamWaitEvent(st, p->mixed->ev_xgrad, 0));
   {
     ProfScope ps(p, kKAdjoint, st);
-    k_sparse_bwd_split<<<sgrid, kSparseThreads, 0, st>>>(p->dev, M, G, ws);
+    k_sparse_bwd_split<<<sgrid, kBwdThreads, 0, st>>>(p->dev, M, G, ws);
   }
   PES_CHECK_LAUNCH();
   {
