@@ -47,8 +47,9 @@ constexpr int k64BinsPerThread = 4;
 constexpr int k64SmallBlocks = 152 * 4 * 2;
 
 // ------------------------------------------------------------------ tables
-// Per bin, seven rows of nbins: f, f^{1/3}, f^{-1/3}, ln(f)/3, 1/f, f^{-1/4}, f^{-7/6}.
-enum { kGf, kGu, kGiu, kGlf3, kGif, kGq, kGp76, kGridRows };
+// Per bin, seven rows of nbins: f, f^{1/3}, f^{-5/3} (rounded once: the phase's leading
+// terms multiply its error by 1e5), ln(f)/3, 1/f, f^{-1/4}, f^{-7/6}.
+enum { kGf, kGu, kGiu5, kGlf3, kGif, kGq, kGp76, kGridRows };
 __global__ void k_grid64(PlanDev P, double* __restrict__ grid, double2* __restrict__ trig) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i < kTrig) {
@@ -61,7 +62,10 @@ __global__ void k_grid64(PlanDev P, double* __restrict__ grid, double2* __restri
   const double u = cbrt(f);
   grid[kGf * P.nbins + i] = f;
   grid[kGu * P.nbins + i] = u;
-  grid[kGiu * P.nbins + i] = 1.0 / u;
+  {
+    const DD c = dd_cbrt({f, 0.0});
+    grid[kGiu5 * P.nbins + i] = dd_div(c, dd_mul({f, 0.0}, {f, 0.0})).h;
+  }
   grid[kGlf3 * P.nbins + i] = log(f) / 3.0;
   grid[kGif * P.nbins + i] = 1.0 / f;
   grid[kGq * P.nbins + i] = 1.0 / sqrt(sqrt(f));
@@ -79,6 +83,8 @@ struct Dense64Block {
   int32_t status;
   int32_t pad;
 };
+
+constexpr int kLeadTerms = 5;  // pin[0..4], the first scalars of FreqCoef (pin[1] = 0)
 
 // The set-up of one sample per block (grid B): warps 0 and 1 the two parts of
 // the coefficient block (phenomd_setup) and then of its rescaled form, a warp per
@@ -119,7 +125,19 @@ k_setup64(PlanDev P, const double* __restrict__ theta, SampleBlock<double>* __re
     response_tables(P, th, wid - 2, lane, v[wid - 2], w9, resp[(size_t)s * P.n_det + wid - 2]);
   }
   __syncthreads();
-  if (lane != 0 || wid > 1) return;
+  if (lane != 0 || wid > 2) return;
+  if (wid == 2) {
+    // the leading phase terms' coefficients, rounded once (their phases reach 1e5 rad), beside the others
+    const DD icu = dd_div({1.0, 0.0}, dd_cbrt({b.wf.Msec, 0.0})), icu2 = dd_mul(icu, icu), icu3 = dd_mul(icu2, icu);
+    const double lead[kLeadTerms] = {dd_mul(dd_mul(icu3, icu2), {b.wf.pin[0], 0.0}).h, 0.0, dd_mul(icu3, {b.wf.pin[2], 0.0}).h,
+                                     dd_mul(icu2, {b.wf.pin[3], 0.0}).h, dd_mul(icu, {b.wf.pin[4], 0.0}).h};
+#pragma unroll
+    for (int j = 0; j < kLeadTerms; ++j) {
+      o.c.pin[j] = lead[j];
+      o.rin[j] = lead[j] * ((j - 5) / (6.0 * kPi));
+    }
+    return;
+  }
   const double iM = 1.0 / b.wf.Msec;
   FreqCoef<double> c;
   if (wid == 0) {
@@ -127,9 +145,9 @@ k_setup64(PlanDev P, const double* __restrict__ theta, SampleBlock<double>* __re
     double* dst = reinterpret_cast<double*>(&o.c);
     const double* src = reinterpret_cast<const double*>(&c);
 #pragma unroll
-    for (int k = 0; k < (int)(offsetof(FreqCoef<double>, a0) / sizeof(double)); ++k) dst[k] = src[k];
+    for (int k = kLeadTerms; k < (int)(offsetof(FreqCoef<double>, a0) / sizeof(double)); ++k) dst[k] = src[k];
 #pragma unroll
-    for (int j = 0; j < 12; ++j) o.rin[j] = c.pin[j] * ((j - 5) / (6.0 * kPi));
+    for (int j = kLeadTerms; j < 12; ++j) o.rin[j] = c.pin[j] * ((j - 5) / (6.0 * kPi));
     o.ifd = 1.0 / c.fd;
     o.fd2 = c.fd * c.fd;
     o.fj1 = kPhiJoinIns * iM;
@@ -170,8 +188,7 @@ __device__ __forceinline__ double bin64(const PlanDev& P, const Dense64Block& b,
   const int preg = f < b.fj1 ? 0 : (f < b.fj2 ? 1 : 2);
   double psi, tf, at = 0.0, rden = 0.0, q14 = 0.0, x5 = 0.0;
   if (preg == 0) {
-    const double iu = grid[kGiu * n + i];
-    const double iu5 = iu * iu * jf;
+    const double iu5 = grid[kGiu5 * n + i];
     double p = c.pin[11], r = b.rin[11];
 #pragma unroll
     for (int j = 10; j >= 0; --j) {
@@ -440,9 +457,8 @@ __device__ __forceinline__ double bin64(const PlanDev& P, const Dense64Block& b,
 #define PES_W(field) W[offsetof(FreqCoef<double>, field) / sizeof(double)]
   const double g2 = RT * (1.0 / (2.0 * kPi));
   if (preg == 0) {
-    const double iu = grid[kGiu * n + i];
     const double g = (RT * (1.0 / (6.0 * kPi))) * jf;
-    double bj = iu * iu * jf;
+    double bj = grid[kGiu5 * n + i];
     double* wp = &PES_W(pin);
 #pragma unroll
     for (int j = 0; j < 12; ++j) {

@@ -111,6 +111,29 @@ __device__ __forceinline__ void fill_trig(double2* tab) {
   }
 }
 
+// Products and quotients of pairs hi + lo.
+struct DD {
+  double h, l;
+};
+PES_HD DD dd_two(double a, double b) {
+  const double s = a + b, t = s - a;
+  return {s, (a - (s - t)) + (b - t)};
+}
+PES_HD DD dd_mul(const DD& a, const DD& b) {
+  const double p = a.h * b.h;
+  return dd_two(p, ::fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h));
+}
+PES_HD DD dd_div(const DD& a, const DD& b) {
+  const double q = a.h / b.h;
+  const double p = q * b.h, e = ::fma(q, b.h, -p);
+  return dd_two(q, (((a.h - p) - e) + a.l - q * b.l) / b.h);
+}
+PES_HD DD dd_cbrt(const DD& a) {
+  const double c = ::cbrt(a.h);
+  const DD c3 = dd_mul(dd_mul({c, 0.0}, {c, 0.0}), {c, 0.0});
+  return dd_two(c, ((a.h - c3.h) + (a.l - c3.l)) / (3.0 * c * c));
+}
+
 // IMRPhenomD's coefficients for frequencies in Hz (PhenomDCoef times powers of
 // the total mass), so that a bin's tabulated powers of f multiply them.
 template <class T>

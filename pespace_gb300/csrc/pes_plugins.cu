@@ -189,20 +189,56 @@ __global__ void __launch_bounds__(kLinkThreads) k_response_links(const __grid_co
   }
 }
 
-__global__ void k_tdi(const double* __restrict__ freqs, int64_t n, double arm, int gen20, int orth,
-                      const double2* __restrict__ links, double2* __restrict__ out) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// Michelson TDI of the six links.  FP64-bound: 80 FP64 instructions per bin (the plain
+// formulae with the library's sine and cosine took 140, 27 us on 125 410 bins): the A/E/T
+// norms join the generation prefactor, which is (1 - D^2) or (1 - D^2)(1 - D^4).
+constexpr int kTdiThreads = 128;
+__global__ void __launch_bounds__(kTdiThreads) k_tdi(const double* __restrict__ freqs, int64_t n, double arm, int gen20,
+                                                     int orth, const double2* __restrict__ links,
+                                                     double2* __restrict__ out) {
+  __shared__ double2 tab[kTrig];
+  fill_trig(tab);
+  __syncthreads();
+  const int64_t i = blockIdx.x * (int64_t)kTdiThreads + threadIdx.x;
   if (i >= n) return;
-  Cx<double> D, P, L[6], C[3];
-  tdi_factors(freqs[i], arm, gen20, D, P);
-#pragma unroll
-  for (int l = 0; l < 6; ++l) {
-    double2 v = links[l * n + i];
-    L[l] = cx(v.x, v.y);
+  double Dr, Di;
+  sincos64(tab, -2.0 * kPi * freqs[i] * arm, &Di, &Dr);
+  const double d2r = fma(Dr, Dr, -(Di * Di)), d2i = 2.0 * (Dr * Di);
+  double pr = 1.0 - d2r, pi = -d2i;
+  if (gen20) {
+    const double qr = 1.0 - fma(d2r, d2r, -(d2i * d2i)), qi = -2.0 * (d2r * d2i);
+    const double t = fma(pr, qr, -(pi * qi));
+    pi = fma(pr, qi, pi * qr);
+    pr = t;
   }
-  tdi_channels<double>(D, P, orth, L, C);
+  double2 L[6];
 #pragma unroll
-  for (int c = 0; c < 3; ++c) out[c * n + i] = make_double2(C[c].re, C[c].im);
+  for (int l = 0; l < 6; ++l) L[l] = links[l * n + i];
+  // L: 0=12 1=21 2=23 3=32 4=31 5=13; X = (l13 - l12) + D (l31 - l21) and cyclic
+  double xr[3], xi[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const double2 a = L[(5 + 2 * k) % 6], b = L[2 * k], c = L[(4 + 2 * k) % 6], d = L[2 * k + 1];
+    const double vr = c.x - d.x, vi = c.y - d.y;
+    xr[k] = fma(Dr, vr, fma(-Di, vi, a.x - b.x));
+    xi[k] = fma(Dr, vi, fma(Di, vr, a.y - b.y));
+  }
+  if (orth) {
+    const double sr = xr[0] + xr[2], si = xi[0] + xi[2], ar = xr[2] - xr[0], ai = xi[2] - xi[0];
+    const double yr = xr[1], yi = xi[1];
+    xr[0] = ar;
+    xi[0] = ai;
+    xr[1] = fma(-2.0, yr, sr);
+    xi[1] = fma(-2.0, yi, si);
+    xr[2] = sr + yr;
+    xi[2] = si + yi;
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double w = c == 0 ? 0.70710678118654752 : (c == 1 ? 0.40824829046386302 : 0.57735026918962576);
+    const double gr = orth ? pr * w : pr, gi = orth ? pi * w : pi;
+    out[c * n + i] = make_double2(fma(gr, xr[c], -(gi * xi[c])), fma(gr, xi[c], gi * xr[c]));
+  }
 }
 
 constexpr int kWhittleThreads = 256;
@@ -318,35 +354,12 @@ struct WaveArg {
   WaveMode md[kModes];
 };
 
-// host: products and quotients of pairs hi + lo (the leading phase terms reach
-// 1e5 rad: their coefficients are rounded once)
-struct DD {
-  double h, l;
-};
-static DD dd_two(double a, double b) {
-  const double s = a + b, t = s - a;
-  return {s, (a - (s - t)) + (b - t)};
-}
-static DD dd_mul(const DD& a, const DD& b) {
-  const double p = a.h * b.h;
-  return dd_two(p, std::fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h));
-}
-static DD dd_div(const DD& a, const DD& b) {
-  const double q = a.h / b.h;
-  const double p = q * b.h, e = std::fma(q, b.h, -p);
-  return dd_two(q, (((a.h - p) - e) + a.l - q * b.l) / b.h);
-}
-static DD dd_cbrt(const DD& a) {
-  const double c = std::cbrt(a.h);
-  const DD c3 = dd_mul(dd_mul({c, 0.0}, {c, 0.0}), {c, 0.0});
-  return dd_two(c, ((a.h - c3.h) + (a.l - c3.l)) / (3.0 * c * c));
-}
-
 static void wave_mode(const PhenomDCoef<double>& c, const HMMode<double>& md, const PhenomHMCoef<double>* h, int k,
                       WaveMode& o) {
   const double M = c.Msec, iM = 1.0 / M;
   const double m = (double)kHMlmHost[k][1], hm = 0.5 * m, qt = md.qt;
-  // inspiral at 2 f / m: powers of tm M
+  // inspiral at 2 f / m: powers of tm M (the leading phase terms reach 1e5 rad: their
+  // coefficients are rounded once)
   const DD tm = dd_div({2.0, 0.0}, {m, 0.0}), Mt = dd_mul(tm, {M, 0.0}), cu = dd_cbrt(Mt), one = {1.0, 0.0};
   const DD icu = dd_div(one, cu), icu2 = dd_mul(icu, icu);
   DD pw = dd_mul(dd_mul(icu2, icu2), icu);
@@ -460,13 +473,18 @@ __global__ void __launch_bounds__(kWaveThreads) k_wave(const __grid_constant__ W
   if (i < n) {
     const double f = freqs[i];
     const bool in = !(f > f_cut);
-    double u = 0.0, jf = 0.0, lf3 = 0.0, iu5 = 0.0, p76 = 0.0;
+    double u = 0.0, jf = 0.0, lf3 = 0.0, iu5 = 0.0, iu5l = 0.0, p76 = 0.0;
     if (in) {
       u = cbrt(f);
       jf = rcp64(f);
       lf3 = log(f) * (1.0 / 3.0);
-      iu5 = (jf * jf) * u;  // u^{-5} = u / f^2
       p76 = jf * rsqrt(u);
+      // u^{-5} = u / f^2 as a pair: the phase's leading terms multiply its error by 1e5
+      const double q = jf * jf, eq = fma(jf, jf, -q), ej = fma(-f, jf, 1.0);
+      const double u2 = u * u, e2 = fma(u, u, -u2), u3 = u2 * u, e3 = fma(u2, u, -u3);
+      const double du = ((f - u3) - fma(e2, u, e3)) * jf * (1.0 / 3.0);  // relative error of u
+      iu5 = q * u;
+      iu5l = fma(eq, u, fma(q, u, -iu5)) + iu5 * fma(2.0, ej, du);
     }
 #pragma unroll 1
     for (int k = blockIdx.y; k < kModes; k += gridDim.y) {
@@ -519,7 +537,7 @@ __global__ void __launch_bounds__(kWaveThreads) k_wave(const __grid_constant__ W
           if (j != 5) r = fma(r, u, c.rin[j]); else r *= u;
         }
         const double l1 = c.lg1 * u;
-        psi = fma(p, iu5, (c.lg0 + l1) * lf3);
+        psi = fma(p, iu5, fma(p, iu5l, (c.lg0 + l1) * lf3));
         t = jf * fma(r, iu5, fma(l1, lf3 + 1.0, c.lg0) * (1.0 / (6.0 * kPi)));
       } else if (f < c.fj2) {
         double jx = jf, l = 3.0 * lf3;
@@ -1144,7 +1162,7 @@ int pes_tdi_combination(const double* freqs, int64_t n, double arm_sec, int32_t 
   PES_REQUIRE(n >= 0, "pes_tdi_combination: n < 0");
   if (n == 0) return PES_OK;
   PES_REQUIRE(freqs && links && out, "pes_tdi_combination: null pointer");
-  k_tdi<<<ceil_div(n, 128), 128, 0, as_stream(stream)>>>(freqs, n, arm_sec, generation == 20, orthogonal != 0,
+  k_tdi<<<ceil_div(n, kTdiThreads), kTdiThreads, 0, as_stream(stream)>>>(freqs, n, arm_sec, generation == 20, orthogonal != 0,
                                                           reinterpret_cast<const double2*>(links),
                                                           reinterpret_cast<double2*>(out));
   PES_CHECK_LAUNCH();
@@ -1153,7 +1171,9 @@ int pes_tdi_combination(const double* freqs, int64_t n, double arm_sec, int32_t 
 
 int64_t pes_whittle_workspace_len(int64_t n) {
   if (n <= 0) return 1;
-  int64_t blocks = (n + 4 * kWhittleThreads - 1) / (4 * kWhittleThreads);
+  // one bin per thread up to 1024 blocks (four per thread left most SMs a block or none:
+  // 20 us on 125 410 bins)
+  int64_t blocks = (n + kWhittleThreads - 1) / kWhittleThreads;
   return blocks < kWhittleMaxBlocks ? blocks : kWhittleMaxBlocks;
 }
 
