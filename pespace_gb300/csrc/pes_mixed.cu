@@ -1428,7 +1428,7 @@ __global__ void __launch_bounds__(kSplineThreads) k_spline_adjoint_wide(MixedDev
 // lane keeps its segment's rows in registers (fully unrolled, predicated
 // loops), so the recurrences wait on arithmetic only.  Phase (q == 0) in FP64,
 // transfer quantities in FP32 with FP64 slopes and right-hand sides.
-constexpr int kSegMax = 64;  // longest register segment (grids of up to 64 x 32 intervals)
+constexpr int kSegMax = 64;  // longest segment (grids of up to 64 x 32 intervals)
 
 // Register segment length for a grid of J nodes (0: use the global-scratch kernels).
 inline int spline_seg(int J) { return J <= 32 * 32 + 1 ? 32 : (J <= kSegMax * 32 + 1 ? kSegMax : 0); }
@@ -3555,7 +3555,7 @@ static int alloc(MixedBuffers* mb, X** ptr, size_t count) {
   return PES_OK;
 }
 
-// Spline fit of the first B samples: staged register-segment kernels (phase
+// Spline fit of the first B samples: staged segment kernels (phase
 // systems in FF, transfer systems in FP32), or the global-scratch kernel for
 // grids beyond 64 x 32 intervals.
 // The phase systems on st_phase, the transfer systems on st_transfer (the
