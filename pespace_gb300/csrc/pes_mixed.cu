@@ -875,7 +875,8 @@ __device__ __forceinline__ void range_sample(const PlanDev& P, const MixedDev& M
                                              const SampleBlock<double>* __restrict__ blocks, int64_t B, int64_t t) {
   // one thread per virtual sample
   const int nm = M.n_modes;
-  if (t < 2) M.rcount[t] = 0;  // this call's re-evaluation lists
+  // this call's re-evaluation lists: one thread, since a launch may have no second one
+  if (t == 0) M.rcount[0] = M.rcount[1] = 0;
   if (t >= B * nm) return;
   const int64_t s = t / nm;
   const int kmode = (int)(t % nm);
@@ -3893,6 +3894,7 @@ int mixed_create(PesPlan* p) {
   PES_CHECK_CUDA(cudaMemset(wspk, 0, sizeof(int32_t) * nd * J));
   M.rpart = rpart;
   M.rcount = rcount;
+  PES_CHECK_CUDA(cudaMemset(rcount, 0, sizeof(int32_t) * 2));
   M.trig_ff = trig;
   k_trig_ff<<<1, kFfTrig>>>(trig);
   PES_CHECK_LAUNCH();
