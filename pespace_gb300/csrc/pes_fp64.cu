@@ -45,6 +45,14 @@ constexpr int k64Threads = 128;
 // prologue and the reduction of the gradient's accumulators over more bins.
 constexpr int k64BinsPerThread = 4;
 constexpr int k64SmallBlocks = 152 * 4 * 2;
+// Block partials.  lnL needs one double per block, the gradient k64Acc; a gradient
+// of many samples runs in chunks of them, so that its workspace is the larger of
+// what k64GradRows blocks take (6.7 MB: 54 times the 304 gradient blocks that the
+// chip holds, so that the chunks' last waves do not matter) and of k64RowDoubles
+// doubles per block of the whole batch (51 made 10.9 GB of 4096 samples on
+// 3 354 437 bins).
+constexpr int64_t k64GradRows = 16384;
+constexpr int k64RowDoubles = 5;
 
 // ------------------------------------------------------------------ tables
 // Per bin, seven rows of nbins: f, f^{1/3}, f^{-5/3} (rounded once: the phase's leading
@@ -698,6 +706,7 @@ struct Fp64Buffers {
   Dense64Block* blocks = nullptr;
   RespTab* resp = nullptr;
   double* partial = nullptr;
+  int64_t grad_rows = 0;  // blocks of a gradient chunk that `partial` holds
   SampleBlock<Dual<4>>* tan = nullptr;
   cudaStream_t side = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
@@ -708,12 +717,14 @@ int fp64_create(PesPlan* p) {
   p->fp64 = b;
   const int64_t n = p->desc.nbins, B = p->desc.max_batch;
   // block partials: of the largest batch at 4 bins per thread, or of a small call at 1
-  const int64_t rows = std::max<int64_t>(B * ceil_div(n, k64Threads * k64BinsPerThread), k64SmallBlocks);
+  const int64_t nblk = ceil_div(n, k64Threads * k64BinsPerThread), rows = std::max<int64_t>(B * nblk, k64SmallBlocks);
+  b->grad_rows = std::max(std::min(rows, k64GradRows), std::max(nblk, B * nblk * k64RowDoubles / k64Acc));
+  const int64_t partial = std::max(rows, b->grad_rows * k64Acc);
   cudaError_t e = cudaMalloc(&b->grid, sizeof(double) * kGridRows * n);
   if (e == cudaSuccess) e = cudaMalloc(&b->trig, sizeof(double2) * kTrig);
   if (e == cudaSuccess) e = cudaMalloc(&b->blocks, sizeof(Dense64Block) * B);
   if (e == cudaSuccess) e = cudaMalloc(&b->resp, sizeof(RespTab) * B * p->desc.n_det);
-  if (e == cudaSuccess) e = cudaMalloc(&b->partial, sizeof(double) * rows * k64Acc);
+  if (e == cudaSuccess) e = cudaMalloc(&b->partial, sizeof(double) * partial);
   if (e == cudaSuccess) e = cudaMalloc(&b->tan, sizeof(SampleBlock<Dual<4>>) * B);
   if (e != cudaSuccess) {
     set_error("pes_plan_create: cudaMalloc failed: %s", cudaGetErrorString(e));
@@ -768,26 +779,39 @@ int fp64_lnl(PesPlan* p, const double* theta, int64_t B, double* lnl, double* gr
   const int64_t n = p->desc.nbins;
   const int bpt = B * (int64_t)ceil_div(n, k64Threads) <= k64SmallBlocks ? 1 : k64BinsPerThread;
   const int nblk = (int)ceil_div(n, k64Threads * bpt);
-  const dim3 grid(nblk, (unsigned)B);
-  {
-    ProfScope ps(p, kKDenseFp64, st);
-    if (grad)
-      k_dense64<true><<<grid, k64Threads, dense64_smem<true>(), st>>>(p->dev, b->blocks, b->resp, b->grid, b->trig, nblk,
-                                                                      bpt, b->partial);
-    else
-      k_dense64<false><<<grid, k64Threads, 0, st>>>(p->dev, b->blocks, b->resp, b->grid, b->trig, nblk, bpt, b->partial);
-  }
-  PES_CHECK_LAUNCH();
-  if (grad) PES_CHECK_CUDA(cudaStreamWaitEvent(st, b->join, 0));
-  {
-    ProfScope ps(p, kKFinalize, st);
-    if (grad)
-      k_final64<true><<<ceil_div(B, 2), 64, 0, st>>>(p->dev, b->blocks, B, nblk, bpt, b->partial, b->tan, lnl, grad, status);
-    else
+  if (!grad) {
+    {
+      ProfScope ps(p, kKDenseFp64, st);
+      k_dense64<false><<<dim3(nblk, (unsigned)B), k64Threads, 0, st>>>(p->dev, b->blocks, b->resp, b->grid, b->trig, nblk,
+                                                                       bpt, b->partial);
+    }
+    PES_CHECK_LAUNCH();
+    {
+      ProfScope ps(p, kKFinalize, st);
       k_final64<false><<<ceil_div(B, 2), 64, 0, st>>>(p->dev, b->blocks, B, nblk, bpt, b->partial, nullptr, lnl, nullptr,
                                                      status);
+    }
+    PES_CHECK_LAUNCH();
+    return PES_OK;
   }
-  PES_CHECK_LAUNCH();
+  // in chunks of the samples whose partials the workspace holds
+  const int64_t most = std::min<int64_t>(B, b->grad_rows / nblk);
+  for (int64_t s0 = 0; s0 < B; s0 += most) {
+    const int64_t Bc = std::min(most, B - s0);
+    {
+      ProfScope ps(p, kKDenseFp64, st);
+      k_dense64<true><<<dim3(nblk, (unsigned)Bc), k64Threads, dense64_smem<true>(), st>>>(
+          p->dev, b->blocks + s0, b->resp + s0 * p->desc.n_det, b->grid, b->trig, nblk, bpt, b->partial);
+    }
+    PES_CHECK_LAUNCH();
+    if (s0 == 0) PES_CHECK_CUDA(cudaStreamWaitEvent(st, b->join, 0));
+    {
+      ProfScope ps(p, kKFinalize, st);
+      k_final64<true><<<ceil_div(Bc, 2), 64, 0, st>>>(p->dev, b->blocks + s0, Bc, nblk, bpt, b->partial, b->tan + s0,
+                                                     lnl + s0, grad + 11 * s0, status ? status + s0 : nullptr);
+    }
+    PES_CHECK_LAUNCH();
+  }
   return PES_OK;
 }
 
