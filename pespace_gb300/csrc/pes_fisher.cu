@@ -161,9 +161,8 @@ __global__ void k_fisher_final(const SampleBlock<FisherScalar>* __restrict__ blo
 // depending on the mass and spin parameters only.  Its derivatives are
 //   dh/dtheta = (d(A Y)/dtheta - i A Y dphase/dtheta) exp(-i phase),
 // and the phase factor cancels in conj(dh_a) dh_b, so the Fisher needs no
-// phase values.  The waveform's part per bin (A, t(f), and the tangents of Psi
-// and t(f) in float-float, of A in FP32, which enters beside Psi's with a factor
-// of 1e-2) is linear in the tangents of the model's coefficients: Horner
+// phase values.  The waveform's part per bin (A, t(f) and the tangents of A, Psi
+// and t(f), in float-float) is linear in the tangents of the model's coefficients: Horner
 // sums over tabulated powers of f, each sample's coefficients rescaled to them.
 // The response per unit amplitude takes FP32 duals over (T, lambda, sin beta,
 // psi, cos iota); ln D_L and phi_c are analytic (dh = -h and 2 i h).
@@ -176,8 +175,9 @@ __global__ void k_fisher_final(const SampleBlock<FisherScalar>* __restrict__ blo
 // 6, three of four warps waiting).  Float-float dual numbers through the
 // waveform, and FP64 square roots and conversions of the weights per bin, took
 // most of the time before: 100 samples on 125 410 bins 5.21 -> 2.04 ms, and 1.88 ms with
-// two groups of 128 bins per block, whose warps fetch the same code (5 200 FP32
-// operations per bin and detector, two thirds in the response).
+// two groups of 128 bins per block, whose warps fetch the same code; 1.98 ms with A's
+// tangents in float-float too (about 5 500 FP32 operations per bin and detector, most of
+// them in the response).
 constexpr int kFastThreads = 128;  // bins per group
 constexpr int kFastGroups = 2;     // groups per block
 constexpr int kFastBins = kFastThreads * kFastGroups;
@@ -223,12 +223,10 @@ struct FisherSample {
   // t(f): inspiral (j - 5) pin_j / (6 pi), lg / (6 pi); intermediate; merger-ringdown
   float2 rin[12], rl0, rl1, ri[3], rm[4];  // rm: pm1, pm2, 0.75 pm3, pm4 fd, over 2 pi
   float2 drin[12][4], drl0[4], drl1[4], dri[3][4], drm[4][4];
-  float2 f5, ifd, fd2;
-  float fd, pm4, df5[4], dfd[4];
+  float2 f5, ifd, fd, fd2, pm4, df5[4], dfd[4];
   // amplitude: a0 scaled; Ahat and its tangents (intermediate in (f - fc) / hw)
-  float2 a0, ai[8], ei[5], fc, ihw, gm, w2, fr, gx;
-  float wf;
-  float dlna0[4], dai[8][4], dei[5][4], dlngm[4], dw[4], dfr[4], dgx[4];
+  float2 a0, ai[8], ei[5], fc, ihw, gm, wf, w2, fr, gx;
+  float2 dlna0[4], dai[8][4], dei[5][4], dlngm[4], dw[4], dfr[4], dgx[4];
   float fj1, fj2, fa1, fa2;
   Polar<FR> pol;
   FR pfac, cfac;
@@ -324,16 +322,16 @@ __global__ void __launch_bounds__(64) k_fisher_prep(double scale, const SampleBl
       o.drm[j][lane] = ff2(rm[j] * i2p * x.d[0]);
       if (lane == 0) o.rm[j] = ff2(rm[j] * i2p * x.v);
     }
-    o.df5[lane] = (float)fc.f5.d[0];
-    o.dfd[lane] = (float)fc.fd.d[0];
+    o.df5[lane] = ff2(fc.f5.d[0]);
+    o.dfd[lane] = ff2(fc.fd.d[0]);
     if (lane == 0) {
       o.rl0 = ff2(i6p * fc.lg0.v);
       o.rl1 = ff2(i6p * fc.lg1.v);
       o.f5 = ff2(fc.f5.v);
       o.ifd = ff2(1.0 / fc.fd.v);
-      o.fd = (float)fc.fd.v;
+      o.fd = ff2(fc.fd.v);
       o.fd2 = ff2(fc.fd.v * fc.fd.v);
-      o.pm4 = (float)fc.pm[4].v;
+      o.pm4 = ff2(fc.pm[4].v);
       o.fj1 = (float)(kPhiJoinIns * iM);
       o.fj2 = (float)(0.5 * (c.fRD.v * iM));
       o.status = kSampleOk;
@@ -355,27 +353,27 @@ __global__ void __launch_bounds__(64) k_fisher_prep(double scale, const SampleBl
     double pw = 1.0;
 #pragma unroll
     for (int j = 0; j < 5; ++j) {
-      o.dei[j][lane] = (float)(e[j].d[0] * pw);
+      o.dei[j][lane] = ff2(e[j].d[0] * pw);
       if (lane == 0) o.ei[j] = ff2(e[j].v * pw);
       pw *= hw;
     }
   }
-  o.dlna0[lane] = (float)(fc.a0.d[0] / fc.a0.v);
+  o.dlna0[lane] = ff2(fc.a0.d[0] / fc.a0.v);
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    o.dai[j][lane] = (float)fc.ai[j].d[0];
+    o.dai[j][lane] = ff2(fc.ai[j].d[0]);
     if (lane == 0) o.ai[j] = ff2(fc.ai[j].v);
   }
-  o.dlngm[lane] = (float)(fc.gm.d[0] / fc.gm.v);
-  o.dw[lane] = (float)fc.w.d[0];
-  o.dfr[lane] = (float)fc.fr.d[0];
-  o.dgx[lane] = (float)fc.gx.d[0];
+  o.dlngm[lane] = ff2(fc.gm.d[0] / fc.gm.v);
+  o.dw[lane] = ff2(fc.w.d[0]);
+  o.dfr[lane] = ff2(fc.fr.d[0]);
+  o.dgx[lane] = ff2(fc.gx.d[0]);
   if (lane == 0) {
     o.a0 = ff2(fc.a0.v * scale);
     o.fc = ff2(mid);
     o.ihw = ff2(1.0 / hw);
     o.gm = ff2(fc.gm.v);
-    o.wf = (float)fc.w.v;
+    o.wf = ff2(fc.w.v);
     o.w2 = ff2(fc.w.v * fc.w.v);
     o.fr = ff2(fc.fr.v);
     o.gx = ff2(fc.gx.v);
@@ -396,7 +394,7 @@ __device__ __forceinline__ void wave_tangents(const FisherSample& sb, const floa
   float (&ps)[4] = o.ps, (&dt)[4] = o.dt;
   const float4 r0 = rows[i], r1 = rows[n + i], r2 = rows[2 * n + i];
   const FF ff = ff_make(r0.x, r0.y), uu = ff_make(r0.z, r0.w), jj = ff_make(r1.x, r1.y), ll = ff_make(r1.z, r1.w);
-  const float f = ff.hi, u = uu.hi, jf = jj.hi, lf3 = ll.hi;
+  const float f = ff.hi;
   // ---- phase tangents, t(f) and its tangents
   FF tf;
   if (f < sb.fj1) {
@@ -421,7 +419,7 @@ __device__ __forceinline__ void wave_tangents(const FisherSample& sb, const floa
       p = ff_mad(p, iu5, l);
       ps[k] = p.hi + p.lo;
       r = ff_mad(r, iu5, ff_mad(ff_load(sb.drl1[k]), ul, ff_load(sb.drl0[k])));
-      dt[k] = jf * (r.hi + r.lo);
+      dt[k] = (jj * ff_fast_two_sum(r.hi, r.lo)).hi;
     }
   } else if (f < sb.fj2) {
     const FF j3 = (jj * jj) * jj;
@@ -441,7 +439,7 @@ __device__ __forceinline__ void wave_tangents(const FisherSample& sb, const floa
     const FF q = ff_make(r2.z, r2.w), fq = ff * q;
     const FF xx = ff - ff_load(sb.f5);
     const FF rd = ff_make(1.0f, 0.0f) / (xx * xx + ff_load(sb.fd2));
-    const float x = xx.hi, rden = rd.hi;
+    const FF fd = ff_load(sb.fd), m4 = -(ff_load(sb.pm4) * rd), rm4 = ff_mulf(ff_load(sb.rm[3]) * rd, 2.0f) * rd;
     const FF at = datan(xx * ff_load(sb.ifd));
     tf = ff_mad(ff_load(sb.rm[1]), jj * jj, ff_load(sb.rm[0]));
     tf = ff_mad(ff_load(sb.rm[2]), q, tf);
@@ -452,60 +450,63 @@ __device__ __forceinline__ void wave_tangents(const FisherSample& sb, const floa
       p = ff_mad(ff_load(sb.pm[2][k]), jj, p);
       p = ff_mad(ff_load(sb.pm[3][k]), fq, p);
       p = ff_mad(ff_load(sb.pm[4][k]), at, p);
-      p = ff_addf(p, -(sb.pm4 * rden) * fmaf(sb.df5[k], sb.fd, x * sb.dfd[k]));
+      const FF d5 = ff_load(sb.df5[k]), dd = ff_load(sb.dfd[k]);
+      p = ff_mad(m4, ff_dot2(d5, fd, xx, dd), p);
       ps[k] = p.hi + p.lo;
-      const float drden = 2.0f * rden * fmaf(x, sb.df5[k], -(sb.fd * sb.dfd[k]));  // over rden
       FF r = ff_mad(ff_load(sb.drm[1][k]), jj * jj, ff_load(sb.drm[0][k]));
       r = ff_mad(ff_load(sb.drm[2][k]), q, r);
       r = ff_mad(ff_load(sb.drm[3][k]), rd, r);
-      dt[k] = fmaf(rden * sb.rm[3].x, drden, r.hi + r.lo);
+      r = ff_mad(rm4, ff_dot2(xx, d5, -fd, dd), r);  // rm[3] times the tangent of rd
+      dt[k] = r.hi + r.lo;
     }
   }
   tf = ff_fast_two_sum(tf.hi, tf.lo);
   o.tf = tf.hi;
   // ---- amplitude, the tangents of its logarithm
-  FF ah;
-  float da[4];
+  FF ah, da[4];
   if (f < sb.fa1) {
     FF p = ff_load(sb.ai[7]);
 #pragma unroll
     for (int j = 6; j >= 0; --j) p = ff_mad(p, uu, ff_load(sb.ai[j]));
     ah = ff_addf(ff_fast_two_sum(p.hi, p.lo) * (uu * uu), 1.0f);
-    const float g = u * u / ah.hi;
+    const FF g = uu * uu / ah;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      float r = sb.dai[7][k];
+      FF r = ff_load(sb.dai[7][k]);
 #pragma unroll
-      for (int j = 6; j >= 0; --j) r = fmaf(r, u, sb.dai[j][k]);
-      da[k] = fmaf(r, g, sb.dlna0[k]);
+      for (int j = 6; j >= 0; --j) r = ff_mad(r, uu, ff_load(sb.dai[j][k]));
+      da[k] = ff_mad(r, g, ff_load(sb.dlna0[k]));
     }
   } else if (f < sb.fa2) {
     const FF xx = (ff - ff_load(sb.fc)) * ff_load(sb.ihw);
-    const float x = xx.hi;
     ah = ff_load(sb.ei[4]);
 #pragma unroll
     for (int j = 3; j >= 0; --j) ah = ff_mad(ah, xx, ff_load(sb.ei[j]));
     ah = ff_fast_two_sum(ah.hi, ah.lo);
-    const float g = 1.0f / ah.hi;
+    const FF g = ff_make(1.0f, 0.0f) / ah;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const float r = fmaf(x, fmaf(x, fmaf(x, fmaf(x, sb.dei[4][k], sb.dei[3][k]), sb.dei[2][k]), sb.dei[1][k]), sb.dei[0][k]);
-      da[k] = fmaf(r, g, sb.dlna0[k]);
+      FF r = ff_load(sb.dei[4][k]);
+#pragma unroll
+      for (int j = 3; j >= 0; --j) r = ff_mad(r, xx, ff_load(sb.dei[j][k]));
+      da[k] = ff_mad(r, g, ff_load(sb.dlna0[k]));
     }
   } else {
     const FF xx = ff - ff_load(sb.fr);
-    const float x = xx.hi;
-    const FF den = xx * xx + ff_load(sb.w2);
-    const float rw = 1.0f / den.hi;
-    ah = ff_load(sb.gm) / den * dexp(-(ff_load(sb.gx) * xx));
+    const FF den = xx * xx + ff_load(sb.w2), gx = ff_load(sb.gx), w = ff_load(sb.wf);
+    const FF rw2 = ff_make(2.0f, 0.0f) / den;
+    ah = ff_load(sb.gm) / den * dexp(-(gx * xx));
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-      da[k] = sb.dlna0[k] + sb.dlngm[k] + 2.0f * rw * fmaf(x, sb.dfr[k], -(sb.wf * sb.dw[k])) +
-              fmaf(sb.gx.x, sb.dfr[k], -(sb.dgx[k] * x));
+    for (int k = 0; k < 4; ++k) {
+      const FF dr = ff_load(sb.dfr[k]);
+      const FF c = ff_load(sb.dlna0[k]) + ff_load(sb.dlngm[k]);
+      da[k] = ff_mad(rw2, ff_dot2(xx, dr, -w, ff_load(sb.dw[k])), ff_add_lazy(c, ff_dot2(gx, dr, -ff_load(sb.dgx[k]), xx)));
+    }
   }
-  o.A = (ff_load(sb.a0) * ff_load(p76[i]) * ah).hi;
+  const FF A = ff_load(sb.a0) * ff_load(p76[i]) * ah;
+  o.A = A.hi;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) o.dA[k] = o.A * da[k];
+  for (int k = 0; k < 4; ++k) o.dA[k] = (A * ff_fast_two_sum(da[k].hi, da[k].lo)).hi;
 }
 
 // The summing warp's share: rows of the upper triangle in pieces of up to three pairs, one per lane.
