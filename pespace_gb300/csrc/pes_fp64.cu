@@ -236,11 +236,7 @@ __device__ __forceinline__ double bin64(const PlanDev& P, const Dense64Block& b,
   const double a0p = c.a0 * grid[kGp76 * n + i], A = a0p * ah;
   // ---- phase 2 pi f t_c, rounded as the plain formula's argument is, whole turns removed
   const double w2 = (2.0 * kPi) * f;
-  double ptc;
-  {
-    const double p = w2 * b.tc, kf = fma(p, k64InvTwoPi, k64Magic) - k64Magic;
-    ptc = fma(-kf, k64TwoPiLo, fma(-kf, k64TwoPi, p));
-  }
+  const double ptc = turns64(w2 * b.tc);
   const double T = tf + b.tc, pif = kPi * f;
   double sum = 0.0;
   double reS = 0.0, imS = 0.0, RT = 0.0;  // adjoints of A (over A), of the phase and of T

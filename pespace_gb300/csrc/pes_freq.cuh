@@ -14,9 +14,25 @@ constexpr double k64TwoPi = 6.283185307179586;              // 2 pi, head
 constexpr double k64TwoPiLo = 2.4492935982947064e-16;       // 2 pi - head
 constexpr double k64InvTwoPi = 0.15915494309189535;
 
-// sin and cos of |x| < 1e9: x = k 2 pi / 256 + r, |r| <= pi / 256, table of the
-// first, Taylor polynomials of the second (truncation below 1e-19), angle sum.
+// |x| from 2^45 on (also infinities and NaN): past what sincos64 reduces
+__device__ __forceinline__ bool far64(double x) { return (__double2hiint(x) & 0x7fffffff) >= 0x42c00000; }
+// sin and cos of such arguments (phases of light sources decades before they merge): the library's.
+static __device__ __noinline__ double2 sincos64_far(double x) {
+  double2 r;
+  sincos(x, &r.x, &r.y);
+  return r;
+}
+
+// sin and cos: x = k 2 pi / 256 + r, |r| <= pi / 256, table of the first, Taylor
+// polynomials of the second (truncation below 1e-19), angle sum.  The rounding to k by
+// k64Magic holds below 2^51 steps: |x| < 2^45.
 __device__ __forceinline__ void sincos64(const double2* __restrict__ tab, double x, double* s, double* c) {
+  if (far64(x)) {
+    const double2 v = sincos64_far(x);
+    *s = v.x;
+    *c = v.y;
+    return;
+  }
   const double t = fma(x, k64InvTwoPi * kTrig, k64Magic);
   const int k = __double2loint(t) & (kTrig - 1);
   const double kf = t - k64Magic;
@@ -28,6 +44,13 @@ __device__ __forceinline__ void sincos64(const double2* __restrict__ tab, double
   const double2 e = tab[k];
   *s = e.x + fma(e.x, cm, e.y * sr);
   *c = e.y + fma(e.y, cm, -(e.x * sr));
+}
+
+// x less its whole turns (x itself where far64)
+__device__ __forceinline__ double turns64(double x) {
+  if (far64(x)) return x;
+  const double kf = fma(x, k64InvTwoPi, k64Magic) - k64Magic;
+  return fma(-kf, k64TwoPiLo, fma(-kf, k64TwoPi, x));
 }
 
 // 1 / x for normal positive x: the hardware estimate and two Newton steps

@@ -121,11 +121,7 @@ __global__ void __launch_bounds__(kLinkThreads) k_response_links(const __grid_co
     const double f = freqs[i], pif = kPi * f, w2 = 2.0 * kPi * f, aL = pif * a.arm_sec;
     const int tier = sinc_tier(2.0 * fabs(aL));
     // 2 pi f t_c, rounded as the plain formula's argument is, whole turns removed
-    double ptc;
-    {
-      const double p = w2 * a.tc, kf = fma(p, k64InvTwoPi, k64Magic) - k64Magic;
-      ptc = fma(-kf, k64TwoPiLo, fma(-kf, k64TwoPi, p));
-    }
+    const double ptc = turns64(w2 * a.tc);
     double ar[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, ai[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
 #pragma unroll 1
     for (int m = 0; m < nmodes; ++m) {
