@@ -3,6 +3,7 @@
 // IMRPhenomD / IMRPhenomHM waveform producers.  FP64 throughout, one thread per frequency.
 #include <cmath>
 #include <cstdarg>
+#include <cstddef>
 #include <cstdio>
 #include <mutex>
 
@@ -46,7 +47,7 @@ struct LinkArg {
   double om[2], ph[2];  // revolution, rotation: rate and initial angle
   double arm_sec, tc;
   int32_t helio;
-  int32_t pad;
+  int32_t finite;  // every number above is
 };
 
 static void link_arg(const PesOrbit& ob, double lam, double beta, double psi, double tc, LinkArg& o) {
@@ -102,7 +103,9 @@ static void link_arg(const PesOrbit& ob, double lam, double beta, double psi, do
   o.arm_sec = ob.arm_sec;
   o.tc = tc;
   o.helio = ob.kind == 0;
-  o.pad = 0;
+  o.finite = 1;
+  const double* v = reinterpret_cast<const double*>(&o);
+  for (size_t k = 0; k < offsetof(LinkArg, helio) / sizeof(double); ++k) o.finite &= std::isfinite(v[k]);
 }
 
 constexpr int kLinkThreads = 128;
@@ -127,9 +130,9 @@ __global__ void __launch_bounds__(kLinkThreads) k_response_links(const __grid_co
     for (int m = 0; m < nmodes; ++m) {
       const double2 h1 = hp[m * n + i], h2 = hc[m * n + i];
       const double t = tf[m * n + i];
-      // above its cut a mode is zero, and so are its links
-      if (h1.x == 0.0 && h1.y == 0.0 && h2.x == 0.0 && h2.y == 0.0 && isfinite(t)) continue;
       const double T = t + a.tc;
+      // above its cut a mode is zero, and so are its links (of finite angles and times)
+      if (h1.x == 0.0 && h1.y == 0.0 && h2.x == 0.0 && h2.y == 0.0 && a.finite && isfinite(T) && isfinite(f)) continue;
       double ca, sa, c1, s1, c2 = 0.0, s2 = 0.0;
       sincos64(tab, fma(a.om[0], T, a.ph[0]), &sa, &ca);
       c1 = ca;
