@@ -876,7 +876,7 @@ static int launch_td_tdi(const TdLayout& lay, const double* links, int64_t B, in
 // once per window sample and a channel interpolates 3 or 7 terms instead of 6
 // or 14.  Each channel goes back to a double from the
 // bits and one FP64 add.  Scaled magnitudes below 2^-126 (2^-126 of the
-// window's largest link sample), and the tails of those below 2^-74, flush to
+// window's largest link sample), and the tails of those below 2^-103, flush to
 // zero; a NaN or an infinity among the inputs gives NaN in the outputs that
 // read it.
 //
@@ -913,26 +913,26 @@ static void td_layout_ff(const TdLayout& lay, TdLayoutFF& out) {
 // of |x| and the exponent's shift.
 struct TdScale {
   unsigned rebias;        // (896 + scale) << 23
-  unsigned head0, tail0;  // high words from which x * 2^-scale is at least 2^-126 (and x normal), 2^-74
+  unsigned head0, tail0;  // high words from which x * 2^-scale is at least 2^-126 (and x normal), 2^-103
 };
 __device__ __forceinline__ TdScale td_scale(int scale) {
   TdScale s;
   s.rebias = (unsigned)(896 + scale) << 23;
   s.head0 = (unsigned)max(1, 1023 - 126 + scale) << 20;
-  s.tail0 = (unsigned)max(1, 1023 - 74 + scale) << 20;
+  s.tail0 = (unsigned)max(1, 1023 - 103 + scale) << 20;
   return s;
 }
 
 // x * 2^-scale as a float-float pair: head = sign, exponent and the top 23
 // fraction bits (the exponent's low 9 bits, shifted modulo 2^32); tail = the
-// other 29 fraction bits, rounded to 24 significant bits, times the head's
-// power of two.
+// other 29 fraction bits over 2^29, rounded to 24 significant bits, times the
+// head's power of two over 2^23.
 __device__ __forceinline__ FF td_split(double x, const TdScale& s) {
   const unsigned H = (unsigned)__double2hiint(x), L = (unsigned)__double2loint(x);
   const unsigned a = H & 0x7fffffffu, sign = H & 0x80000000u;
   unsigned hb = (__funnelshift_l(L, H, 3) - s.rebias) | sign;
-  const float pw = __uint_as_float((hb & 0xff800000u) - (52u << 23));  // +-2^(e - 52)
-  float lo = __uint2float_rn(L & 0x1fffffffu) * pw;
+  const float pw = __uint_as_float((hb & 0xff800000u) - (23u << 23));  // +-2^(e - 23)
+  float lo = (__uint2float_rn(L & 0x1fffffffu) * 1.862645149230957e-09f) * pw;
   lo = a < s.tail0 ? 0.0f : lo;
   hb = a < s.head0 ? 0u : hb;
   hb = a >= 0x7ff00000u ? 0x7fc00000u : hb;
