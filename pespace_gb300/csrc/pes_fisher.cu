@@ -634,6 +634,30 @@ __global__ void __launch_bounds__(kFastBlock, 1) k_fisher_fast(PlanDev P, const 
       partial[((size_t)s * gridDim.x * kFastGroups + blockIdx.x * kFastGroups + grp) * kPairs + (pa * 11 - pa * (pa - 1) / 2 + (pb + k - pa))] = acc[k];
 }
 
+// The first call's buffers and tables (fisher_blocks last: it marks them complete).
+// The tables are filled on a stream of their own: later calls may come on another
+// stream, and the caller's may be capturing a graph.
+static int fisher_create(PesPlan* p, bool fast) {
+  const int64_t M = p->desc.max_batch, n = p->desc.nbins, nd = p->desc.n_det;
+  const int64_t rows = std::max<int64_t>(M * kFisherBlocks, kFastRows + M * (int64_t)kFastGroups);
+  PES_CHECK_CUDA(cudaMalloc(&p->fisher_partial, sizeof(double) * rows * kPairs));
+  if (fast) {
+    PES_CHECK_CUDA(cudaMalloc(&p->fisher_samples, sizeof(FisherSample) * M));
+    PES_CHECK_CUDA(cudaMalloc(&p->fisher_rows, sizeof(float4) * n * (3 + 2 * nd)));
+    PES_CHECK_CUDA(cudaMalloc(&p->fisher_p76, sizeof(float2) * n));
+    PES_CHECK_CUDA(cudaFuncSetAttribute(k_fisher_fast, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fisher_smem()));
+    cudaStream_t own;
+    PES_CHECK_CUDA(cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking));
+    k_fisher_grid<<<ceil_div(n, 128), 128, 0, own>>>(p->dev, p->fisher_rows, p->fisher_p76);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(own);
+    cudaStreamDestroy(own);
+    PES_CHECK_CUDA(e);
+  }
+  PES_CHECK_CUDA(cudaMalloc(&p->fisher_blocks, sizeof(SampleBlock<FisherScalar>) * M));
+  return PES_OK;
+}
+
 }  // namespace pes
 
 using namespace pes;
@@ -649,25 +673,25 @@ extern "C" int pes_fisher_batch(PesPlan* p, const double* theta, int64_t B, doub
   if (B == 0) return PES_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool hm = p->desc.approximant == PES_APPROX_PHENOMHM, fast = p->mixed && !hm;
-  const int64_t M = p->desc.max_batch, n = p->desc.nbins, nd = p->desc.n_det;
+  const int64_t n = p->desc.nbins, nd = p->desc.n_det;
   // partial sums per sample: kFisherBlocks, more in calls that would leave SMs idle
   const int64_t nrow = !fast ? (int64_t)kFisherBlocks
                              : std::min<int64_t>(ceil_div(n, kFastThreads),
                                                  std::max<int64_t>(kFisherBlocks, ceil_div(kFastRows, B)));
   const int64_t nblk = !fast ? nrow : ceil_div(nrow, kFastGroups) * (int64_t)kFastGroups;
   if (!p->fisher_blocks) {
-    const int64_t rows = std::max<int64_t>(M * kFisherBlocks, kFastRows + M * (int64_t)kFastGroups);
-    PES_CHECK_CUDA(cudaMalloc(&p->fisher_partial, sizeof(double) * rows * kPairs));
-    if (fast) {
-      PES_CHECK_CUDA(cudaMalloc(&p->fisher_samples, sizeof(FisherSample) * M));
-      PES_CHECK_CUDA(cudaMalloc(&p->fisher_rows, sizeof(float4) * n * (3 + 2 * nd)));
-      PES_CHECK_CUDA(cudaMalloc(&p->fisher_p76, sizeof(float2) * n));
-      PES_CHECK_CUDA(cudaFuncSetAttribute(k_fisher_fast, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fisher_smem()));
-      k_fisher_grid<<<ceil_div(n, 128), 128, 0, st>>>(p->dev, p->fisher_rows, p->fisher_p76);
-      PES_CHECK_LAUNCH();
-      PES_CHECK_CUDA(cudaStreamSynchronize(st));  // later calls may come on another stream
+    const int rc = fisher_create(p, fast);
+    if (rc != PES_OK) {  // a later call begins again
+      cudaFree(p->fisher_partial);
+      cudaFree(p->fisher_samples);
+      cudaFree(p->fisher_rows);
+      cudaFree(p->fisher_p76);
+      p->fisher_partial = nullptr;
+      p->fisher_samples = nullptr;
+      p->fisher_rows = nullptr;
+      p->fisher_p76 = nullptr;
+      return rc;
     }
-    PES_CHECK_CUDA(cudaMalloc(&p->fisher_blocks, sizeof(SampleBlock<FisherScalar>) * M));
   }
   auto* blocks = reinterpret_cast<SampleBlock<FisherScalar>*>(p->fisher_blocks);
   k_setup<FisherScalar><<<setup_blocks(B), 64, 0, st>>>(p->dev, theta, B, 0, blocks, hm_blocks<FisherScalar>(p));

@@ -1,9 +1,11 @@
 """Mixed Fisher matrices where the waveform's tangents are hardest: unequal masses,
 high spins and heavy sources whose merger-ringdown fills the band, against the
-FP64 plan (the mixed plan's bar, 1e-5)."""
+FP64 plan (the mixed plan's bar, 1e-5); and the first call of a plan under a
+relaxed stream capture."""
 
 import numpy as np
 import pytest
+import torch
 
 pytestmark = pytest.mark.gpu
 
@@ -36,3 +38,20 @@ def test_unequal_masses_and_high_spins(cuda_lib, oracle, q, mtot):
     got = _engine(oracle, "mixed", th0, 3).fisher_matrix(thetas).cpu().numpy()
     want = _engine(oracle, "fp64", th0, 3).fisher_matrix(thetas).cpu().numpy()
     assert _normalised_err(got, want) < 1e-5
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_first_call_under_relaxed_capture(cuda_lib, oracle, precision):
+    """The first call allocates and fills its tables; a relaxed capture permits that."""
+    th0 = config0_theta(GRID[0] - 20000.0)
+    eng = _engine(oracle, precision, th0, 2)
+    theta = torch.as_tensor(np.stack([th0, th0]), device="cuda")
+    theta[1, 0] += 0.5
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, capture_error_mode="relaxed"):
+        out = eng.fisher_matrix(theta)
+    graph.replay()
+    torch.cuda.synchronize()
+    captured = out.clone()
+    assert torch.equal(captured, eng.fisher_matrix(theta)) and bool(torch.isfinite(captured).all())
