@@ -7,8 +7,9 @@ atomics may sum in another order):
   each run's inputs one run ahead into shared memory, or loads them
   directly.  Copying wins when the inputs stream from DRAM; direct loads win
   when they sit in L2.  The default is a size threshold (64 MB).
-* ``sample_threads``: threads per block of the one-thread-per-sample kernels
-  of the mixed plan (exact-bin ranges, peak kink).
+* ``sample_threads``: threads per block of the mixed plan's ranges and kinks (a
+  thread per sample and mode, and per detector) and exact-bin ranges (a pair
+  of threads per sample, mode and detector).  FP64 plans have no such launch.
 
 ``autotune`` searches one option at a time (the others held at their current
 values).  It times every candidate on the caller's batch with CUDA events on
@@ -58,7 +59,8 @@ def autotune(likelihood, theta, grad=True, reps=5, candidates=None):
 
     grad : time the lnL+gradient call (True) or the lnL call.
     candidates : {name: values} to search (default ``CANDIDATES``);
-        ``dense_stage`` is skipped for FP64 plans, which ignore it.
+        FP64 plans ignore both options: ``dense_stage`` is skipped and
+        ``sample_threads`` keeps its value, timed once.
 
     Returns {name: {"chosen": value, "ms": {value: median ms per call}}}; the
     chosen values stay set in the plan.
@@ -71,6 +73,8 @@ def autotune(likelihood, theta, grad=True, reps=5, candidates=None):
         raise ValueError(f"unknown launch options: {sorted(unknown)}")
     if likelihood.precision != "mixed":
         cands.pop("dense_stage", None)
+        if "sample_threads" in cands:
+            cands["sample_threads"] = (get_option(likelihood, "sample_threads"),)
     theta = likelihood._prep(theta)[: likelihood.max_batch]
     fn = likelihood.log_likelihood_and_grad if grad else likelihood.log_likelihood_batch
     report = {}
