@@ -816,7 +816,7 @@ def run_native(args):
         ms64 = replicas.reduce_max(timed(lambda: ref.log_likelihood_and_grad(th64), 2), "cuda")
         fp64_gpu = {"value": replicas.job_rate(world, fp64_n, ms64), "unit": "lnL+grad evals/s",
                     "ms_per_step": ms64, "steps": 2, "warmup": 1, "samples": fp64_n,
-                    "path": "FP64 plan: dense FP64 evaluation of every live bin, forward-mode gradient"}
+                    "path": "FP64 plan: dense FP64 evaluation of every live bin, adjoint gradient"}
         del ref
 
     # ---------------- roofline of the dominant kernel (the dense stage)

@@ -242,9 +242,10 @@ const char* pes_kernel_class_name(int32_t k);
  *     1 = the gradient pass of the dense stage copies each run's inputs one
  *     run ahead into shared memory (cp.async), 0 = plain loads.  Default: 1
  *     when the packed dense inputs exceed 64 MB (they stream from DRAM).
- *   PES_OPT_SAMPLE_THREADS: threads per block of the one-thread-per-sample
- *     kernels of the mixed lnL calls (exact-bin ranges, peak kink), 1..128;
- *     default 8.
+ *   PES_OPT_SAMPLE_THREADS (mixed plans; FP64 plans keep and ignore it):
+ *     threads per block of the ranges and kinks (a thread per sample and
+ *     mode, and per detector) and, up to 64, of the exact-bin ranges (a
+ *     pair of threads per sample, mode and detector), 1..128; default 8.
  * One option changes results, not speed, and is not tuned:
  *   PES_OPT_REFINE_ALL (mixed plans): 1 = every sample's dense range is
  *     re-evaluated as the samples whose error estimates approach the

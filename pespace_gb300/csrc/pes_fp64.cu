@@ -24,9 +24,9 @@
 //    adjoints of the coefficients over the bins and the tangents multiply their
 //    sums once per sample (their set-up runs beside the dense pass).
 //
-// Measured: lnL and gradient of 12 samples on LISA + TianQin (2^20 s) 9.6 -> 0.95 ms
+// Measured: lnL and gradient of 12 samples on LISA + TianQin (2^20 s) 10.6 -> 0.97 ms
 // against three passes of Dual<4> through the plain model; lnL of 37 samples on
-// 65 471 bins 1.19 -> 0.73 ms.  The FP64 pipe is active 88% of the cycles of
+// 65 471 bins 1.42 -> 0.88 ms (0.67 to 0.88 ms with the draws' live bins).  The FP64 pipe is active 88% of the cycles of
 // either pass (424 and about 800 FP64 instructions per bin and detector).
 #include <algorithm>
 #include <cmath>
@@ -681,7 +681,8 @@ __global__ void __launch_bounds__(64) k_final64(PlanDev P, const Dense64Block* _
 // thread per sample in the plain order of the formulae: the tangents of the
 // intermediate amplitude's coefficients are ill-conditioned (1e-9 of some
 // gradients), and this order is the one its results are known by.  It runs
-// beside the dense pass, which does not read it.
+// beside the dense pass, which does not read it; calls of a few samples wait for it
+// (one sample on 7 839 bins: 255 us, lnL alone 90 us).
 __global__ void k_tangents64(PlanDev P, const double* __restrict__ theta, int64_t B,
                              SampleBlock<Dual<4>>* __restrict__ blocks) {
   const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;

@@ -46,9 +46,11 @@ constexpr int kMoments = 4;       // t^0..t^3
 // Blocks of the node stage's forward and backward passes: all the warps that an SM
 // holds at their registers in one block.  A node evaluation is about 100 KB of
 // straight-line code, and instruction fetch is its top stall; the warps of one block
-// start together and share what they fetch (blocks of 128: lnL of 1024 prior draws
-// 2.75 ms, with the gradient 3.95 ms; so 2.65 and 3.83 ms.  Loops rolled around arrays in
-// local memory, or only the Horner sums, were slower: 2.83 and 2.93 ms).
+// start together and share what they fetch.  Blocks of 128 against these: lnL of 1024
+// prior draws 2.78 and 2.75 ms, lnL of 64 six-mode samples on the network 7.67 and 7.41 ms,
+// lnL and gradient of 96 samples on it 2.37 and 2.29 ms; the gradient of 1024 draws and
+// calls of 1 to 256 samples on one detector within 1.5% either way.  Loops rolled around
+// arrays in local memory, or only the Horner sums, were slower (2.83 and 2.93 ms).
 constexpr int kSparseThreads = 512;
 constexpr int kBwdThreads = 384;
 // FP32 copies of the shared grid's spline factors, [kGfCount][J]: h, 1/h, lo, up, 1/den, cp.
@@ -248,9 +250,10 @@ __device__ __forceinline__ bool in_zero_window(const MixedDev& M, int d, int64_t
 }
 constexpr double kSpikeRatio = 8.0;
 constexpr int kMomStride = 21;  // moments per bin (and interval) of wmom / wtot
-// The exact re-evaluation: a listed sample's bins go to rblocks parts of at
-// least kRefineBins bins, a partial sum each, and the parts of all listed
-// samples to the blocks that the chip holds.  (A few samples are listed, of up
+// The exact re-evaluation: a listed sample's bins go to rblocks parts, a partial
+// sum each: one per kRefineBins bins of the grid, but from kRefinePartsMin to
+// kRefinePartsMax of them; the parts of all listed samples go to the blocks that
+// the chip holds.  (A few samples are listed, of up
 // to 10^5 bins: with 32 blocks each they left most of the SMs idle.)
 constexpr int kRefineBins = 512;
 constexpr int kRefinePartsMax = 256, kRefinePartsMin = 32;
@@ -488,7 +491,7 @@ __device__ __forceinline__ void kink_sample(const PlanDev& P, const MixedDev& M,
   }
 }
 
-// Forward: node values in float-float arithmetic.  grid (ceil(J/128), n_det, B)
+// Forward: node values in float-float arithmetic.  grid (ceil(J / kSparseThreads), n_det, B n_modes)
 // kMid: the six transfer quantities at the midpoints of intervals 0..nsp-1
 // instead (the exact model that the splines' error estimates compare with).
 template <bool kMid>
@@ -555,7 +558,11 @@ __global__ void __launch_bounds__(kSparseThreads) k_sparse_fwd(PlanDev P, MixedD
 // batch.  Groups of lanes, one tangent per lane, and the two parts on two
 // warps as in k_setup (k_setup_grad_lanes): 74 us at 24 samples, for batches
 // whose other stages do not hide it; at 1024 samples its warps took register
-// space from the node stage (4.11 against 4.03 ms per lnL+gradient call).
+// space from the node stage (4.11 against 4.03 ms per lnL+gradient call).  The line
+// lies where the two are alike: lanes against threads, lnL and gradient on 31 353 bins
+// 390 and 488 us at 24 samples, 583 and 589 at 96, 823 and 822 at 192, 975 and 971 at 256,
+// 1651 and 1607 at 512; on three detectors, 210 000 bins, 0.88 and 1.08 ms at 24
+// samples, 2.32 and 2.26 at 96, 4.28 and 4.21 at 192.
 constexpr int kSetupGradLanesMax = 192;
 __global__ void k_setup_grad(PlanDev P, const double* __restrict__ theta, int64_t B,
                              SampleBlock<GradScalar>* __restrict__ out) {
@@ -1424,14 +1431,14 @@ __global__ void __launch_bounds__(kSplineThreads) k_spline_adjoint_wide(MixedDev
   }
 }
 
-// Register-segment versions (n <= 64 x 32 intervals; segments of 32 rows for
-// the default grid of 1024 nodes, of 64 rows up to 2049 nodes): each
-// lane keeps its segment's rows in registers (fully unrolled, predicated
-// loops), so the recurrences wait on arithmetic only.  Phase (q == 0) in FP64,
-// transfer quantities in FP32 with FP64 slopes and right-hand sides.
+// Segmented versions (n <= 64 x 32 intervals; segments of 32 rows for the
+// default grid of 1024 nodes, of 64 rows up to 2049 nodes): a lane runs its
+// segment's recurrences in rolled loops, the unknowns in shared memory.  The fits'
+// phase systems in float-float, the adjoint's in FP64, transfer quantities in
+// FP32 with float-float slopes.
 constexpr int kSegMax = 64;  // longest segment (grids of up to 64 x 32 intervals)
 
-// Register segment length for a grid of J nodes (0: use the global-scratch kernels).
+// Segment length for a grid of J nodes (0: use the global-scratch kernels).
 inline int spline_seg(int J) { return J <= 32 * 32 + 1 ? 32 : (J <= kSegMax * 32 + 1 ? kSegMax : 0); }
 
 template <class R>
@@ -1479,8 +1486,9 @@ __host__ __device__ __forceinline__ int fit_rows(int J) { return fit_pad(J) + 1;
 // unknowns in registers, each warp ran 200 KB of straight-line code once, and its
 // instruction fetch took half of the fit of a small call (phase fit of 16 systems of 1024
 // intervals 98 -> 57 us, of 72 systems of 2048 intervals 170 -> 87 us).
-// Grids of more than 32 x 32 intervals leave the tables in global memory
-// (staging them would leave room for one block per SM).
+// Grids of more than 32 x 32 intervals leave the tables in global memory: the node
+// values and unknowns alone take up to 133 KB of a phase fit's block (which has its SM to
+// itself at 2049 nodes) and 100 KB of a transfer fit's (two per SM).
 template <class R, bool kStageTables, int kSeg>
 __host__ __device__ __forceinline__ size_t fit_smem_bytes(int J) {
   const size_t rows = (size_t)fit_rows(J);
@@ -3994,7 +4002,7 @@ int mixed_ingest(PesPlan* p, int det, const double* data, const double* psd, cud
   return PES_OK;
 }
 
-// The value set-up: IMRPhenomD plans in the plain order (phenomd_setup_serial).
+// Ranges and kinks in blocks of sample_threads threads.
 static void launch_ranges_kink(PesPlan* p, const SampleBlock<double>* blocks, int64_t B, cudaStream_t st) {
   const MixedDev& M = p->mixed->dev;
   const int64_t V = B * M.n_modes;
@@ -4011,6 +4019,7 @@ static void launch_exact_ranges(PesPlan* p, const SampleBlock<double>* blocks, i
   k_exact_ranges<<<ceil_div(B, threads / group), threads, 0, st>>>(p->dev, M, blocks, B, group);
 }
 
+// The value set-up: IMRPhenomD plans in the plain order (phenomd_setup_serial).
 static void launch_setup(PesPlan* p, const double* theta, int64_t B, SampleBlock<double>* blocks, cudaStream_t st) {
   if (p->desc.approximant == PES_APPROX_PHENOMHM)
     k_setup<double><<<setup_blocks(B), 64, 0, st>>>(p->dev, theta, B, 0, blocks, hm_blocks<double>(p));

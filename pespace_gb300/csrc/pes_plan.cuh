@@ -63,11 +63,12 @@ enum KernelClass : int {
   kKOther = 7,
 };
 
-// Threads per block of the one-thread-per-sample kernels (ranges, kink): each
+// Threads per block of the mixed plan's ranges and kinks, and of the gradient's
+// set-up by one thread per sample (k_setup_grad, k_tangents64): each
 // thread runs a long FP64 chain, and GB300 issues FP64 at 2 lanes per cycle
 // per SM, so small blocks spread the samples over all SMs instead of
 // queueing 64 lanes on each SM's FP64 pipe.
-// The default; a plan's lnL launches use PesPlan::sample_threads, which
+// The default; the ranges and kinks use PesPlan::sample_threads, which
 // PES_OPT_SAMPLE_THREADS (the autotuner) may change.
 constexpr int kPerSampleThreads = 8;
 
